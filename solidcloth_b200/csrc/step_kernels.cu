@@ -13,6 +13,7 @@
 // the reference decides them. acosf/atan2f are CUDA's and may differ from glibc's
 // by a few ulp (bend angles, angle-weighted normals).
 #include "step_common.cuh"
+#include "quick_fp.cuh"
 #include <cooperative_groups.h>
 #include <cuda/atomic>
 #include <cstdio>
@@ -146,6 +147,7 @@ void launch_solve_cr(cudaStream_t s, const DevCloth& c, const SolverParams& P, c
     }
 }
 
+#define SC_QUICK           // projections on quick_fp.cuh (the fast build has its own approximate forms)
 #include "solver.cuh"     // projections, contact solves and the solver kernels (IEEE build)
 
 // ----------------------------------------------------------- normals
