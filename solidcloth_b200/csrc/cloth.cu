@@ -461,6 +461,7 @@ void ClothModel::release_buffers()
 void ClothModel::release_device()
 {
     release_buffers();
+    release_tile_plan();
     for (void* p : allocs) cudaFree(p);
     allocs.clear();
     dc = DevCloth{};
@@ -923,6 +924,410 @@ size_t ClothModel::band_smem()
     if (prm.dihedral && fits(bend)) { bytes += bend; v.stageBend = 1; }
     if (!prm.fem && fits(link)) { bytes += link; v.stageLink = 1; }
     return bytes;
+}
+
+// ------------------------------------------------------------ tile plan
+// What k_gs_tile needs: the particles of a cloth split into tiles, and per tile
+// and colour the constraints it runs (its own and, redundantly, those its
+// particles depend on inside a group of colours).
+
+// recursive bisection of ids[lo, hi) into k parts along the longer extent
+static void bisect(std::vector<int>& ids, int lo, int hi, int k, const std::vector<V3>& at, std::vector<std::vector<int>>& out)
+{
+    if (k <= 1 || hi - lo <= 1) { out.emplace_back(ids.begin() + lo, ids.begin() + hi); return; }
+    V3 mn3 = at[ids[lo]], mx3 = mn3;
+    for (int i = lo; i < hi; i++) { mn3 = vmin(mn3, at[ids[i]]); mx3 = vmax(mx3, at[ids[i]]); }
+    const V3 ext = mx3 - mn3;
+    const int dir = ext.y > ext.x ? (ext.z > ext.y ? 2 : 1) : (ext.z > ext.x ? 2 : 0);
+    const int kl = k / 2;
+    const int mid = lo + (int)((int64_t)(hi - lo) * kl / k);
+    std::nth_element(ids.begin() + lo, ids.begin() + mid, ids.begin() + hi, [&](int a, int b) {
+        const float x = comp(at[a], dir), y = comp(at[b], dir);
+        return x < y || (x == y && a < b);
+    });
+    bisect(ids, lo, mid, kl, at, out);
+    bisect(ids, mid, hi, k - kl, at, out);
+}
+
+// one class of constraints as the plan sees it, in colour order
+struct TileSource
+{
+    int arity, n, nCol;
+    const std::vector<int>* order;
+    const std::vector<int>* start;
+    std::function<void(int, uint32_t*)> get;
+    double step, each;                          // measured model: us a colour, us a projection of a tile
+    std::vector<int> conOf{};                   // colour * N + particle -> position in the colour order, or -1
+};
+
+void ClothModel::release_tile_plan()
+{
+    for (void* p : tileAllocs) cudaFree(p);
+    tileAllocs.clear();
+    tilePlan = TilePlan{};
+}
+
+// colliders that make triangle / edge contacts
+int ClothModel::feature_colliders() const
+{
+    int n = 0;
+    for (const VColl& g : vcollHost) n += g.type == CT_SPHERE || g.type == CT_SDF || g.type == CT_MESH;
+    return n;
+}
+
+// k_gs_tile takes the Gauss-Seidel solver's tuned mode; a batch's iteration counts
+// must not depend on all its instances at once (its tiles do not wait for one
+// another), and triangle / edge contacts must not reach the serial colour
+bool ClothModel::tile_eligible() const
+{
+    if (solverMode != SOLVE_AUTO || prm.solverType != 1 || N == 0) return false;
+    if (triColourStart.size() > 65 || bendColourStart.size() > 65 || linkColourStart.size() > 65) return false;
+    if (!instV.empty() && (!prm.fixedIterations || prm.resTol > 0.f)) return false;
+    const int slots = feature_colliders();
+    if ((prm.flags & CF_TRIANGLES) && slots * dc.nTriColours >= MAX_COLOURS - 1) return false;
+    if ((prm.flags & CF_EDGES) && slots * dc.nEdgeColours >= MAX_COLOURS - 1) return false;
+    return dc.nTriColours <= 64 && dc.nEdgeColours <= 64;
+}
+
+bool ClothModel::ensure_tile_plan()
+{
+    if (!tile_eligible()) { release_tile_plan(); return false; }
+    const bool selfProx = (prm.flags & CF_SELF) != 0;
+    const int edgeSlots = (prm.flags & CF_EDGES) && instV.empty() ? feature_colliders() : 0;
+    const int triSlots = (prm.flags & CF_TRIANGLES) && instV.empty() ? feature_colliders() : 0;
+    const std::vector<int> key = {N, prm.fem, prm.dihedral, selfProx, prm.ccd, edgeSlots, triSlots, (int)tris.size(), (int)bends.size(), (int)links.size()};
+    if (tilePlan.key == key) return tilePlan.valid;
+    release_tile_plan();
+    tilePlan.key = key;
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (sms < 1) return false;
+    constexpr int K = 5;                        // FEM, bends, links, edge contacts, triangle contacts
+    TileSource src[K];
+    auto fill = [&](TileSource& q, int arity, const std::vector<int>& order, const std::vector<int>& start, double step, double each) {
+        q.arity = arity; q.order = &order; q.start = &start; q.n = (int)order.size(); q.nCol = (int)start.size() - 1;
+        q.step = step; q.each = each;
+    };
+    static const std::vector<int> none, noStart{0};
+    fill(src[0], 3, prm.fem ? triOrder : none, prm.fem ? triColourStart : noStart, 0.3, 0.0015);
+    fill(src[1], 4, prm.dihedral ? bendOrder : none, prm.dihedral ? bendColourStart : noStart, 0.45, 0.003);
+    fill(src[2], 2, prm.fem ? none : linkOrder, prm.fem ? noStart : linkColourStart, 0.1, 0.0005);
+    // contacts: the edges / triangles they may be on, in static colour order
+    std::vector<int> edgeOrder, edgeStart{0};
+    if (edgeSlots)
+    {
+        edgeOrder.resize(dc.E);
+        std::iota(edgeOrder.begin(), edgeOrder.end(), 0);
+        std::stable_sort(edgeOrder.begin(), edgeOrder.end(), [&](int a, int b) { return edgeColourHost[a] < edgeColourHost[b]; });
+        edgeStart.assign(dc.nEdgeColours + 1, 0);
+        for (int c : edgeColourHost) edgeStart[c + 1]++;
+        for (int c = 0; c < dc.nEdgeColours; c++) edgeStart[c + 1] += edgeStart[c];
+    }
+    const std::vector<HEdge>& meshEdges = owner->mesh.edges;
+    fill(src[3], 2, edgeOrder, edgeStart, 0.6, 0.003);
+    fill(src[4], 3, triSlots ? triOrder : none, triSlots ? triColourStart : noStart, 0.8, 0.004);
+    src[3].get = [&](int i, uint32_t* v) { v[0] = meshEdges[i].i1; v[1] = meshEdges[i].i2; };
+    src[4].get = [&](int i, uint32_t* v) { v[0] = tris[i].i1; v[1] = tris[i].i2; v[2] = tris[i].i3; };
+    src[0].get = [&](int i, uint32_t* v) { v[0] = tris[i].i1; v[1] = tris[i].i2; v[2] = tris[i].i3; };
+    src[1].get = [&](int i, uint32_t* v) { v[0] = bends[i].x; v[1] = bends[i].y; v[2] = bends[i].z; v[3] = bends[i].w; };
+    src[2].get = [&](int i, uint32_t* v) { v[0] = links[i].x; v[1] = links[i].y; };
+    // ---- the clothes (batch instances) and how many tiles each gets
+    std::vector<int> first = instV.empty() ? std::vector<int>{0, N} : instV;
+    const int G = (int)first.size() - 1;
+    const int fit = TILE_SMEM_MAX / (int)sizeof(float4);
+    std::vector<int> parts(G, 1);
+    if (G == 1)
+    {
+        // One tile up to 1,500 particles: a colour of it is a quarter of a microsecond
+        // on one SM, less than a split saves (32 x 32, 10 iterations: see the kernel's
+        // comment). With live self-proximity a cloth that fits stays in one tile as
+        // well: its contacts take a hundred colours an iteration, each a CTA barrier
+        // there and a cluster or grid barrier otherwise.
+        if (N > 1500 && !(selfProx && N <= fit)) parts[0] = sms;
+    }
+    else
+    {
+        // shares of the SMs in proportion to the particles; what is worth less than
+        // one SM, or is small, is one closed tile
+        const double each = (double)N / sms;
+        int open = 0;
+        for (int g = 0; g < G; g++)
+        {
+            const int n = first[g + 1] - first[g];
+            int k = n <= 1500 ? 1 : std::max(1, (int)(n / each));
+            if (n > fit) k = std::max(k, 2);
+            parts[g] = k;
+            if (k > 1) open += k;
+        }
+        if (open > sms) return false;
+    }
+    std::vector<std::vector<int>> own;             // particles of each tile
+    std::vector<int> tileInst, instTile(G + 1, 0);
+    std::vector<V3> at = hpos;
+    if ((int)gridIJ.size() == N)
+        for (int i = 0; i < N; i++) at[i] = mk((float)gridIJ[i].x, (float)gridIJ[i].y, 0.f);
+    bool open = false;
+    for (int g = 0; g < G; g++)
+    {
+        instTile[g] = (int)own.size();
+        std::vector<int> ids(first[g + 1] - first[g]);
+        std::iota(ids.begin(), ids.end(), first[g]);
+        bisect(ids, 0, (int)ids.size(), parts[g], at, own);
+        while (tileInst.size() < own.size()) tileInst.push_back(g);
+        open = open || (int)own.size() - instTile[g] > 1;
+    }
+    instTile[G] = (int)own.size();
+    const int nt = (int)own.size();
+    const bool identity = G == 1 && nt == 1 && (selfProx || prm.ccd || edgeSlots || triSlots);
+    // Local numbering. Colour patterns of grids repeat every two or four columns, so
+    // the records of a warp touch every second or fourth particle of a row; numbering
+    // the columns of a row by their remainder first puts those next to one another
+    // (16-byte accesses two or four apart conflict on the shared-memory banks).
+    auto byPattern = [&](int a, int b) {
+        if ((int)gridIJ.size() != N || identity) return a < b;
+        const int2 p = gridIJ[a], q = gridIJ[b];
+        if (p.x != q.x) return p.x < q.x;
+        return (p.y & 3) != (q.y & 3) ? (p.y & 3) < (q.y & 3) : p.y < q.y;
+    };
+    for (auto& o : own) std::sort(o.begin(), o.end(), byPattern);
+    // ---- per class, tile and colour: positions (in the colour order) of the records
+    std::vector<std::vector<std::vector<int>>> rec[K];
+    std::vector<std::vector<int>> halo(nt);
+    TileClass cls[K] = {};
+    for (int k = 0; k < K; k++)
+    {
+        TileSource& q = src[k];
+        rec[k].assign(nt, std::vector<std::vector<int>>(q.nCol));
+        cls[k].nCol = q.nCol;
+        if (q.n == 0) continue;
+        // closed tiles: every record of the instance
+        for (int c = 0; c < q.nCol; c++)
+            for (int j = (*q.start)[c]; j < (*q.start)[c + 1]; j++)
+            {
+                uint32_t v[4];
+                q.get((*q.order)[j], v);
+                const int g = G == 1 ? 0 : (int)(std::upper_bound(first.begin(), first.end(), (int)v[0]) - first.begin()) - 1;
+                if (instTile[g + 1] - instTile[g] == 1) rec[k][instTile[g]][c].push_back(j);
+            }
+        if (!open) continue;
+        q.conOf.assign((size_t)q.nCol * N, -1);
+        for (int c = 0; c < q.nCol; c++)
+            for (int j = (*q.start)[c]; j < (*q.start)[c + 1]; j++)
+            {
+                uint32_t v[4];
+                q.get((*q.order)[j], v);
+                for (int a = 0; a < q.arity; a++)
+                {
+                    int& slot = q.conOf[(size_t)c * N + v[a]];
+                    if (slot >= 0) return false;                   // the overflow colour of a greedy colouring
+                    slot = j;
+                }
+            }
+        // the records tile t runs when the sweep has ng groups, and its halo particles
+        std::vector<int> mark(N, -1), seen(q.n, -1);
+        int tag = 0;
+        auto follow = [&](int t, int ng, std::vector<std::vector<int>>& r, std::vector<int>& all) {
+            const int first = tag;
+            for (int g = 0; g < ng; g++)
+            {
+                std::vector<int> need = own[t];
+                for (int p : need) mark[p] = tag;
+                for (int c = q.nCol * (g + 1) / ng - 1; c >= q.nCol * g / ng; c--)
+                {
+                    const int* con = &q.conOf[(size_t)c * N];
+                    const size_t m = need.size();
+                    for (size_t i = 0; i < m; i++)
+                    {
+                        const int j = con[need[i]];
+                        if (j < 0 || seen[j] >= first) continue;
+                        seen[j] = first;
+                        r[c].push_back(j);
+                        uint32_t v[4];
+                        q.get((*q.order)[j], v);
+                        for (int a = 0; a < q.arity; a++)
+                            if (mark[v[a]] != tag) { mark[v[a]] = tag; need.push_back((int)v[a]); }
+                    }
+                }
+                all.insert(all.end(), need.begin() + own[t].size(), need.end());
+                tag++;
+            }
+            std::sort(all.begin(), all.end());
+            all.erase(std::unique(all.begin(), all.end()), all.end());
+        };
+        std::vector<int> opened;
+        for (int t = 0; t < nt; t++) if (instTile[tileInst[t] + 1] - instTile[tileInst[t]] > 1) opened.push_back(t);
+        // how often to exchange: 1 to 4 groups of colours, the cheapest by the model
+        // over a sample of the tiles
+        double best = 1e30;
+        int groups = 1;
+        for (int ng = 1; ng <= (k < 3 ? std::min(TILE_MAX_GROUPS, q.nCol) : 1); ng++)
+        {
+            std::vector<size_t> most(q.nCol, 0);
+            size_t mostLoc = 0;
+            for (size_t i = 0; i < opened.size(); i += std::max<size_t>(1, opened.size() / 9))
+            {
+                std::vector<std::vector<int>> r(q.nCol);
+                std::vector<int> all;
+                follow(opened[i], ng, r, all);
+                for (int c = 0; c < q.nCol; c++) most[c] = std::max(most[c], r[c].size());
+                mostLoc = std::max(mostLoc, own[opened[i]].size() + all.size());
+            }
+            double cost = 1.5 * ng;
+            for (int c = 0; c < q.nCol; c++) cost += q.step + q.each * (double)most[c];
+            if (mostLoc > (size_t)fit) cost += 1e6;
+            if (cost < best) { best = cost; groups = ng; }
+        }
+        for (int g = 1; g < groups; g++) cls[k].cutMask |= 1ull << (q.nCol * g / groups - 1);
+        for (int t : opened)
+        {
+            follow(t, groups, rec[k][t], halo[t]);
+            for (auto& list : rec[k][t]) std::sort(list.begin(), list.end());
+        }
+        q.conOf.clear();
+        q.conOf.shrink_to_fit();
+    }
+    // ---- reading is mutual: a tile that another one reads from reads a particle of it
+    std::vector<int> ownerOf(N, 0);
+    for (int t = 0; t < nt; t++) for (int p : own[t]) ownerOf[p] = t;
+    {
+        std::vector<std::vector<int>> reads(nt);
+        for (int t = 0; t < nt; t++)
+        {
+            std::sort(halo[t].begin(), halo[t].end());
+            halo[t].erase(std::unique(halo[t].begin(), halo[t].end()), halo[t].end());
+            for (int p : halo[t]) reads[t].push_back(ownerOf[p]);
+            std::sort(reads[t].begin(), reads[t].end());
+            reads[t].erase(std::unique(reads[t].begin(), reads[t].end()), reads[t].end());
+        }
+        for (int t = 0; t < nt; t++)
+            for (int u : reads[t])
+                if (!std::binary_search(reads[u].begin(), reads[u].end(), t)) halo[u].push_back(own[t][0]);
+        for (auto& h : halo) std::sort(h.begin(), h.end(), byPattern);
+    }
+    // ---- local numbering, flattened arrays
+    std::vector<TileDesc> desc(nt);
+    std::vector<int> ids, off[K];
+    std::vector<int4> entry[2];
+    std::vector<float4> fem, link;
+    std::vector<uint4> bend;
+    std::vector<int> loc(N, -1);
+    std::vector<double> cost(nt, 0.0);
+    size_t mostLoc = 0, mostRec = 0;
+    for (int t = 0; t < nt; t++)
+    {
+        TileDesc& d = desc[t];
+        d.idBase = (int)ids.size();
+        d.nOwn = (int)own[t].size();
+        d.nLoc = d.nOwn + (int)halo[t].size();
+        d.peerFirst = instTile[tileInst[t]];
+        d.peers = instTile[tileInst[t] + 1] - d.peerFirst;
+        mostLoc = std::max(mostLoc, (size_t)d.nLoc);
+        int l = 0;
+        for (int p : own[t]) { loc[p] = l++; ids.push_back(p); }
+        for (int p : halo[t]) { loc[p] = l++; ids.push_back(p); }
+        auto count = [&](int k) { return (int)(k == 0 ? fem.size() / 3 : k == 1 ? bend.size() : k == 2 ? link.size() : entry[k - 3].size()); };
+        for (int k = 0; k < K; k++)
+        {
+            for (int c = 0; c < src[k].nCol; c++)
+            {
+                off[k].push_back(count(k));
+                if (k < 3) cost[t] += src[k].step + src[k].each * (double)rec[k][t][c].size();
+                mostRec = std::max(mostRec, rec[k][t][c].size());
+                for (int j : rec[k][t][c])
+                {
+                    const int i = (*src[k].order)[j];
+                    uint32_t pv[4];
+                    src[k].get(i, pv);
+                    for (int a = 0; a < src[k].arity; a++) if (loc[pv[a]] < 0) return false;    // not a particle of the tile
+                    if (k == 0)
+                    {
+                        const FemHost& f = tris[i];
+                        fem.push_back(make_float4(bits_f(loc[f.i1]), bits_f(loc[f.i2]), bits_f(loc[f.i3]), f.du1));
+                        fem.push_back(make_float4(f.du2, f.dv1, f.dv2, f.invDet));
+                        fem.push_back(make_float4(f.lu2, f.lv2, f.lu0 * f.lv0, f.area));
+                    }
+                    else if (k == 1) bend.push_back(make_uint4(loc[bends[i].x], loc[bends[i].y], loc[bends[i].z], loc[bends[i].w]));
+                    else if (k == 3) entry[0].push_back(make_int4(i, loc[meshEdges[i].i1], loc[meshEdges[i].i2], 0));
+                    else if (k == 4) entry[1].push_back(make_int4(i, loc[tris[i].i1], loc[tris[i].i2], loc[tris[i].i3]));
+                    else link.push_back(make_float4(bits_f(loc[links[i].x]), bits_f(loc[links[i].y]), linkRest[i].x, linkRest[i].y));
+                }
+            }
+            off[k].push_back(count(k));
+        }
+        for (int i = d.idBase; i < (int)ids.size(); i++) loc[ids[i]] = -1;
+    }
+    if (mostLoc > (size_t)fit) return false;
+    // ---- CTAs: open tiles one each (all resident), closed ones to the least loaded, largest first
+    std::vector<int> idx(nt);
+    std::iota(idx.begin(), idx.end(), 0);
+    std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) {
+        const bool oa = desc[a].peers > 1, ob = desc[b].peers > 1;
+        return oa != ob ? oa : cost[a] > cost[b];
+    });
+    const int ctas = std::min(nt, sms);
+    std::vector<std::vector<int>> of(ctas);
+    std::vector<double> load(ctas, 0.0);
+    for (int i = 0; i < nt; i++)
+    {
+        const int t = idx[i];
+        const int b = i < ctas ? i : (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        of[b].push_back(t);
+        load[b] += cost[t];
+    }
+    std::vector<int> ctaStart{0}, ctaTile;
+    for (auto& o : of) { ctaTile.insert(ctaTile.end(), o.begin(), o.end()); ctaStart.push_back((int)ctaTile.size()); }
+    tilePlan.smem = mostLoc * sizeof(float4);
+    // as many threads as the largest colour of a tile has records: idle warps cost
+    // issue slots (a 17 x 17 cloth, 64 records a colour: 107 us a substep with 512
+    // threads, 95 with 128)
+    const int threads = mostRec <= 128 && !selfProx ? 128 : mostRec <= 256 && !selfProx ? 256 : 512;
+    if (gs_tile_max_blocks_per_sm(threads, tilePlan.smem) < 1) return false;
+    // ---- device copies
+    bool ok = true;
+    auto put = [&](const void* h, size_t bytes) -> void* {
+        void* p = nullptr;
+        if (!ok || cudaMalloc(&p, std::max<size_t>(bytes, 16)) != cudaSuccess) { cudaGetLastError(); ok = false; return nullptr; }
+        tileAllocs.push_back(p);
+        if (h ? cudaMemcpy(p, h, bytes, cudaMemcpyHostToDevice) != cudaSuccess : cudaMemset(p, 0, bytes) != cudaSuccess) ok = false;
+        return p;
+    };
+    TileView& v = tilePlan.view;
+    v.nTiles = nt;
+    v.N = N;
+    v.threads = threads;
+    v.identity = identity;
+    v.ctaStart = (int*)put(ctaStart.data(), sizeof(int) * ctaStart.size());
+    v.ctaTile = (int*)put(ctaTile.data(), sizeof(int) * ctaTile.size());
+    v.tile = (TileDesc*)put(desc.data(), sizeof(TileDesc) * desc.size());
+    v.ids = (int*)put(ids.data(), sizeof(int) * ids.size());
+    v.fem = cls[0]; v.bend = cls[1]; v.link = cls[2];
+    v.fem.off = (int*)put(off[0].data(), sizeof(int) * off[0].size());
+    v.bend.off = (int*)put(off[1].data(), sizeof(int) * off[1].size());
+    v.link.off = (int*)put(off[2].data(), sizeof(int) * off[2].size());
+    v.femRec = (float4*)put(fem.data(), sizeof(float4) * fem.size());
+    v.bendRec = (uint4*)put(bend.data(), sizeof(uint4) * bend.size());
+    v.linkRec = (float4*)put(link.data(), sizeof(float4) * link.size());
+    for (int k = 0; k < 2; k++)
+    {
+        TileContacts& tc = k == 0 ? v.edgeCt : v.triCt;
+        tc.nSlot = identity ? 0 : k == 0 ? edgeSlots : triSlots;
+        if (!tc.nSlot) continue;
+        tc.nEntry = (int)entry[k].size();
+        tc.cls = cls[3 + k];
+        tc.cls.off = (int*)put(off[3 + k].data(), sizeof(int) * off[3 + k].size());
+        tc.entry = (int4*)put(entry[k].data(), sizeof(int4) * entry[k].size());
+        tc.rec = (float4*)put(nullptr, sizeof(float4) * TILE_CT_WORDS * (size_t)tc.nSlot * (size_t)tc.nEntry);
+    }
+    if (open)
+    {
+        v.xch = (float4*)put(nullptr, sizeof(float4) * 2 * (size_t)N);
+        v.xred = (unsigned long long*)put(nullptr, sizeof(unsigned long long) * 2 * (size_t)nt);
+    }
+    if (!ok) { release_tile_plan(); tilePlan.key = key; return false; }
+    tilePlan.ctas = ctas;
+    tilePlan.open = open;
+    tilePlan.valid = true;
+    return true;
 }
 
 bool ClothModel::upload_topology(const HMesh& mesh)
@@ -1953,7 +2358,7 @@ void ClothPatch::record_substep(float h)
     if (learn) launch_mlp_features(s, c, b, m.sampleFeat ? m.sampleFeat + sub * m.N * MLP_IN : nullptr);
     if (m.warmStart && m.mlpPrm) launch_mlp_warm(s, c, b, m.mlpPrm, m.mlpPrm + MLP_NPARAM);
     // ClothModelPBD::SolveGS (Physics/ClothPBD.cpp:324-369)
-    launch_reset_gs(s, c);
+    launch_reset_gs(s, c, m.choice.kind == SOLVE_TILE ? &m.tilePlan.view : nullptr);
     timing_mark(SEC_GS, false, s);
     record_solve(s, P, m.choice);
     timing_mark(SEC_GS, true, s);
@@ -2007,11 +2412,24 @@ bool ClothPatch::record_solve(cudaStream_t s, const SolverParams& P, const Solve
         plan.nLinkCol = (int)m.linkColourStart.size() - 1;
         for (size_t k = 0; k < m.linkColourStart.size(); k++) plan.linkStart[k] = m.linkColourStart[k];
     }
+    int shift = 0;
+    size_t smem = 0;
+    if (ch.kind == SOLVE_TILE && m.tilePlan.valid)
+    {
+        // self contacts across tiles go to the launch after it (GUARD_*)
+        const bool other = !m.tilePlan.view.identity && ((m.prm.flags & CF_SELF) || m.prm.ccd);
+        if (!ops.tile(s, c, P, b, m.tilePlan.view, m.tilePlan.ctas, m.tilePlan.smem, iterations, other ? GUARD_IF_NO_SELF : GUARD_NONE))
+            return false;
+        if (!other) return true;
+        plan.guard = GUARD_IF_SELF;
+        const int cs = ops.cluster_size(m.N, shift, smem);
+        plan.shift = shift;
+        if (cs > 0) { ops.cluster(s, c, P, b, plan, cs, smem, 0); return true; }
+        return ops.grid(s, c, P, b, plan, 0, 1);
+    }
     if (ch.kind == SOLVE_BAND && m.band_active() &&
         ops.band(s, c, P, b, plan, m.bandPlan.view, m.bandPlan.clusterSize, m.band_smem(), ch.variant))
         return true;                                                 // includes the velocity update
-    int shift = 0;
-    size_t smem = 0;
     const int cluster = (ch.kind == SOLVE_CLUSTER && planFits) ? ops.cluster_size(m.N, shift, smem) : 0;
     if (cluster > 0)
     {
@@ -2102,15 +2520,19 @@ bool ClothPatch::autotune(float h)
     }
     std::vector<SolverChoice> cand;
     int shift = 0; size_t smem = 0;
+    // the tile solver where it applies: it measured faster than every other one over
+    // the whole range (16 x 16 to 256 x 256, batches), so nothing else is timed
+    const bool tile = m.tilePlan.valid;
+    if (tile) cand.push_back({SOLVE_TILE, 0, 0, 0.f});
     const bool fits = m.triColourStart.size() <= 65 && m.bendColourStart.size() <= 65 && m.linkColourStart.size() <= 65;
     const SolverOps& ops = solver_ops(m.prm.fastMath);
     // the band solver (mode 4) sweeps in its own order: only its thread counts are timed
     const bool band = m.band_active();
     if (band)
         for (int v = 0; v < gs_band_variants(); v++) cand.push_back({SOLVE_BAND, v, 0, 0.f});
-    if (!band && fits && (m.solverMode == SOLVE_AUTO || m.solverMode == SOLVE_CLUSTER) && ops.cluster_size(m.N, shift, smem) > 0)
+    if (!tile && !band && fits && (m.solverMode == SOLVE_AUTO || m.solverMode == SOLVE_CLUSTER) && ops.cluster_size(m.N, shift, smem) > 0)
         for (int v = 0; v < gs_cluster_variants(); v++) cand.push_back({SOLVE_CLUSTER, v, 0, 0.f});
-    if (!band && fits && (m.solverMode == SOLVE_AUTO || m.solverMode == SOLVE_GRID))
+    if (!tile && !band && fits && (m.solverMode == SOLVE_AUTO || m.solverMode == SOLVE_GRID))
         for (int v = 0; v < gs_grid_variants(); v++)
         {
             const int mb = ops.grid_max_blocks_per_sm(v);
@@ -2122,7 +2544,7 @@ bool ClothPatch::autotune(float h)
                     if (!dup) cand.push_back({SOLVE_GRID, v, bps, 0.f});
                 }
         }
-    if (!band && m.solverMode == SOLVE_AUTO) cand.push_back({SOLVE_KERNELS, 0, 0, 0.f});
+    if (!tile && !band && m.solverMode == SOLVE_AUTO) cand.push_back({SOLVE_KERNELS, 0, 0, 0.f});
     if (cand.empty()) cand.push_back({SOLVE_KERNELS, 0, 0, 0.f});
     const size_t bytes = sizeof(float4) * (size_t)m.N;
     float4* backup = nullptr;
@@ -2138,7 +2560,7 @@ bool ClothPatch::autotune(float h)
         cudaGraph_t g = nullptr;
         cudaGraphExec_t ge = nullptr;
         if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) continue;
-        launch_reset_gs(stream, m.dc);
+        launch_reset_gs(stream, m.dc, ch.kind == SOLVE_TILE ? &m.tilePlan.view : nullptr);
         record_solve(stream, P, ch);
         if (cudaStreamEndCapture(stream, &g) != cudaSuccess || cudaGraphInstantiate(&ge, g, 0) != cudaSuccess)
         {
@@ -2274,8 +2696,10 @@ bool ClothPatch::step(float dt)
     if (directLaunch)
     {
         // the same substeps, launched one kernel at a time (no graph, no section timing)
+        // a tile plan that came or went (a collider added, a new cloth) retunes the automatic mode
+        const bool had = m.tilePlan.valid, replan = m.ensure_tile_plan() != had && m.solverMode == SOLVE_AUTO;
         if (m.solverMode == SOLVE_KERNELS) m.choice = {SOLVE_KERNELS, 0, 0, 0.f};
-        else if (!m.tuned || m.tunedVersion != m.paramVersion)
+        else if (replan || !m.tuned || m.tunedVersion != m.paramVersion)
         {
             if (!autotune(h)) return false;
             m.tunedVersion = m.paramVersion;
@@ -2292,8 +2716,10 @@ bool ClothPatch::step(float dt)
     if (!graph || graphDt != dt || graphSteps != n || graphParamVersion != m.paramVersion || graphWorldVersion != world.version)
     {
         if (graph) { cudaGraphExecDestroy(graph); graph = nullptr; }
+        // a tile plan that came or went (a collider added, a new cloth) retunes the automatic mode
+        const bool had = m.tilePlan.valid, replan = m.ensure_tile_plan() != had && m.solverMode == SOLVE_AUTO;
         if (m.solverMode == SOLVE_KERNELS) m.choice = {SOLVE_KERNELS, 0, 0, 0.f};
-        else if (!m.tuned || m.tunedVersion != m.paramVersion)
+        else if (replan || !m.tuned || m.tunedVersion != m.paramVersion)
         {
             if (!autotune(h)) return false;
             m.tunedVersion = m.paramVersion;

@@ -110,7 +110,7 @@ struct HostParams
 struct BatchColl { std::shared_ptr<Collidable> coll; int vBegin, vCount, inst; };
 
 // solver selection (autotuned unless forced)
-enum SolverKind { SOLVE_AUTO = 0, SOLVE_CLUSTER = 1, SOLVE_GRID = 2, SOLVE_KERNELS = 3, SOLVE_BAND = 4 };
+enum SolverKind { SOLVE_AUTO = 0, SOLVE_CLUSTER = 1, SOLVE_GRID = 2, SOLVE_KERNELS = 3, SOLVE_BAND = 4, SOLVE_TILE = 5 };
 struct SolverChoice { int kind, variant, blocksPerSm; float ms; int broad; };
 
 struct FemHost { uint32_t i1, i2, i3; float du1, du2, dv1, dv2, det, invDet, lu0, lv0, su, sv, lu2, lv2, area; };
@@ -213,6 +213,21 @@ public:
         BandView view{};                                   // device arrays (in allocs)
     } bandPlan;
     void build_band_plan();
+    // tile solver (k_gs_tile): the plan in use, rebuilt when what it depends on changes
+    struct TilePlan
+    {
+        bool valid = false;
+        std::vector<int> key;
+        int ctas = 0;
+        bool open = false;                                 // some cloth spans several tiles
+        size_t smem = 0;
+        TileView view{};
+    } tilePlan;
+    std::vector<void*> tileAllocs;
+    bool ensure_tile_plan();
+    bool tile_eligible() const;
+    int feature_colliders() const;
+    void release_tile_plan();
     LinkSolve linkSolve{};                      // Jacobi / conjugate-residual link solves (uploaded with the links)
     bool band_active() const { return bandPlan.valid && solverMode == SOLVE_BAND; }
     size_t band_smem();

@@ -113,7 +113,9 @@ void launch_ccd(cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t
 // hits appended (ccd; vertex-triangle on `side` between fork and join)
 void launch_compact_self(cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, const DevCloth& c,
                          const SolverParams& P, const Buffers& b, bool self, bool ccd);
-void launch_reset_gs(cudaStream_t s, const DevCloth& c);
+struct TileView;
+// clears the solver's error and exit words; with a tile plan also its exchange tags
+void launch_reset_gs(cudaStream_t s, const DevCloth& c, const TileView* tv = nullptr);
 
 // The reference's other link solvers (ClothModel::SetSolver, Physics/ClothPBD.cpp:293-298):
 // links in index order, per-link displacements, and each particle's incident links
@@ -150,7 +152,12 @@ struct GsPlan
     int bendStart[65];
     int nLinkCol;            // mass-spring path (FEM off): link colours
     int linkStart[65];
+    int guard;               // GUARD_*: whether the launch does its work
 };
+// A tile launch cannot solve self contacts that reach across its tiles: it works
+// only while there are none, and the launch after it only when there are some
+// (the counts are known on the device alone).
+enum { GUARD_NONE = 0, GUARD_IF_SELF = 1, GUARD_IF_NO_SELF = 2 };
 // cluster size usable for N particles (0: too large or unsupported); sets the
 // log2 particles-per-CTA and the dynamic shared memory per CTA
 int gs_cluster_size(int N, int& shift, size_t& smem);
@@ -193,8 +200,55 @@ constexpr int BAND_SMEM_MAX = 220 * 1024;  // dynamic shared memory per CTA of t
 // threads-per-CTA variants of the band solver (same order, bit-identical results)
 int gs_band_variants();
 int gs_band_threads(int variant);
+// resident CTAs of the tile solver per SM with smem bytes each (0: none)
+int gs_tile_max_blocks_per_sm(int threads, size_t smem);
 // true if a cluster of clusterSize CTAs with smem bytes each can run the band solver
 bool gs_band_fits(int clusterSize, size_t smem);
+
+// tile solver (k_gs_tile): each CTA keeps a tile of the cloth in shared memory,
+// its own particles and a halo around them, and runs several colours between two
+// exchanges, with the halo's constraints computed redundantly
+constexpr int TILE_SMEM_MAX = 200 * 1024;    // dynamic shared memory per CTA: local particles
+constexpr int TILE_MAX_GROUPS = 4;           // exchanges of one class sweep
+struct TileDesc
+{
+    int idBase, nOwn, nLoc;      // its particles in ids[]: nOwn own, then the halo
+    int peers, peerFirst;        // tiles of its cloth and the first of them (1: closed, no exchange)
+};
+struct TileClass
+{
+    int nCol;
+    unsigned long long cutMask;  // an exchange follows colour c inside the sweep (bit c)
+    const int* off;                 // (tile * (nCol + 1) + colour): first record
+};
+// edge or triangle collider contacts: the cloth's edges / triangles a tile may have
+// to solve contacts of, by static colour, and its contact records of the substep
+constexpr int TILE_CT_WORDS = 6;
+struct TileContacts
+{
+    int nSlot;                   // colliders that make such contacts (0: none)
+    int nEntry;                  // entries of all tiles
+    TileClass cls;
+    const int4* entry;           // edge / triangle, its local particles (two or three)
+    float4* rec;                 // nSlot x nEntry x TILE_CT_WORDS
+};
+struct TileView
+{
+    int nTiles, N;
+    int threads;                 // per CTA: 128, 256 or 512
+    int identity;                // one closed tile whose local indices are the particle indices
+    const int* ctaStart;         // tiles of CTA b: ctaTile[ctaStart[b] .. ctaStart[b + 1])
+    const int* ctaTile;
+    const TileDesc* tile;
+    const int* ids;              // global particle of each local one
+    TileClass fem, bend, link;
+    TileContacts edgeCt, triCt;
+    const float4* femRec;        // records as in DevCloth, with local particle indices
+    const uint4* bendRec;
+    const float4* linkRec;
+    float4* xch;                 // 2 N: exchanged positions, w = exchange number (as bits)
+    unsigned long long* xred;    // 2 nTiles: exchanged iteration-end words (number << 32 | value)
+};
 
 // The solver's entry points as one table per build of solver.cuh: IEEE division
 // and square root without FMA contraction (bit-exact with the reference's
@@ -215,6 +269,7 @@ struct SolverOps
     bool (*grid)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&, GsPlan, int, int);
     bool (*band)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&, GsPlan, const BandView&, int, size_t,
                  int);
+    bool (*tile)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&, const TileView&, int, size_t, int, int);
 };
 const SolverOps& solver_ops(bool fast);
 

@@ -27,6 +27,7 @@ enum StatusBits {
     ST_MESH_STACK_OVERFLOW = 32,
     ST_BVH_STACK_OVERFLOW = 64,
     ST_TC_TIMEOUT = 128,         // a tensor-core completion wait of the warm-start network gave up
+    ST_SOLVER_TIMEOUT = 256,     // an exchange wait of the tile solver gave up
 };
 
 struct SolverParams

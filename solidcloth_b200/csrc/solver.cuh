@@ -405,9 +405,25 @@ __global__ void k_solve_vertex_contacts(DevCloth c, SolverParams P, Buffers b)
     if (!P.fixedIterations && err > 0.f) atomic_max_pos(&c.scal[3], err);
 }
 
+// what the edge and triangle contact solves read besides the particles: from the
+// mesh and the start-of-substep positions (the tile solver has it in one record)
+struct GlobalSrc
+{
+    const DevCloth& c;
+    const Buffers& b;
+    __device__ __forceinline__ V3 prev(uint32_t particle, int) const { return ldg3(c.prev, particle); }
+    __device__ __forceinline__ void mesh_edge(const EC& k, V3& p, V3& q) const
+    {
+        const MeshView m = mesh_view(b, k.mesh);
+        const int4 ed = __ldg(&m.edge[k.feature]);
+        p = ldg3(m.v, ed.x); q = ldg3(m.v, ed.y);
+    }
+    __device__ __forceinline__ V3 mesh_normal(const TC& k) const { return ldg3(mesh_view(b, k.mesh).n, k.feature); }
+};
+
 // SolveEdgeContacts for one contact (Physics/ClothCollisionHandler.cpp:289-362)
-template <class PA>
-__device__ float solve_edge_contact(const PA& pa, const DevCloth& c, const SolverParams& P, const Buffers& b, EC& k)
+template <class PA, class SRC>
+__device__ __forceinline__ float solve_edge_contact(const PA& pa, const SRC& src, const SolverParams& P, EC& k)
 {
     float4 a4 = pa.ld(k.idx.x), b4 = pa.ld(k.idx.y);
     V3 x1 = mk(a4.x, a4.y, a4.z), x2 = mk(b4.x, b4.y, b4.z);
@@ -417,10 +433,10 @@ __device__ float solve_edge_contact(const PA& pa, const DevCloth& c, const Solve
     V3 p = w1 * x1 + w2 * x2;
     if (k.mesh >= 0)
     {
-        const MeshView m = mesh_view(b, k.mesh);
-        const int4 ed = __ldg(&m.edge[k.feature]);
+        V3 e1, e2;
+        src.mesh_edge(k, e1, e2);
         float s1, t;
-        closest_segm_segm(ldg3(m.v, ed.x), ldg3(m.v, ed.y), x1, x2, s1, t, point, p);
+        closest_segm_segm(e1, e2, x1, x2, s1, t, point, p);
         w1 = 1.0f - t; w2 = t;
         k.point = f4(point, 0.f);
     }
@@ -435,7 +451,7 @@ __device__ float solve_edge_contact(const PA& pa, const DevCloth& c, const Solve
     V3 disp = dLambda * normal;
     if (P.friction != 0)
     {
-        V3 p0 = w1 * ldg3(c.prev, k.idx.x) + w2 * ldg3(c.prev, k.idx.y);
+        V3 p0 = w1 * src.prev(k.idx.x, 0) + w2 * src.prev(k.idx.y, 1);
         V3 v12 = p - p0 - mk(0.f, 0.f, 0.f);
         float vnrel = dot(normal, v12);
         V3 vt = v12 - vnrel * normal;
@@ -459,8 +475,8 @@ __device__ float solve_edge_contact(const PA& pa, const DevCloth& c, const Solve
 }
 
 // SolveTriContacts for one contact (Physics/ClothCollisionHandler.cpp:204-287)
-template <class PA>
-__device__ float solve_tri_contact(const PA& pa, const DevCloth& c, const SolverParams& P, const Buffers& b, TC& k)
+template <class PA, class SRC>
+__device__ __forceinline__ float solve_tri_contact(const PA& pa, const SRC& src, const SolverParams& P, TC& k)
 {
     float4 a4 = pa.ld(k.idx.x), b4 = pa.ld(k.idx.y), c4 = pa.ld(k.idx.z);
     V3 x1 = mk(a4.x, a4.y, a4.z), x2 = mk(b4.x, b4.y, b4.z), x3 = mk(c4.x, c4.y, c4.z);
@@ -474,7 +490,7 @@ __device__ float solve_tri_contact(const PA& pa, const DevCloth& c, const Solver
     V3 normal = n;
     if (k.mesh >= 0 && k.feature >= 0)
     {
-        V3 mnrm = ldg3(mesh_view(b, k.mesh).n, k.feature);
+        V3 mnrm = src.mesh_normal(k);
         if (dot(n, mnrm) < 0) normal = -n;
     }
     k.normal = f4(normal, 0.f);
@@ -488,7 +504,7 @@ __device__ float solve_tri_contact(const PA& pa, const DevCloth& c, const Solver
     V3 disp = dLambda * normal;
     if (P.friction != 0)
     {
-        V3 p0 = w1 * ldg3(c.prev, k.idx.x) + w2 * ldg3(c.prev, k.idx.y) + w3 * ldg3(c.prev, k.idx.z);
+        V3 p0 = w1 * src.prev(k.idx.x, 0) + w2 * src.prev(k.idx.y, 1) + w3 * src.prev(k.idx.z, 2);
         V3 v12 = p - p0 - mk(0.f, 0.f, 0.f);
         float vnrel = dot(normal, v12);
         V3 vt = v12 - vnrel * normal;
@@ -597,8 +613,9 @@ template <class PA>
 __device__ __forceinline__ float solve_contact(const PA& pa, const DevCloth& c, const SolverParams& P, const Buffers& b, int cls, int i)
 {
     float e;
-    if (cls == 0) { EC k = b.ecList[i]; e = solve_edge_contact(pa, c, P, b, k); b.ecList[i] = k; }
-    else if (cls == 1) { TC k = b.tcList[i]; e = solve_tri_contact(pa, c, P, b, k); b.tcList[i] = k; }
+    const GlobalSrc src{c, b};
+    if (cls == 0) { EC k = b.ecList[i]; e = solve_edge_contact(pa, src, P, k); b.ecList[i] = k; }
+    else if (cls == 1) { TC k = b.tcList[i]; e = solve_tri_contact(pa, src, P, k); b.tcList[i] = k; }
     else if (cls == 2) { SCt k = b.stList[i]; e = solve_self_tri(pa, c, P, k); b.stList[i] = k; }
     else { SCt k = b.seList[i]; e = solve_self_edge(pa, c, P, k); b.seList[i] = k; }
     return e;
@@ -674,6 +691,14 @@ __global__ void k_reset_bend_error(DevCloth c)
     if (threadIdx.x == 0 && !gs_done(c)) c.scal[2] = 0.f;
 }
 
+
+// GUARD_*: does this launch do its work? (the same answer in every thread)
+__device__ __forceinline__ bool guard_open(int guard, const ColourArgs& ca)
+{
+    if (guard == GUARD_NONE) return true;
+    const bool self = *ca.cls[2].count + *ca.cls[3].count > 0;
+    return self == (guard == GUARD_IF_SELF);
+}
 
 struct ClusterPos
 {
@@ -921,6 +946,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_cluster(DevCloth c, SolverPar
 {
     extern __shared__ float4 sPos[];
     __shared__ float sErr[8];
+    if (!guard_open(plan.guard, ca)) return;
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
     const int nRank = (int)cl.num_blocks();
@@ -1270,6 +1296,503 @@ __global__ void __launch_bounds__(NT) k_gs_band(DevCloth c, SolverParams P, Buff
     }
 }
 
+// ---------------------------------------------------------- tile solver
+// One launch per substep; each CTA keeps a tile of the cloth in shared memory:
+// the particles it owns and a halo around them. Between two exchanges it runs a
+// group of colours on its own with CTA barriers, computing redundantly those of
+// the halo's constraints that its own particles depend on (the host follows the
+// dependence backwards through the group's colours, so every listed projection
+// reads exactly the values the whole-cloth sweep would give it; what a tile
+// computes outside its own particles is dropped at the exchange). Same
+// projections in the same order as the per-colour kernels: bit-identical.
+//
+// What bounds it: on one cloth a colour step is the latency of a projection (0.2
+// us) plus the issue of the tile's projections; a grid barrier and the particle
+// loads from L2 after it (3 us a step in k_gs_grid on a 256 x 256 cloth) are paid
+// once a group, as one exchange. An exchange is one 16-byte word per particle
+// with the exchange's number in it, written and polled in L2: no barrier and no
+// fence, one L2 round trip. Two words per particle alternate; a tile can be one
+// exchange ahead of the tiles it reads from at most, because reading is mutual.
+//
+// A closed tile (a whole cloth, or a batch instance) has no halo and never
+// waits; a CTA may have several of them, one after the other.
+constexpr int TILE_SPIN_LIMIT = 1 << 21;     // polls of one word before a wait gives up
+
+__device__ __forceinline__ void st_tagged(float4* p, float4 x, unsigned tag)
+{
+    const unsigned long long lo = ((unsigned long long)__float_as_uint(x.y) << 32) | __float_as_uint(x.x);
+    const unsigned long long hi = ((unsigned long long)tag << 32) | __float_as_uint(x.z);
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}"
+                 :: "l"(p), "l"(lo), "l"(hi) : "memory");
+}
+__device__ __forceinline__ float4 ld_tagged(const float4* p, unsigned& tag)
+{
+    unsigned long long lo, hi;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+    tag = (unsigned)(hi >> 32);
+    return make_float4(__uint_as_float((unsigned)lo), __uint_as_float((unsigned)(lo >> 32)), __uint_as_float((unsigned)hi), 0.f);
+}
+
+// particle accessors: the tile's local particles; one particle whatever its index
+struct TilePos
+{
+    float4* p;
+    __device__ __forceinline__ float4 ld(uint32_t v) const { return p[v]; }
+    __device__ __forceinline__ void st(uint32_t v, float4 x) const { p[v] = x; }
+};
+struct TileOnePos
+{
+    float4* p;
+    __device__ __forceinline__ float4 ld(uint32_t) const { return *p; }
+    __device__ __forceinline__ void st(uint32_t, float4 x) const { *p = x; }
+};
+
+// a tile's side of the exchanges
+template <int NT>
+struct TileLink
+{
+    const TileView& tv;
+    float4* sPos;
+    const int* ids;
+    int tile, nOwn, nLoc, peers, peerFirst;
+    unsigned seq;            // exchanges so far in this launch
+    unsigned rseq;           // iteration-end words exchanged so far
+    int* status;
+
+    // own positions out, halo positions in; false if a wait gave up (uniform)
+    __device__ bool exchange()
+    {
+        seq++;
+        float4* buf = tv.xch + (seq & 1u ? (size_t)tv.N : 0);
+        for (int i = threadIdx.x; i < nOwn; i += NT) st_tagged(buf + __ldg(&ids[i]), sPos[i], seq);
+        bool ok = true;
+        // two polls in flight a thread: most tiles' halos take two rounds
+        for (int i = nOwn + (int)threadIdx.x; i < nLoc; i += 2 * NT)
+        {
+            const int j = i + NT;
+            const float4* pi = buf + __ldg(&ids[i]);
+            const float4* pj = buf + (j < nLoc ? __ldg(&ids[j]) : __ldg(&ids[i]));
+            unsigned ti, tj;
+            float4 xi = ld_tagged(pi, ti), xj = ld_tagged(pj, tj);
+            int spin = 0;
+            while ((ti != seq || tj != seq) && ++spin < TILE_SPIN_LIMIT)
+            {
+                if (ti != seq) xi = ld_tagged(pi, ti);
+                if (tj != seq) xj = ld_tagged(pj, tj);
+            }
+            ok = ok && ti == seq && tj == seq;
+            xi.w = sPos[i].w;
+            sPos[i] = xi;
+            if (j < nLoc) { xj.w = sPos[j].w; sPos[j] = xj; }
+        }
+        if (!ok) atomicOr(status, ST_SOLVER_TIMEOUT);
+        return __syncthreads_and(ok) != 0;
+    }
+
+    // largest of the cloth's tiles' words (each already the same in every thread of its CTA)
+    __device__ bool reduce_max(unsigned& v)
+    {
+        __shared__ unsigned sMax;
+        rseq++;
+        unsigned long long* buf = tv.xred + (rseq & 1u ? (size_t)tv.nTiles : 0);
+        if (threadIdx.x == 0)
+        {
+            sMax = v;
+            asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(buf + tile), "l"(((unsigned long long)rseq << 32) | v) : "memory");
+        }
+        __syncthreads();
+        bool ok = true;
+        for (int k = threadIdx.x; k < peers; k += NT)
+        {
+            unsigned long long w = 0;
+            int spin = 0;
+            do asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(buf + peerFirst + k) : "memory");
+            while ((unsigned)(w >> 32) != rseq && ++spin < TILE_SPIN_LIMIT);
+            ok = ok && (unsigned)(w >> 32) == rseq;
+            atomicMax(&sMax, (unsigned)w);
+        }
+        if (!ok) atomicOr(status, ST_SOLVER_TIMEOUT);
+        ok = __syncthreads_and(ok) != 0;
+        v = sMax;
+        __syncthreads();
+        return ok;
+    }
+};
+
+// records of class KIND (0 FEM, 1 bend, 2 link) of a tile, through the
+// non-coherent path: they stay in L1 between the sweeps. Volatile, so that a
+// prefetch stays where it is written (the compiler sinks a plain load to its use).
+__device__ __forceinline__ float4 ld_record(const float4* p)
+{
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+template <int KIND>
+__device__ __forceinline__ BandRec<KIND> tile_load(const TileView& tv, int j)
+{
+    BandRec<KIND> q;
+    if constexpr (KIND == 0)
+    {
+        const float4* r = tv.femRec + 3 * (size_t)j;
+        q.r[0] = ld_record(r); q.r[1] = ld_record(r + 1); q.r[2] = ld_record(r + 2);
+    }
+    else q.r[0] = ld_record(KIND == 1 ? reinterpret_cast<const float4*>(tv.bendRec) + j : tv.linkRec + j);
+    return q;
+}
+
+template <int KIND>
+__device__ __forceinline__ float tile_apply(const TilePos& pa, const SolverParams& P, const BandRec<KIND>& q)
+{
+    const float4 f = q.r[0];
+    if constexpr (KIND == 0) { fem_project(pa, q.r[0], q.r[1], q.r[2], P); return 0.f; }
+    else if constexpr (KIND == 1)
+        return bend_project(pa, make_uint4(__float_as_uint(f.x), __float_as_uint(f.y), __float_as_uint(f.z), __float_as_uint(f.w)), P);
+    else return link_project(pa, f, P);
+}
+
+// one sweep of a class over the tile. Each thread's first record of the next
+// colour is loaded before the current colour's projections. An exchange ends
+// every group but the last; the caller decides on that one. False if a wait gave
+// up. The loop is kept short for the warps that have nothing to do in a colour:
+// they share the schedulers with those that have.
+template <int KIND, int NT>
+__device__ __forceinline__ bool tile_sweep(TileLink<NT>& lk, const SolverParams& P, const TileClass& cl, const int* off, float& err)
+{
+    const TilePos pa{lk.sPos};
+    const int tid = (int)threadIdx.x;
+    const int nCol = cl.nCol;
+    if (nCol == 0) return true;
+    const unsigned long long cuts = lk.peers > 1 ? cl.cutMask : 0ull;
+    int j = off[0] + tid, e = off[1];
+    BandRec<KIND> cur;
+    if (j < e) cur = tile_load<KIND>(lk.tv, j);
+    for (int col = 0; col < nCol; col++)
+    {
+        const int jn = e + tid, en = off[min(col + 2, nCol)];
+        BandRec<KIND> nxt;
+        if (jn < en) nxt = tile_load<KIND>(lk.tv, jn);
+        while (j < e)
+        {
+            err = fmaxf(err, tile_apply<KIND>(pa, P, cur));
+            j += NT;
+            if (j < e) cur = tile_load<KIND>(lk.tv, j);
+        }
+        __syncthreads();
+        if ((cuts >> col) & 1ull) if (!lk.exchange()) return false;
+        cur = nxt;
+        j = jn; e = en;
+    }
+    return true;
+}
+
+// ---- edge and triangle collider contacts in tiles
+// The contacts of a substep sit in per-edge and per-triangle slots and are solved
+// by the static colour of their edge / triangle, so a tile finds the ones it has
+// to run (redundant ones included) in its lists of edges and triangles. It copies
+// each into a record of its own with everything the solve reads besides the
+// particles: one coalesced load per contact and colour in the place of a chain of
+// five to eight dependent ones (order, contact, mesh, index, vertices). The
+// multipliers live in the record (every tile that runs a contact keeps its own
+// copy of them, all equal); the tile that owns the first particle also writes the
+// contact list, which the getters read.
+struct EdgeRecSrc
+{
+    V3 a, b, p1, p2;
+    __device__ __forceinline__ V3 prev(uint32_t, int i) const { return i == 0 ? p1 : p2; }
+    __device__ __forceinline__ void mesh_edge(const EC&, V3& p, V3& q) const { p = a; q = b; }
+};
+struct TriRecSrc
+{
+    V3 n, p1, p2, p3;
+    __device__ __forceinline__ V3 prev(uint32_t, int i) const { return i == 0 ? p1 : i == 1 ? p2 : p3; }
+    __device__ __forceinline__ V3 mesh_normal(const TC&) const { return n; }
+};
+
+// this substep's records of tile t: KIND 0 edge contacts, 1 triangle contacts
+template <int KIND, int NT>
+__device__ __forceinline__ void tile_contact_records(const TileView& tv, const DevCloth& c, const Buffers& b,
+                                                     const TileDesc& d, int t, int* cnt)
+{
+    const TileContacts& tc = KIND == 0 ? tv.edgeCt : tv.triCt;
+    const int* off = tc.cls.off + (size_t)t * (tc.cls.nCol + 1);
+    const int first = __ldg(&off[0]), end = __ldg(&off[tc.cls.nCol]);
+    const int items = KIND == 0 ? c.E : c.T;
+    const int* flag = KIND == 0 ? b.ecFlag : b.tcFlag;
+    for (int slot = 0; slot < tc.nSlot; slot++)
+        for (int j = first + (int)threadIdx.x; j < end; j += NT)
+        {
+            const int4 en = __ldg(&tc.entry[j]);              // item, local particles
+            const int f = __ldg(&flag[(size_t)slot * items + en.x]);
+            if (f == 0) continue;
+            const int col = (int)(KIND == 0 ? c.edgeColour[en.x] : c.triColour[en.x]);
+            const int at = __ldg(&off[col]) + atomicAdd(&cnt[slot * tc.cls.nCol + col], 1);
+            float4* r = tc.rec + TILE_CT_WORDS * ((size_t)slot * tc.nEntry + at);
+            const unsigned own = en.y < d.nOwn ? 0x80000000u : 0u;
+            if constexpr (KIND == 0)
+            {
+                const EC k = b.ecList[f - 1];
+                float4 a = k.point, e = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (k.mesh >= 0)
+                {
+                    const MeshView m = mesh_view(b, k.mesh);
+                    const int4 ed = __ldg(&m.edge[k.feature]);
+                    a = __ldg(&m.v[ed.x]); e = __ldg(&m.v[ed.y]);
+                }
+                r[0] = make_float4(__uint_as_float((unsigned)en.y | ((unsigned)en.z << 16)), __uint_as_float((unsigned)(f - 1) | own), k.lam.x, k.lam.y);
+                r[1] = make_float4(a.x, a.y, a.z, __int_as_float(k.mesh));
+                r[2] = make_float4(e.x, e.y, e.z, k.w.x);
+                r[3] = make_float4(k.normal.x, k.normal.y, k.normal.z, k.w.y);
+                r[4] = __ldg(&c.prev[k.idx.x]);
+                r[5] = __ldg(&c.prev[k.idx.y]);
+            }
+            else
+            {
+                const TC k = b.tcList[f - 1];
+                const bool mesh = k.mesh >= 0 && k.feature >= 0;
+                const float4 n = mesh ? __ldg(&mesh_view(b, k.mesh).n[k.feature]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                r[0] = make_float4(__uint_as_float((unsigned)en.y | ((unsigned)en.z << 16)), __uint_as_float((unsigned)en.w), k.lam.x, k.lam.y);
+                r[1] = make_float4(k.point.x, k.point.y, k.point.z, __uint_as_float((unsigned)(f - 1) | own));
+                r[2] = make_float4(n.x, n.y, n.z, __int_as_float(mesh ? 0 : -1));
+                r[3] = __ldg(&c.prev[k.idx.x]);
+                r[4] = __ldg(&c.prev[k.idx.y]);
+                r[5] = __ldg(&c.prev[k.idx.z]);
+            }
+        }
+}
+
+// one sweep of the tile's edge (KIND 0) or triangle (1) contacts; the caller exchanges after it
+template <int KIND, int NT>
+__device__ __forceinline__ float tile_contact_sweep(const TilePos& pa, const TileView& tv, const SolverParams& P, const Buffers& b,
+                                                    int t, const int* cnt)
+{
+    const TileContacts& tc = KIND == 0 ? tv.edgeCt : tv.triCt;
+    const int* off = tc.cls.off + (size_t)t * (tc.cls.nCol + 1);
+    float err = 0.f;
+    for (int slot = 0; slot < tc.nSlot; slot++)
+        for (int col = 0; col < tc.cls.nCol; col++)
+        {
+            const int n = cnt[slot * tc.cls.nCol + col];
+            if (n == 0) continue;
+            float4* base = tc.rec + TILE_CT_WORDS * ((size_t)slot * tc.nEntry + __ldg(&off[col]));
+            for (int j = (int)threadIdx.x; j < n; j += NT)
+            {
+                float4* r = base + TILE_CT_WORDS * (size_t)j;
+                const float4 q0 = r[0], q1 = r[1], q2 = r[2], q3 = r[3], q4 = r[4], q5 = r[5];
+                const unsigned ids = __float_as_uint(q0.x);
+                if constexpr (KIND == 0)
+                {
+                    EC k;
+                    k.idx = make_uint4(ids & 0xffffu, ids >> 16, 0u, 0u);
+                    k.point = q1; k.normal = q3; k.w = make_float4(q2.w, q3.w, 0.f, 0.f);
+                    k.lam = make_float2(q0.z, q0.w);
+                    k.mesh = __float_as_int(q1.w); k.feature = 0;
+                    const EdgeRecSrc src{mk(q1), mk(q2), mk(q4), mk(q5)};
+                    err = fmaxf(err, solve_edge_contact(pa, src, P, k));
+                    *reinterpret_cast<float2*>(&r[0].z) = k.lam;
+                    const unsigned li = __float_as_uint(q0.y);
+                    if (li & 0x80000000u)
+                    {
+                        EC& o = b.ecList[li & 0x7fffffffu];
+                        o.point = make_float4(k.point.x, k.point.y, k.point.z, 0.f); o.w = k.w; o.lam = k.lam;
+                    }
+                }
+                else
+                {
+                    TC k;
+                    k.idx = make_uint4(ids & 0xffffu, ids >> 16, __float_as_uint(q0.y), 0u);
+                    k.point = q1; k.lam = make_float2(q0.z, q0.w);
+                    k.mesh = k.feature = __float_as_int(q2.w);
+                    const TriRecSrc src{mk(q2), mk(q3), mk(q4), mk(q5)};
+                    err = fmaxf(err, solve_tri_contact(pa, src, P, k));
+                    *reinterpret_cast<float2*>(&r[0].z) = k.lam;
+                    const unsigned li = __float_as_uint(q1.w);
+                    if (li & 0x80000000u)
+                    {
+                        TC& o = b.tcList[li & 0x7fffffffu];
+                        o.normal = k.normal; o.w = k.w; o.lam = k.lam;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    return err;
+}
+
+// The contact classes of a cloth in one closed tile (local indices are the
+// particle indices), colour by colour with CTA barriers.
+template <int NT>
+__device__ __forceinline__ void tile_contact_classes(const TilePos& pa, const DevCloth& c, const SolverParams& P,
+                                                     const Buffers& b, const ColourArgs& ca, bool track, float* sErr)
+{
+    for (int cls = 0; cls < 4; cls++)
+    {
+        const ClassView& cv = ca.cls[cls];
+        const int n = *cv.count;
+        if (n == 0) continue;
+        for (int col = 0; col < MAX_COLOURS; col++)
+        {
+            const int s0 = cv.start[col], s1 = cv.start[col + 1];
+            if (s0 == s1) continue;
+            if (col == MAX_COLOURS - 1)
+            {
+                // colours exhausted: one thread, list order (as the oracle)
+                if (threadIdx.x == 0)
+                    for (int i = 0; i < n; i++)
+                        if (cv.colour[i] == MAX_COLOURS - 1)
+                        {
+                            const float e = solve_contact(pa, c, P, b, cls, i);
+                            if (track && e > 0.f) atomicMax((int*)&sErr[4 + cls], __float_as_int(e));
+                        }
+            }
+            else
+                for (int j = s0 + (int)threadIdx.x; j < s1; j += NT)
+                {
+                    const float e = solve_contact(pa, c, P, b, cls, __ldg(&cv.order[j]));
+                    if (track && e > 0.f) atomicMax((int*)&sErr[4 + cls], __float_as_int(e));
+                }
+            __syncthreads();
+        }
+    }
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT, 1) k_gs_tile(DevCloth c, SolverParams P, Buffers b, ColourArgs ca,
+                                                              __grid_constant__ const TileView tv, int iterations, int guard)
+{
+    extern __shared__ float4 sPos[];
+    __shared__ float sErr[8];
+    __shared__ int sOff[3][65];
+    __shared__ unsigned sRes;
+    __shared__ int sCnt[2][MAX_COLOURS];
+    if (!guard_open(guard, ca)) return;
+    const int tid = (int)threadIdx.x;
+    const bool track = !P.fixedIterations;
+    // collider contacts of this substep (the same answer in every tile)
+    const bool edges = tv.edgeCt.nSlot > 0 && *ca.cls[0].count > 0, triangles = tv.triCt.nSlot > 0 && *ca.cls[1].count > 0;
+    for (int item = tv.ctaStart[blockIdx.x]; item < tv.ctaStart[blockIdx.x + 1]; item++)
+    {
+        const int t = tv.ctaTile[item];
+        const TileDesc d = tv.tile[t];
+        TileLink<NT> lk{tv, sPos, tv.ids + d.idBase, t, d.nOwn, d.nLoc, d.peers, d.peerFirst, 0u, 0u, c.status};
+        for (int i = tid; i < d.nLoc; i += NT) sPos[i] = c.pos[__ldg(&lk.ids[i])];
+        for (int j = tid; j <= tv.fem.nCol; j += NT) sOff[0][j] = __ldg(&tv.fem.off[t * (tv.fem.nCol + 1) + j]);
+        for (int j = tid; j <= tv.bend.nCol; j += NT) sOff[1][j] = __ldg(&tv.bend.off[t * (tv.bend.nCol + 1) + j]);
+        for (int j = tid; j <= tv.link.nCol; j += NT) sOff[2][j] = __ldg(&tv.link.off[t * (tv.link.nCol + 1) + j]);
+        if (tid < 8) sErr[tid] = 0.f;
+        if (edges || triangles)
+        {
+            for (int j = tid; j < 2 * MAX_COLOURS; j += NT) sCnt[j / MAX_COLOURS][j % MAX_COLOURS] = 0;
+            __syncthreads();
+            if (edges) tile_contact_records<0, NT>(tv, c, b, d, t, sCnt[0]);
+            if (triangles) tile_contact_records<1, NT>(tv, c, b, d, t, sCnt[1]);
+        }
+        if (P.resTol > 0.f)
+            for (int i = tid; i < d.nOwn; i += NT) c.xsnap[__ldg(&lk.ids[i])] = sPos[i];
+        __syncthreads();
+        bool ok = true;
+        for (int k = 0; k < iterations && ok; k++)
+        {
+            float err = 0.f;
+            if (P.fem) ok = tile_sweep<0, NT>(lk, P, tv.fem, sOff[0], err);
+            else
+            {
+                ok = tile_sweep<2, NT>(lk, P, tv.link, sOff[2], err);
+                if (track && err > 0.f) atomicMax((int*)&sErr[1], __float_as_int(err));
+            }
+            if (!ok) break;
+            if (P.dihedral && k % P.bendFreq == 0 && tv.bend.nCol > 0)
+            {
+                if (lk.peers > 1 && !(ok = lk.exchange())) break;
+                err = 0.f;
+                if (!(ok = tile_sweep<1, NT>(lk, P, tv.bend, sOff[1], err))) break;
+                if (track && err > 0.f) atomicMax((int*)&sErr[2], __float_as_int(err));
+            }
+            if (b.numVColl > 0)
+            {
+                // a vertex contact moves one particle: the owner's own, ahead of the exchange
+                for (int i = tid; i < d.nOwn; i += NT)
+                {
+                    const float e = vertex_contacts_one(TileOnePos{&sPos[i]}, c, P, b, __ldg(&lk.ids[i]));
+                    if (track && e > 0.f) atomicMax((int*)&sErr[3], __float_as_int(e));
+                }
+                __syncthreads();
+            }
+            if (edges)
+            {
+                if (lk.peers > 1 && !(ok = lk.exchange())) break;
+                err = tile_contact_sweep<0, NT>(TilePos{sPos}, tv, P, b, t, sCnt[0]);
+                if (track && err > 0.f) atomicMax((int*)&sErr[4], __float_as_int(err));
+            }
+            if (triangles)
+            {
+                if (lk.peers > 1 && !(ok = lk.exchange())) break;
+                err = tile_contact_sweep<1, NT>(TilePos{sPos}, tv, P, b, t, sCnt[1]);
+                if (track && err > 0.f) atomicMax((int*)&sErr[5], __float_as_int(err));
+            }
+            if (tv.identity) tile_contact_classes<NT>(TilePos{sPos}, c, P, b, ca, track, sErr);
+            // the last exchange of a launch is needed only if there was none before it:
+            // no tile may write its particles back before its neighbours have loaded them
+            if (lk.peers > 1 && (k + 1 < iterations || lk.seq == 0) && !(ok = lk.exchange())) break;
+            if (tid == 0 && t == 0) c.scal[9] = (float)(k + 1);
+            if (P.resTol > 0.f)
+            {
+                // residual-target mode: the largest displacement of this iteration
+                // (own particles, against the snapshot) over the cloth
+                float r = 0.f;
+                if (tid == 0) sRes = 0u;
+                __syncthreads();
+                for (int i = tid; i < d.nOwn; i += NT)
+                {
+                    const int g = __ldg(&lk.ids[i]);
+                    const float4 x = sPos[i], x0 = c.xsnap[g];
+                    const float dx = x.x - x0.x, dy = x.y - x0.y, dz = x.z - x0.z;
+                    r = fmaxf(r, sqrtf(dx * dx + dy * dy + dz * dz) * P.resScale);
+                    c.xsnap[g] = x;
+                }
+                const unsigned u = __reduce_max_sync(0xffffffffu, __float_as_uint(r));
+                if ((tid & 31) == 0 && u) atomicMax(&sRes, u);
+                __syncthreads();
+                unsigned m = sRes;
+                if (lk.peers > 1 && !(ok = lk.reduce_max(m))) break;
+                if (__uint_as_float(m) <= P.resTol) break;
+            }
+            if (track)
+            {
+                // SolveGS exit test (Physics/ClothPBD.cpp:354-361): the maxima over the
+                // cloth pass iff every tile's do (redundant projections only repeat
+                // another tile's value)
+                __syncthreads();
+                const float eps = 0.01f;
+                const float clk = P.fem ? 0.f : sErr[1];
+                const bool done = clk < 0.05f && sErr[2] < 0.005f && sErr[7] < P.selfThreshold && sErr[6] < P.selfThreshold &&
+                                  sErr[3] < eps && sErr[4] < eps && sErr[5] < eps;
+                unsigned m = done ? 0u : 1u;
+                __syncthreads();
+                if (tid < 8 && (tid != 2 || (k + 1) % P.bendFreq == 0)) sErr[tid] = 0.f;    // [2]: kept until the next bend sweep
+                __syncthreads();
+                if (lk.peers > 1 && !(ok = lk.reduce_max(m))) break;
+                if (m == 0u) { if (tid == 0 && t == 0) c.scal[8] = 1.f; break; }
+            }
+        }
+        __syncthreads();
+        if (tid == 0 && t == 0) c.scal[10] += c.scal[9];
+        // write back own particles and update their velocities (ClothPBD.cpp:314-321)
+        for (int i = tid; i < d.nOwn; i += NT)
+        {
+            const int g = __ldg(&lk.ids[i]);
+            const float4 p = sPos[i];
+            c.pos[g] = p;
+            if (p.w == 0.f) continue;
+            const float4 q = c.prev[g];
+            V3 vel = P.invH * (mk(p.x, p.y, p.z) - mk(q.x, q.y, q.z));
+            c.vel[g] = make_float4(vel.x, vel.y, vel.z, 0.f);
+        }
+        __syncthreads();
+    }
+}
+
 // ---------------------------------------------------- grid-resident solver
 // The same Gauss-Seidel loop as k_gs_cluster for clothes (and batches of
 // clothes) too large for one cluster: one cooperative launch per substep, every
@@ -1360,6 +1883,7 @@ __device__ __forceinline__ float bend_tiles(const DevCloth& c, const SolverParam
 template <int NT, int FT, int BT>
 __global__ void __launch_bounds__(NT) k_gs_grid(DevCloth c, SolverParams P, Buffers b, ColourArgs ca, GsPlan plan)
 {
+    if (!guard_open(plan.guard, ca)) return;
     cg::grid_group grid = cg::this_grid();
     __shared__ float sErr[8];
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
@@ -1661,6 +2185,45 @@ bool launch_gs_band(cudaStream_t s, const DevCloth& c, const SolverParams& P, co
     return cudaLaunchKernelEx(&cfg, kBandVariants[variant], c, P, b, colour_args(b), plan, bv) == cudaSuccess;
 }
 
+// ---------------------------------------------- tile solver launcher
+using TileKernel = void (*)(DevCloth, SolverParams, Buffers, ColourArgs, const TileView, int, int);
+static TileKernel tile_kernel(int threads) { return threads == 128 ? k_gs_tile<128> : threads == 256 ? k_gs_tile<256> : k_gs_tile<512>; }
+
+static void tile_attributes()
+{
+    static std::once_flag once;
+    std::call_once(once, [] {
+        for (int t : {128, 256, 512}) cudaFuncSetAttribute(tile_kernel(t), cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM_MAX);
+        cudaGetLastError();
+    });
+}
+
+int gs_tile_max_blocks_per_sm(int threads, size_t smem)
+{
+    tile_attributes();
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_kernel(threads), threads, smem) != cudaSuccess) n = 0;
+    cudaGetLastError();
+    return n;
+}
+
+// a cooperative launch where tiles wait for one another (all of them resident)
+bool launch_gs_tile(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, const TileView& tv,
+                    int ctas, size_t smem, int iterations, int guard)
+{
+    tile_attributes();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(tv.threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = tv.xch ? 1 : 0;
+    cfg.attrs = &at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, tile_kernel(tv.threads), c, P, b, colour_args(b), tv, iterations, guard) == cudaSuccess;
+}
+
 // ---------------------------------------------- per-colour path launchers
 void launch_reset_link_error(cudaStream_t s, const DevCloth& c)
 {
@@ -1693,4 +2256,5 @@ void launch_solve_multi_contacts(cudaStream_t s, const DevCloth& c, const Solver
 // this build's entry points
 static const SolverOps kSolverOps = {launch_fem, launch_links, launch_reset_link_error, launch_bends,
                                      launch_solve_vertex_contacts, launch_solve_multi_contacts, gs_cluster_size,
-                                     launch_gs_cluster, gs_grid_max_blocks_per_sm, launch_gs_grid, launch_gs_band};
+                                     launch_gs_cluster, gs_grid_max_blocks_per_sm, launch_gs_grid, launch_gs_band,
+                                     launch_gs_tile};

@@ -944,15 +944,18 @@ void scan_ints(cudaStream_t s, const int* in, int* out, int n, int* total, int* 
     k_scan_down<<<nb, SCAN_T, 0, s>>>(in, out, n, tmp);
 }
 
-// gather items with count[i] records from slots[i*K + k] to dense[base + off[i] + k]
+// gather items with count[i] records from slots[i*K + k] to dense[base + off[i] + k];
+// `place` (optional): 1 + the item's first place in the list, for items that have one
 template <typename R>
-__global__ void k_compact(const int* cnt, const int* off, const R* slots, int K, R* dense, int n, const int* base, int cap, int* status, int ovfBit)
+__global__ void k_compact(const int* cnt, const int* off, const R* slots, int K, R* dense, int n, const int* base, int cap, int* status, int ovfBit,
+                          int* place = nullptr)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int m = cnt[i];
     if (m == 0) return;
     int o = off[i] + (base ? *base : 0);
+    if (place && o < cap) place[i] = 1 + o;
     for (int k = 0; k < m; k++)
     {
         if (o + k < cap) dense[o + k] = slots[(size_t)i * K + k];
@@ -2116,7 +2119,7 @@ void launch_tri_edge_colliders(cudaStream_t s, const DevCloth& c, const SolverPa
     {
         int n = ti * c.T;
         scan_ints(s, b.tcFlag, b.scanOff, n, b.tcCount, b.scanBlock);
-        k_compact<TC><<<blocks_for(n), 256, 0, s>>>(b.tcFlag, b.scanOff, b.tcSlot, 1, b.tcList, n, nullptr, b.tcCap, c.status, ST_CONTACT_OVERFLOW);
+        k_compact<TC><<<blocks_for(n), 256, 0, s>>>(b.tcFlag, b.scanOff, b.tcSlot, 1, b.tcList, n, nullptr, b.tcCap, c.status, ST_CONTACT_OVERFLOW, b.tcFlag);
         k_add_counts<<<1, 32, 0, s>>>(b.tcCount, b.tcCount, nullptr, b.tcCap);
     }
     else cudaMemsetAsync(b.tcCount, 0, sizeof(int), s);
@@ -2124,7 +2127,7 @@ void launch_tri_edge_colliders(cudaStream_t s, const DevCloth& c, const SolverPa
     {
         int n = ei * c.E;
         scan_ints(s, b.ecFlag, b.scanOff, n, b.ecCount, b.scanBlock);
-        k_compact<EC><<<blocks_for(n), 256, 0, s>>>(b.ecFlag, b.scanOff, b.ecSlot, 1, b.ecList, n, nullptr, b.ecCap, c.status, ST_CONTACT_OVERFLOW);
+        k_compact<EC><<<blocks_for(n), 256, 0, s>>>(b.ecFlag, b.scanOff, b.ecSlot, 1, b.ecList, n, nullptr, b.ecCap, c.status, ST_CONTACT_OVERFLOW, b.ecFlag);
         k_add_counts<<<1, 32, 0, s>>>(b.ecCount, b.ecCount, nullptr, b.ecCap);
     }
     else cudaMemsetAsync(b.ecCount, 0, sizeof(int), s);
@@ -2266,9 +2269,20 @@ void launch_residual(cudaStream_t s, const DevCloth& c, unsigned* out)
     k_residual<<<2 * 148, 256, 0, s>>>(c, out);
 }
 
-void launch_reset_gs(cudaStream_t s, const DevCloth& c)
+// one launch in the place of the memset: no exchange of an earlier substep may
+// satisfy a wait of this one
+__global__ void k_tile_reset(DevCloth c, TileView tv)
 {
-    cudaMemsetAsync(c.scal + 1, 0, sizeof(float) * 9, s);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 9) c.scal[1 + i] = 0.f;
+    if (i < 2 * tv.nTiles) tv.xred[i] = 0ull;
+    if (i < 2 * tv.N) tv.xch[i].w = 0.f;
+}
+
+void launch_reset_gs(cudaStream_t s, const DevCloth& c, const TileView* tv)
+{
+    if (tv && tv->xch) k_tile_reset<<<blocks_for(std::max(2 * tv->N, 2 * tv->nTiles)), 256, 0, s>>>(c, *tv);
+    else cudaMemsetAsync(c.scal + 1, 0, sizeof(float) * 9, s);
 }
 
 void launch_gs_exit_test(cudaStream_t s, const DevCloth& c, const SolverParams& P, int iter)
