@@ -481,8 +481,8 @@ def run_ours(args):
     algo = {
         # iterations x 144 B per FEM projection + bend iterations x 144 B per bend + velocity 48 B per vertex
         "gs_solve": it * 144 * T + ((it + 1) // 2) * 144 * B + 48 * N,
-        # per query: 2 endpoints x (pos, prev) 64 B + edge 16 B + count 4 B; 4 B per pair; tree read once
-        "ccd_broad_ee": E * 84 + 4 * ee_pairs + 32 * (2 * E - 1),
+        # per edge: 2 endpoints x (pos, prev) 64 B + edge 16 B, its box written and read 64 B; 8 B per pair
+        "ccd_broad_ee": E * 144 + 8 * ee_pairs,
         # per particle: pos + prev 32 B read, one 64 B contact slot written per collider hit (upper bound: one per particle)
         "colliders": 96 * N,
     }
@@ -491,13 +491,14 @@ def run_ours(args):
               2: f"k_gs_grid variant {ch[1]} ({ch[3]} threads, {ch[2]} CTAs/SM; one substep's Gauss-Seidel loop + velocity, one cooperative launch)",
               3: "k_fem / k_bends per colour (one substep's Gauss-Seidel loop)",
               4: f"k_gs_band ({ch[3]} threads per CTA, one {p.model.band_plan()[0]}-CTA cluster of particle bands; "
-                 f"one substep's Gauss-Seidel loop + velocity, one cluster launch)"}.get(ch[0], "solver")
+                 f"one substep's Gauss-Seidel loop + velocity, one cluster launch)",
+              5: "k_gs_tile (one substep's Gauss-Seidel loop + velocity, one launch; tiles exchange their particles "
+                 "between groups of colours)"}.get(ch[0], "solver")
     kernel_names = {"gs_solve": solver,
-                    "ccd_broad_ee": "k_bvh_refit + k_ccd_broad_ee + k_ccd_broad_coop (edge-edge swept-box LBVH "
-                                    "refit and query: one walk per lane, long lists one warp per query)",
+                    "ccd_broad_ee": "k_ccd_boxes + k_ccd_join (edge-edge swept boxes, their join in blocks of 32, and "
+                                    "the first part of the narrow phase)",
                     "colliders": "k_vertex_colliders (+ k_tri_colliders, k_edge_colliders when continuous collision is "
                                  "off: with it on they run on another branch, untimed)"}
-    walk, walk_ms = p.model.broad_phase_mode()
     per = {}
     for k in algo:
         tot, cnt = sections.get(k, (0.0, 0))
@@ -523,9 +524,7 @@ def run_ours(args):
                     "peak_source": peak_kind,
                     "sections": per,
                     "ccd_broad_vt_ms_per_launch": (sections["ccd_broad_vt"][0] / sections["ccd_broad_vt"][1]
-                                                   if sections.get("ccd_broad_vt", (0, 0))[1] else None),
-                    "broad_phase_walk": {"chosen": p.model.BROAD_WALKS[walk],
-                                         "tuned_ms": walk_ms.tolist()}}
+                                                   if sections.get("ccd_broad_vt", (0, 0))[1] else None)}
         if dom == "gs_solve" and ch[0] == 1:
             # the cluster solve is a chain of colour phases: its latency floor is the
             # phase count times the cost of one phase with no projection arithmetic

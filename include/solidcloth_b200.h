@@ -299,12 +299,9 @@ SCEXP void scSetBandVariant(scModel model, int variant);
    cluster (0: no plan), particles per band, halo particles, 1 if it is the
    solver in use}; returns 1 if the cloth has a plan. */
 SCEXP int scGetBandPlan(scModel model, int* out4);
-/* Continuous-collision broad phase walk (additions): 0 = one tree walk per query
-   (lane), 1 = warp packets (32 neighbouring queries walk together, broadcast
-   node loads), -1 (default) = timed at the first step and the faster kept. Same
-   candidate sets. Either walk stops a query at 128 candidates; those queries are
-   finished by a second pass, one warp per query. scGetBroadPhaseMode returns the
-   walk in use and, in ms2, the tuned times of both (ms per substep's detection). */
+/* Continuous-collision broad phase mode (additions): -1 (default), 0 and 1 are
+   accepted and give the same candidate sets; one kernel serves them all. The getter
+   returns the mode asked for (1 by default) and zeros in ms2: nothing is tuned. */
 SCEXP void scSetBroadPhaseMode(scModel model, int mode);
 SCEXP int scGetBroadPhaseMode(scModel model, float* ms2);
 /* info3 = {threads per CTA, FEM constraints per thread, bends per thread} per variant */

@@ -377,12 +377,12 @@ class ClothModel:
     BROAD_WALKS = ("per-query stack walk", "warp packet")
 
     def set_broad_phase_mode(self, mode: int):
-        """0 per-query walks, 1 warp packets, -1 tuned"""
+        """kept for callers: 0, 1 and -1 are accepted, one kernel serves them all"""
         lib().scSetBroadPhaseMode(self.h, int(mode))
         _check("scSetBroadPhaseMode")
 
     def broad_phase_mode(self):
-        """(walk in use, tuned ms of each walk in BROAD_WALKS order)"""
+        """(the mode asked for, zeros: nothing is tuned)"""
         ms = np.zeros(2, np.float32)
         mode = lib().scGetBroadPhaseMode(self.h, ms.ctypes.data_as(_f))
         return int(mode), ms.copy()

@@ -722,17 +722,15 @@ int scGetBandPlan(scModel m, int* out4)
 void scSetBroadPhaseMode(scModel m, int mode)
 {
     if (!M(m) || mode < -1 || mode >= BROAD_WALKS) { set_error(SC_ERR_ARG, "broad-phase mode must be -1, 0 or 1"); return; }
+    // one kernel serves every mode (k_ccd_join): the request is kept for the getter
     M(m)->broadMode = mode;
-    if (mode >= 0) { M(m)->broadWalk = mode; M(m)->buf.broadWalk = mode; }
-    M(m)->tuned = false;
-    M(m)->touch();
 }
 
 int scGetBroadPhaseMode(scModel m, float* ms2)
 {
     if (!M(m)) return -1;
-    if (ms2) for (int k = 0; k < BROAD_WALKS; k++) ms2[k] = M(m)->broadMs[k];
-    return M(m)->broadWalk;
+    if (ms2) for (int k = 0; k < BROAD_WALKS; k++) ms2[k] = 0.f;      // nothing is tuned
+    return M(m)->broadMode >= 0 ? M(m)->broadMode : BROAD_WALKS - 1;
 }
 
 int scGetGridVariants(int* info3, int cap)

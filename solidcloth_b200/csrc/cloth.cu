@@ -1493,37 +1493,16 @@ bool ClothModel::upload_topology(const HMesh& mesh)
     uint8_t* dborder = (uint8_t*)dalloc(N);
     SC_CUDA(cudaMemcpy(dborder, border.data(), N, cudaMemcpyHostToDevice));
     dc.vBorder = dborder;
+    if (!instV.empty())
     {
-        // query orders for the tree traversals: spatially adjacent queries share a
-        // warp, so its lanes walk the same subtrees (vertices and edge centroids by
-        // Morton code of the rest shape)
-        std::vector<V3> ec(E);
-        for (int e = 0; e < E; e++) ec[e] = 0.5f * (hpos[mesh.edges[e].i1] + hpos[mesh.edges[e].i2]);
-        std::vector<int> vq, eq;
-        if (instV.empty()) { vq = morton_order(hpos); eq = morton_order(ec); }
-        else
-        {
-            // a batch: instance after instance, Morton order inside each
-            for (size_t k = 0; k + 1 < instV.size(); k++)
-            {
-                for (int v : morton_order(std::vector<V3>(hpos.begin() + instV[k], hpos.begin() + instV[k + 1])))
-                    vq.push_back(v + instV[k]);
-                for (int e : morton_order(std::vector<V3>(ec.begin() + instE[k], ec.begin() + instE[k + 1])))
-                    eq.push_back(e + instE[k]);
-            }
-            std::vector<int> vi(N);
-            for (size_t k = 0; k + 1 < instV.size(); k++)
-                for (int v = instV[k]; v < instV[k + 1]; v++) vi[v] = (int)k;
-            int* dv = (int*)dalloc(sizeof(int) * ((size_t)N + instV.size()));
-            SC_CUDA(cudaMemcpy(dv, vi.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-            SC_CUDA(cudaMemcpy(dv + N, instV.data(), sizeof(int) * instV.size(), cudaMemcpyHostToDevice));
-            dc.vInst = dv;
-            dc.instStart = dv + N;
-        }
-        int* d = (int*)dalloc(sizeof(int) * ((size_t)N + E + 2));
-        SC_CUDA(cudaMemcpy(d, vq.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-        if (E) SC_CUDA(cudaMemcpy(d + N, eq.data(), sizeof(int) * E, cudaMemcpyHostToDevice));
-        dc.vQuery = d; dc.eQuery = d + N;
+        std::vector<int> vi(N);
+        for (size_t k = 0; k + 1 < instV.size(); k++)
+            for (int v = instV[k]; v < instV[k + 1]; v++) vi[v] = (int)k;
+        int* dv = (int*)dalloc(sizeof(int) * ((size_t)N + instV.size()));
+        SC_CUDA(cudaMemcpy(dv, vi.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
+        SC_CUDA(cudaMemcpy(dv + N, instV.data(), sizeof(int) * instV.size(), cudaMemcpyHostToDevice));
+        dc.vInst = dv;
+        dc.instStart = dv + N;
     }
     {
         // rest length of every edge from the uv layout (warm-start strain feature)
@@ -1593,22 +1572,6 @@ bool ClothModel::upload_topology(const HMesh& mesh)
         SC_CUDA(cudaMemcpy(out.lo, lo.data(), sizeof(float4) * h.numNodes, cudaMemcpyHostToDevice));
         SC_CUDA(cudaMemcpy(out.hi, hi.data(), sizeof(float4) * h.numNodes, cudaMemcpyHostToDevice));
         out.visit = (int*)dalloc(sizeof(int) * h.numNodes);
-        // child records: static link and maximum words (the refit fills the boxes)
-        std::vector<float4> rec(4 * (size_t)h.numNodes, make_float4(0.f, 0.f, 0.f, 0.f));
-        for (int k = 0; k < h.numNodes; k++)
-        {
-            if (h.child[k] < 0) continue;
-            const int side[2] = {k + 1, h.child[k]};
-            for (int j = 0; j < 2; j++)
-            {
-                const int ch = side[j];
-                const int link = h.child[ch] < 0 ? h.child[ch] : ch;
-                rec[4 * (size_t)k + 2 * j + 1].z = bits_f((uint32_t)link);
-                rec[4 * (size_t)k + 2 * j + 1].w = bits_f((uint32_t)h.maxPrim[ch]);
-            }
-        }
-        out.rec = (float4*)dalloc(sizeof(float4) * rec.size());
-        SC_CUDA(cudaMemcpy(out.rec, rec.data(), sizeof(float4) * rec.size(), cudaMemcpyHostToDevice));
         return true;
     };
     // batch: one tree per instance over its own primitives [start[k], start[k+1]),
@@ -1639,26 +1602,10 @@ bool ClothModel::upload_topology(const HMesh& mesh)
         }
         return upload_bvh(all, out, &roots);
     };
-    // a tree over cen, or (shareTopo) a second set of boxes over another tree's topology
-    auto mkbvh = [&](const std::vector<V3>& cen, DevBVH& out, DevBVH* shareTopo) -> bool {
-        if (!shareTopo)
-        {
-            LBVHHost h;
-            h.build(cen);
-            return upload_bvh(h, out, nullptr);
-        }
-        out = *shareTopo;
-        std::vector<float4> lo(out.numNodes), hi(out.numNodes);
-        SC_CUDA(cudaMemcpy(lo.data(), shareTopo->lo, sizeof(float4) * out.numNodes, cudaMemcpyDeviceToHost));
-        SC_CUDA(cudaMemcpy(hi.data(), shareTopo->hi, sizeof(float4) * out.numNodes, cudaMemcpyDeviceToHost));
-        out.lo = (float4*)dalloc(sizeof(float4) * out.numNodes);
-        out.hi = (float4*)dalloc(sizeof(float4) * out.numNodes);
-        SC_CUDA(cudaMemcpy(out.lo, lo.data(), sizeof(float4) * out.numNodes, cudaMemcpyHostToDevice));
-        SC_CUDA(cudaMemcpy(out.hi, hi.data(), sizeof(float4) * out.numNodes, cudaMemcpyHostToDevice));
-        out.visit = (int*)dalloc(sizeof(int) * out.numNodes);
-        out.rec = (float4*)dalloc(sizeof(float4) * 4 * (size_t)out.numNodes);
-        SC_CUDA(cudaMemcpy(out.rec, shareTopo->rec, sizeof(float4) * 4 * (size_t)out.numNodes, cudaMemcpyDeviceToDevice));
-        return true;
+    auto mkbvh = [&](const std::vector<V3>& cen, DevBVH& out) -> bool {
+        LBVHHost h;
+        h.build(cen);
+        return upload_bvh(h, out, nullptr);
     };
     std::vector<V3> tc(T), ec(E);
     for (int t = 0; t < T; t++)
@@ -1666,16 +1613,75 @@ bool ClothModel::upload_topology(const HMesh& mesh)
     for (int e = 0; e < E; e++) ec[e] = 0.5f * (hpos[mesh.edges[e].i1] + hpos[mesh.edges[e].i2]);
     if (instV.empty())
     {
-        if (!mkbvh(tc, triBvh, nullptr)) return false;
-        if (!mkbvh(ec, edgeBvh, nullptr)) return false;
+        if (!mkbvh(tc, triBvh)) return false;
+        if (!mkbvh(ec, edgeBvh)) return false;
     }
     else
     {
         if (!mkforest(tc, instT, triBvh)) return false;
         if (!mkforest(ec, instE, edgeBvh)) return false;
     }
-    if (!mkbvh(tc, sweptTriBvh, &triBvh)) return false;
-    if (!mkbvh(ec, sweptEdgeBvh, &edgeBvh)) return false;
+    // the continuous broad phase's boxes: spatial order per instance, in blocks of 32
+    // (vertices) or groups of 1,024 (triangles, edges) that do not cross instances
+    auto spatial = [&](const std::vector<V3>& cen, const std::vector<int>& start, int unit, std::vector<int>& out, std::vector<int2>& range) {
+        for (size_t k = 0; k + 1 < start.size(); k++)
+        {
+            const int first = (int)(out.size() / unit);
+            for (int x : morton_order(std::vector<V3>(cen.begin() + start[k], cen.begin() + start[k + 1]))) out.push_back(x + start[k]);
+            out.resize((out.size() + unit - 1) / unit * unit, -1);
+            range.push_back(make_int2(first, (int)(out.size() / unit) - first));
+        }
+    };
+    auto upload = [&](const void* h, size_t bytes) -> void* {
+        void* d = dalloc(bytes);
+        if (d && bytes && cudaMemcpy(d, h, bytes, cudaMemcpyHostToDevice) != cudaSuccess) d = nullptr;
+        return d;
+    };
+    auto owners = [](const std::vector<int2>& range) {
+        std::vector<int> of;
+        for (size_t k = 0; k < range.size(); k++) of.insert(of.end(), range[k].y, (int)k);
+        return of;
+    };
+    auto mkset = [&](const std::vector<V3>& cen, const std::vector<int>& inst, auto ends, BoxSet& out) -> bool {
+        std::vector<int> prim;
+        std::vector<int2> range;
+        spatial(cen, inst.empty() ? std::vector<int>{0, (int)cen.size()} : inst, 1024, prim, range);
+        out = BoxSet{};
+        out.nGroups = (int)(prim.size() / 1024);
+        const size_t G = (size_t)out.nGroups;
+        std::vector<int4> en(prim.size(), make_int4(-1, -1, -1, -1));
+        for (size_t k = 0; k < prim.size(); k++) if (prim[k] >= 0) en[k] = ends(prim[k]);
+        out.prim = (int*)upload(prim.data(), sizeof(int) * prim.size());
+        out.ends = (int4*)upload(en.data(), sizeof(int4) * en.size());
+        float4* box = (float4*)dalloc(sizeof(float4) * 2 * (1024 + 32 + 1) * G);
+        if (!out.prim || !out.ends || !box) return false;
+        out.lo = box; out.hi = box + 1024 * G;
+        out.blo = box + 2048 * G; out.bhi = out.blo + 32 * G;
+        out.glo = out.bhi + 32 * G; out.ghi = out.glo + G;
+        if (inst.empty()) return true;
+        const std::vector<int> of = owners(range);
+        out.inst = (int2*)upload(range.data(), sizeof(int2) * range.size());
+        out.groupInst = (int*)upload(of.data(), sizeof(int) * of.size());
+        return out.inst && out.groupInst;
+    };
+    auto triEnds = [&](int t) { return make_int4((int)mesh.idx[3 * t], (int)mesh.idx[3 * t + 1], (int)mesh.idx[3 * t + 2], -1); };
+    auto edgeEnds = [&](int e) { return make_int4((int)mesh.edges[e].i1, (int)mesh.edges[e].i2, -1, -1); };
+    if (!mkset(tc, instT, triEnds, sweptTris) || !mkset(ec, instE, edgeEnds, sweptEdges)) return false;
+    {
+        std::vector<int> vertex;
+        std::vector<int2> range;
+        spatial(hpos, instV.empty() ? std::vector<int>{0, N} : instV, 32, vertex, range);
+        sweptVerts = VertexBlocks{};
+        sweptVerts.nBlocks = (int)(vertex.size() / 32);
+        sweptVerts.vertex = (int*)upload(vertex.data(), sizeof(int) * vertex.size());
+        if (!sweptVerts.vertex) return false;
+        if (!instV.empty())
+        {
+            const std::vector<int> of = owners(range);
+            sweptVerts.blockInst = (int*)upload(of.data(), sizeof(int) * of.size());
+            if (!sweptVerts.blockInst) return false;
+        }
+    }
     bufWorldVersion = ~0ull;
     return true;
 }
@@ -1865,27 +1871,20 @@ bool ClothModel::ensure_buffers(const CollisionWorld& world, cudaStream_t s)
     buf.seFlag = (int*)dalloc(sizeof(int) * E, true);
     buf.seSlot = (SCt*)dalloc(sizeof(SCt) * (size_t)E, true);
     buf.seList = (SCt*)dalloc(sizeof(SCt) * (size_t)buf.seCap, true);
-    buf.ccdVtCnt = (int*)dalloc(sizeof(int) * N, true);
-    buf.ccdEeCnt = (int*)dalloc(sizeof(int) * E, true);
-    buf.ccdVtCand = (int*)dalloc(sizeof(int) * (size_t)(ccd ? N * KCCD : 1), true);
-    buf.ccdEeCand = (int*)dalloc(sizeof(int) * (size_t)(ccd ? E * KCCD : 1), true);
     buf.ccdVtPairs = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdVtCap, true);
     buf.ccdEePairs = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdEeCap, true);
-    buf.ccdVtHit = (uint8_t*)dalloc((size_t)buf.ccdVtCap, true);
-    buf.ccdEeHit = (uint8_t*)dalloc((size_t)buf.ccdEeCap, true);
-    buf.ccdVtOff = (int*)dalloc(sizeof(int) * N, true);
-    buf.ccdEeOff = (int*)dalloc(sizeof(int) * E, true);
+    buf.ccdVtTest = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdVtCap, true);
+    buf.ccdEeTest = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdEeCap, true);
+    buf.ccdVtTestCount = counts + 9; buf.ccdEeTestCount = counts + 10;
+    buf.ccdVtHitCap = ccd ? N * CCD_VT_HITS : 1;
+    buf.ccdEeHitCap = ccd ? E * CCD_EE_HITS : 1;
+    buf.ccdVtHits = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdVtHitCap, true);
+    buf.ccdEeHits = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdEeHitCap, true);
+    buf.ccdVtSorted = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdVtHitCap, true);
+    buf.ccdEeSorted = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdEeHitCap, true);
+    buf.ccdVtHitTotal = counts + 6; buf.ccdEeHitTotal = counts + 7;
     buf.ccdVtHitCnt = (int*)dalloc(sizeof(int) * N, true);
     buf.ccdEeHitCnt = (int*)dalloc(sizeof(int) * E, true);
-    buf.ccdVtPoolOff = (int*)dalloc(sizeof(int) * N, true);
-    buf.ccdEePoolOff = (int*)dalloc(sizeof(int) * E, true);
-    buf.ccdPoolCap = ccd ? std::max(buf.ccdEeCap, std::max(N, E) * KCCD / 2) : 1;
-    buf.ccdPool = (int*)dalloc(sizeof(int) * (size_t)buf.ccdPoolCap, true);
-    buf.ccdPoolUsed = counts + 6;
-    buf.ccdVtOvf = (int*)dalloc(sizeof(int) * (size_t)(ccd ? N : 1), true);
-    buf.ccdEeOvf = (int*)dalloc(sizeof(int) * (size_t)(ccd ? E : 1), true);
-    buf.ccdOvfN = (int*)dalloc(sizeof(int) * 2, true);
-    if (ccd) ccd_kernel_setup();
     // colouring
     buf.vmin = (unsigned long long*)dalloc(sizeof(unsigned long long) * N, true);
     SC_CUDA(cudaMemset(buf.vmin, 0xff, sizeof(unsigned long long) * N));
@@ -1899,7 +1898,6 @@ bool ClothModel::ensure_buffers(const CollisionWorld& world, cudaStream_t s)
     buf.scanBlock = (int*)dalloc(sizeof(int) * (maxScan / 1024 + 8), true);
     buf.scanBlock2 = (int*)dalloc(sizeof(int) * (maxScan / 1024 + 8), true);
     buf.scanOff2 = (int*)dalloc(sizeof(int) * (maxScan + 1), true);
-    buf.broadWalk = broadWalk;
     bufWorldVersion = world.version;
     bufFlags = prm.flags;
     bufCcd = ccd;
@@ -2346,9 +2344,9 @@ void ClothPatch::record_substep(float h)
                 marks[2] = timingCapture[k + 2 * SEC_BROAD_VT]; marks[3] = timingCapture[k + 2 * SEC_BROAD_VT + 1];
             }
         }
-        launch_ccd(s, side, evFork, evJoin, c, P, b, m.sweptTriBvh, m.sweptEdgeBvh, marks);
+        launch_ccd(s, side, evFork, evJoin, c, P, b, m.sweptTris, m.sweptEdges, m.sweptVerts, marks);
     }
-    if (self || ccd) launch_compact_self(s, side, evFork, evJoin, c, P, b, self, ccd);
+    if (self || ccd) launch_compact_self(s, c, P, b, self, ccd);
     else cudaMemsetAsync(b.stCount, 0, 2 * sizeof(int), s);
     launch_colour_contacts(s, c, b);
     // learned warm start (no reference counterpart): record the features and the
@@ -2502,8 +2500,8 @@ bool ClothPatch::autotune(float h)
     const SolverParams P = m.solver_params(h);
     std::vector<int> key = {m.N, m.dc.T, m.dc.B, m.prm.iterations, m.prm.dihedral, m.prm.fem, m.prm.fixedIterations,
                             (int)m.buf.numVColl, m.prm.bendFreq, (int)m.prm.stageRecords, m.solverMode,
-                            (int)m.prm.ccd, m.broadMode, (int)m.prm.fastMath, (int)m.band_active(),
-                            m.bandPlan.clusterSize, m.bandPlan.halo};
+                            (int)m.prm.ccd, (int)m.prm.fastMath, (int)m.band_active(),
+                            m.bandPlan.clusterSize, m.bandPlan.halo, (int)m.tilePlan.valid};
     key.insert(key.end(), m.triColourStart.begin(), m.triColourStart.end());
     key.insert(key.end(), m.bendColourStart.begin(), m.bendColourStart.end());
     {
@@ -2512,8 +2510,6 @@ bool ClothPatch::autotune(float h)
             if (kv.first == key)
             {
                 m.choice = kv.second;
-                m.broadWalk = m.broadMode >= 0 ? m.broadMode : kv.second.broad;
-                m.buf.broadWalk = m.broadWalk;
                 m.tuned = true;
                 return true;
             }
@@ -2589,43 +2585,6 @@ bool ClothPatch::autotune(float h)
     cudaStreamSynchronize(stream);
     cudaFree(backup);
     m.tuneLog = cand;
-    m.choice = best;
-    // continuous broad phase: the first-pass walks (BROAD_*; same pair sets), timed
-    // on this cloth's current state (the detection changes no particle)
-    if (m.prm.ccd && m.buf.ccdVtCnt)
-    {
-        for (int mode = 0; mode < BROAD_WALKS; mode++)
-        {
-            m.buf.broadWalk = mode;
-            m.broadMs[mode] = 1e30f;
-            cudaGraph_t g = nullptr;
-            cudaGraphExec_t ge = nullptr;
-            if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) continue;
-            launch_ccd(stream, side, evFork, evJoin, m.dc, P, m.buf, m.sweptTriBvh, m.sweptEdgeBvh);
-            if (cudaStreamEndCapture(stream, &g) != cudaSuccess || cudaGraphInstantiate(&ge, g, 0) != cudaSuccess)
-            {
-                if (g) cudaGraphDestroy(g);
-                cudaGetLastError();
-                continue;
-            }
-            cudaGraphDestroy(g);
-            cudaGraphLaunch(ge, stream);
-            cudaEventRecord(e0, stream);
-            for (int r = 0; r < 3; r++) cudaGraphLaunch(ge, stream);
-            cudaEventRecord(e1, stream);
-            float ms = 0.f;
-            if (cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess)
-                m.broadMs[mode] = ms / 3;
-            cudaGetLastError();
-            cudaGraphExecDestroy(ge);
-        }
-        m.broadWalk = 0;
-        for (int mode = 1; mode < BROAD_WALKS; mode++)
-            if (m.broadMs[mode] < m.broadMs[m.broadWalk]) m.broadWalk = mode;
-    }
-    if (m.broadMode >= 0) m.broadWalk = m.broadMode;
-    m.buf.broadWalk = m.broadWalk;
-    best.broad = m.broadWalk;
     m.choice = best;
     cudaEventDestroy(e0); cudaEventDestroy(e1);
     m.tuned = true;

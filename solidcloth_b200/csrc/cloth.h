@@ -111,7 +111,7 @@ struct BatchColl { std::shared_ptr<Collidable> coll; int vBegin, vCount, inst; }
 
 // solver selection (autotuned unless forced)
 enum SolverKind { SOLVE_AUTO = 0, SOLVE_CLUSTER = 1, SOLVE_GRID = 2, SOLVE_KERNELS = 3, SOLVE_BAND = 4, SOLVE_TILE = 5 };
-struct SolverChoice { int kind, variant, blocksPerSm; float ms; int broad; };
+struct SolverChoice { int kind, variant, blocksPerSm; float ms; };
 
 struct FemHost { uint32_t i1, i2, i3; float du1, du2, dv1, dv2, det, invDet, lu0, lv0, su, sv, lu2, lv2, area; };
 
@@ -157,7 +157,9 @@ public:
     int device = -1;
     std::vector<void*> allocs;
     DevCloth dc{};
-    DevBVH triBvh{}, edgeBvh{}, sweptTriBvh{}, sweptEdgeBvh{};
+    DevBVH triBvh{}, edgeBvh{};
+    BoxSet sweptTris{}, sweptEdges{};
+    VertexBlocks sweptVerts{};
     Buffers buf{};
     std::vector<VColl> vcollHost;
     std::vector<void*> bufAllocs;
@@ -195,9 +197,7 @@ public:
     bool tuned = false;
     uint64_t tunedVersion = 0;
     std::vector<SolverChoice> tuneLog;          // candidates and their times of the last tuning
-    int broadWalk = 0;                          // tuned: continuous broad phase first-pass walk (BROAD_*)
-    int broadMode = -1;                         // forced walk (BROAD_*) or -1: tuned
-    float broadMs[BROAD_WALKS] = {};            // tuned times of the broad-phase walks
+    int broadMode = -1;                         // what scSetBroadPhaseMode asked for
     void colour_constraints();
     void touch() { paramVersion++; }
 

@@ -7,12 +7,7 @@ namespace sc {
 constexpr int KVT = 48;        // self vertex-triangle contact slots per vertex
 constexpr int KCAND = 256;     // BVH candidates kept per proximity query
 constexpr int KRES = 96;       // distinct features tracked per vertex for the dedup
-constexpr int KADJ = 16;       // adjacent primitives held in registers by a broad-phase query
-constexpr int KCCD = 128;      // continuous-collision candidates kept in a query's own slots
-// second broad-phase pass: warps per block, blocks, stack entries per depth level
-constexpr int CCD_COOP_THREADS = 128, CCD_COOP_BLOCKS = 4 * 148, CCD_COOP_GROUP = 64;
-// first-pass walks: one query per lane, or warp packets
-enum { BROAD_LANE = 0, BROAD_PACKET = 1, BROAD_WALKS = 2 };
+constexpr int BROAD_WALKS = 2; // broad-phase modes callers may name (one kernel serves both)
 constexpr int CCD_VT_PAIRS = 128, CCD_EE_PAIRS = 96; // pair store per vertex / edge
 constexpr int CCD_VT_HITS = 32, CCD_EE_HITS = 16;   // continuous contacts per vertex / edge
 constexpr int MAX_COLOURS = 128; // independent-set colouring rounds per contact class
@@ -50,22 +45,19 @@ struct Buffers
     int numVColl;
     const VColl* vcoll;       // device copy
     const int2* instColl;     // batch: (first collider, count) per instance; null: all colliders act on all
-    int broadWalk;            // continuous broad phase first-pass walk (BROAD_*, tuned)
     // triangle / edge contacts: per-collider slot arrays, flags, dense lists
     TC* tcSlot; int* tcFlag; TC* tcList; int* tcCount; int tcCap;
     EC* ecSlot; int* ecFlag; EC* ecList; int* ecCount; int ecCap;
     // self contacts
     int* stCnt; SCt* stSlot; SCt* stList; int* stCount; int stCap;
     int* seFlag; SCt* seSlot; SCt* seList; int* seCount; int seCap;
-    // continuous collision
-    int* ccdVtCnt; int* ccdVtCand; int* ccdEeCnt; int* ccdEeCand;
+    // continuous collision: candidate pairs (query, candidate), those left to the full
+    // test, and the hits among them with each query's number of hits
     int2* ccdVtPairs; int2* ccdEePairs; int* ccdVtPairCount; int* ccdEePairCount; int ccdVtCap, ccdEeCap;
-    uint8_t* ccdVtHit; uint8_t* ccdEeHit;  // per pair: 1 if the narrow phase reports a contact
-    int* ccdVtOff; int* ccdEeOff;          // first pair of each query
-    int* ccdVtHitCnt; int* ccdEeHitCnt;    // hits per query
-    int* ccdPool; int ccdPoolCap; int* ccdPoolUsed;  // candidate lists longer than KCCD
-    int* ccdVtPoolOff; int* ccdEePoolOff;
-    int* ccdVtOvf; int* ccdEeOvf; int* ccdOvfN;      // queries with more than KCCD candidates; counts (vt, ee)
+    int2* ccdVtTest; int2* ccdEeTest; int* ccdVtTestCount; int* ccdEeTestCount;
+    int2* ccdVtHits; int2* ccdEeHits; int* ccdVtHitTotal; int* ccdEeHitTotal; int ccdVtHitCap, ccdEeHitCap;
+    int* ccdVtHitCnt; int* ccdEeHitCnt;
+    int2* ccdVtSorted; int2* ccdEeSorted;
     // colouring scratch
     unsigned long long* vmin;  // N, kept at ~0
     int* colour; int* order; int* colourStart; int colourCap;
@@ -94,25 +86,22 @@ void launch_solve_vertex_contacts(cudaStream_t s, const DevCloth& c, const Solve
 void launch_solve_multi_contacts(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, int iter);
 void launch_colour_contacts(cudaStream_t s, const DevCloth& c, const Buffers& b);
 void launch_bvh_refit(cudaStream_t s, const DevBVH& bvh, const DevCloth& c, int kind, float tol);
-size_t ccd_coop_smem(int depth);      // dynamic shared memory of the second broad-phase pass
 // microseconds a phase of the cluster solver's barrier structure costs (kind 0:
 // barrier only; 1: plus one distributed-shared-memory read and write), -1 if no
 // cluster of the solver's size fits
 float probe_cluster_phase(int kind, int phases);
-void ccd_kernel_setup();              // kernel attributes (once per device, outside capture)
 void launch_self_proximity(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b,
                            const DevBVH& triBvh, const DevBVH& edgeBvh);
-// swept-tree refits + continuous-collision broad and narrow phases; the
-// vertex-triangle half runs on `side` (forked from / joined to s by the events);
-// marks (optional, entries may be null): records around the edge-edge and the
-// vertex-triangle broad phases {ee start, ee end, vt start, vt end}
+// swept boxes + continuous-collision broad and narrow phases; the vertex-triangle
+// half runs on `side` (forked from / joined to s by the events); marks (optional,
+// entries may be null): records around the edge-edge and the vertex-triangle
+// halves {ee start, ee end, vt start, vt end}
 void launch_ccd(cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, const DevCloth& c,
-                const SolverParams& P, const Buffers& b, const DevBVH& triBvh, const DevBVH& edgeBvh,
+                const SolverParams& P, const Buffers& b, const BoxSet& tris, const BoxSet& edges, const VertexBlocks& verts,
                 const cudaEvent_t* marks = nullptr);
 // self-contact lists: proximity contacts (self) compacted, then the continuous
-// hits appended (ccd; vertex-triangle on `side` between fork and join)
-void launch_compact_self(cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, const DevCloth& c,
-                         const SolverParams& P, const Buffers& b, bool self, bool ccd);
+// hits appended (ccd)
+void launch_compact_self(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, bool self, bool ccd);
 struct TileView;
 // clears the solver's error and exit words; with a tile plan also its exchange tags
 void launch_reset_gs(cudaStream_t s, const DevCloth& c, const TileView* tv = nullptr);

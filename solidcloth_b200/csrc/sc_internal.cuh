@@ -70,8 +70,6 @@ struct DevCloth
     float4* xsnap;              // N: positions at the start of the current iteration (update residual)
     float4* xpred;              // N: positions after the substep's prediction (warm start / samples)
     float* lastCorr;            // N: last substep's solver correction along the collision normal
-    const int* vQuery;          // N: vertices in spatial (Morton, rest shape) order: neighbouring
-    const int* eQuery;          // E: edges likewise; queries of one warp walk the same subtrees
     float4* prevN;              // collision mesh vertex normals (refreshed per frame)
     float4* prevTriN;           // collision mesh triangle normals
     float4* meshN;              // render mesh normals
@@ -100,8 +98,33 @@ struct DevBVH
     const int* instRoot;    // batch: root node of each instance's tree (a forest); null: one tree at 0
     float4* lo;             // numNodes: box min; w = child[] as int bits
     float4* hi;             // numNodes: box max; w = escape[] as int bits
-    float4* rec;            // numNodes x 4: an internal node's two child records (box, link, max primitive)
     int* visit;             // numNodes refit counters
+};
+
+// Swept boxes of the continuous broad phase in three levels: the primitives in
+// spatial (Morton, rest shape) order, blocks of 32 of them, groups of 32 blocks.
+// Every instance of a batch starts a group; unused places hold primitive -1 and a
+// box that overlaps nothing. Fixed order, boxes rebuilt every substep.
+struct BoxSet
+{
+    int nGroups;            // 1024 places each
+    const int* prim;        // primitive of each place
+    const int4* ends;       // its particles (two of an edge, three of a triangle)
+    float4* lo;             // place: box min; w = primitive (as bits)
+    float4* hi;             // place: box max
+    float4* blo;            // block boxes
+    float4* bhi;
+    float4* glo;            // group boxes
+    float4* ghi;
+    const int2* inst;       // batch: (first group, groups) of each instance; null: one cloth
+    const int* groupInst;   // batch: instance of each group
+};
+// vertices in the same spatial order, in blocks of 32 that do not cross instances
+struct VertexBlocks
+{
+    int nBlocks;
+    const int* vertex;      // nBlocks * 32, -1: none
+    const int* blockInst;   // batch: instance of each block
 };
 
 // Static collider tree, identical to Geometry::ComputeMeshTree's, flattened.

@@ -997,15 +997,6 @@ __device__ __forceinline__ Box leaf_box(const DevCloth& c, int kind, int prim, f
 // sibling's visible), the arriving thread keeps its own box in registers and
 // loads only the sibling's, and it puts the counter back to zero for the next
 // refit (counters start at zero when the tree is allocated).
-// a child's box into its half of the parent's record (the link and maximum
-// words after it are static)
-__device__ __forceinline__ void store_child_box(float4* rec, int parent, int node, const Box& b)
-{
-    float4* h = rec + 4 * (size_t)parent + (node == parent + 1 ? 0 : 2);
-    h[0] = make_float4(b.lo.x, b.lo.y, b.lo.z, b.hi.x);
-    *reinterpret_cast<float2*>(h + 1) = make_float2(b.hi.y, b.hi.z);
-}
-
 __global__ void k_bvh_refit(DevBVH t, DevCloth c, int kind, float tol)
 {
     int prim = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1015,7 +1006,6 @@ __global__ void k_bvh_refit(DevBVH t, DevCloth c, int kind, float tol)
     t.lo[node] = f4(b.lo, __int_as_float(~prim));
     t.hi[node] = f4(b.hi, __int_as_float(node + 1));
     int p = t.parent[node];
-    if (p >= 0) store_child_box(t.rec, p, node, b);
     while (p >= 0)
     {
         cuda::atomic_ref<int, cuda::thread_scope_device> visit(t.visit[p]);
@@ -1033,10 +1023,8 @@ __global__ void k_bvh_refit(DevBVH t, DevCloth c, int kind, float tol)
         b = m;
         t.lo[p] = f4(b.lo, __int_as_float(r));
         t.hi[p] = f4(b.hi, __int_as_float(t.escape[p]));
-        const int gp = t.parent[p];
-        if (gp >= 0) store_child_box(t.rec, gp, p, b);
         node = p;
-        p = gp;
+        p = t.parent[p];
     }
 }
 
@@ -1063,191 +1051,6 @@ __device__ __forceinline__ void bvh_query(const DevBVH& t, const Box& q, F&& f, 
         }
         else node = esc;
     }
-}
-
-// Child records: every internal node keeps, for each of its two children, one
-// 32-byte half with the child's box, its link (node index, or ~primitive for a
-// leaf) and the largest primitive index below it, so one step of a walk is two
-// 256-bit loads from one 64-byte record (the refit writes the boxes, the links
-// and maxima are static).
-struct ChildRec { float lx, ly, lz, hx, hy, hz; int link, maxPrim; };
-
-__device__ __forceinline__ ChildRec ld_child(const float4* rec, int node, int side)
-{
-    const float* a = reinterpret_cast<const float*>(rec + 4 * (size_t)node + 2 * side);
-    float v[8];
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-        : "l"(a));
-    ChildRec r;
-    r.lx = v[0]; r.ly = v[1]; r.lz = v[2]; r.hx = v[3]; r.hy = v[4]; r.hz = v[5];
-    r.link = __float_as_int(v[6]); r.maxPrim = __float_as_int(v[7]);
-    return r;
-}
-
-__device__ __forceinline__ bool overlaps(const ChildRec& c, const Box& q)
-{
-    return !(c.hx < q.lo.x || c.hy < q.lo.y || c.hz < q.lo.z || q.hi.x < c.lx || q.hi.y < c.ly || q.hi.z < c.lz);
-}
-
-// Per-thread traversal that tests both children of an entered node in one round
-// trip (the node's two child records) and keeps the second one on a short stack:
-// the dependent-load chain is the number of entered internal nodes, about a
-// third of the stackless walk's. Reports the same leaf set as bvh_query, in a
-// different order. A median-split tree over n < 2^31 leaves is at most 31 deep,
-// so the 32-entry stack cannot overflow. A walk ends early once *stop is set
-// (by f).
-template <typename F>
-__device__ __forceinline__ void bvh_query2(const DevBVH& t, const Box& q, bool active, F&& f, int above = -1, int root = 0,
-                                           const bool* stop = nullptr)
-{
-    if (!active || t.numNodes == 0) return;
-    const float4 rlo = __ldg(&t.lo[root]), rhi = __ldg(&t.hi[root]);
-    const bool rootHit = !(rhi.x < q.lo.x || rhi.y < q.lo.y || rhi.z < q.lo.z || q.hi.x < rlo.x || q.hi.y < rlo.y ||
-                           q.hi.z < rlo.z);
-    if (!rootHit || (above >= 0 && __ldg(&t.maxPrim[root]) <= above)) return;
-    if (__float_as_int(rlo.w) < 0) { f(~__float_as_int(rlo.w)); return; }
-    int stack[32];
-    int sp = 0;
-    int node = root;
-    while (!(stop && *stop))
-    {
-        const ChildRec cl = ld_child(t.rec, node, 0), cr = ld_child(t.rec, node, 1);
-        bool oL = overlaps(cl, q) && (above < 0 || cl.maxPrim > above);
-        bool oR = overlaps(cr, q) && (above < 0 || cr.maxPrim > above);
-        if (oL && cl.link < 0) { f(~cl.link); oL = false; }
-        if (oR && cr.link < 0) { f(~cr.link); oR = false; }
-        if (oL)
-        {
-            if (oR && sp < 32) stack[sp++] = cr.link;
-            node = cl.link;
-        }
-        else if (oR) node = cr.link;
-        else
-        {
-            if (sp == 0) break;
-            node = stack[--sp];
-        }
-    }
-}
-
-// Warp-packet form of bvh_query2: the 32 lanes (spatially adjacent queries in
-// the same tree) walk it together, testing both children of an entered node per
-// step; a child is entered when any lane's box overlaps it (ballot), so every
-// record load is one broadcast request instead of up to 32 scattered ones, at
-// the price of visiting the union of the lanes' nodes. Each lane reports exactly
-// its own leaves. All 32 lanes must call it; a warp whose lanes start in
-// different trees (a batch instance boundary) takes the per-lane walk. A lane
-// whose *stop is set (by f) stops reporting and no longer steers the walk.
-template <typename F>
-__device__ __forceinline__ void bvh_query2_warp(const DevBVH& t, const Box& q, bool active, F&& f, int above, int root,
-                                                const bool* stop = nullptr)
-{
-    const unsigned full = 0xffffffffu;
-    const unsigned act = __ballot_sync(full, active);
-    if (!act) return;
-    const int r0 = __shfl_sync(full, root, __ffs(act) - 1);
-    if (!__all_sync(full, !active || root == r0)) { bvh_query2(t, q, active, f, above, root, stop); return; }
-    const float4 rlo = __ldg(&t.lo[r0]), rhi = __ldg(&t.hi[r0]);
-    const bool rootHit = active &&
-                         !(rhi.x < q.lo.x || rhi.y < q.lo.y || rhi.z < q.lo.z || q.hi.x < rlo.x || q.hi.y < rlo.y ||
-                           q.hi.z < rlo.z) &&
-                         (above < 0 || __ldg(&t.maxPrim[r0]) > above);
-    if (__float_as_int(rlo.w) < 0) { if (rootHit) f(~__float_as_int(rlo.w)); return; }
-    if (!__any_sync(full, rootHit)) return;
-    int stack[32];
-    int sp = 0;
-    int node = r0;
-    while (true)
-    {
-        const ChildRec cl = ld_child(t.rec, node, 0), cr = ld_child(t.rec, node, 1);
-        const bool live = active && !(stop && *stop);
-        bool oL = live && overlaps(cl, q) && (above < 0 || cl.maxPrim > above);
-        bool oR = live && overlaps(cr, q) && (above < 0 || cr.maxPrim > above);
-        if (cl.link < 0) { if (oL) f(~cl.link); oL = false; }
-        if (cr.link < 0) { if (oR) f(~cr.link); oR = false; }
-        const bool anyL = __any_sync(full, oL), anyR = __any_sync(full, oR);
-        if (anyL)
-        {
-            if (anyR && sp < 32) stack[sp++] = cr.link;
-            node = cl.link;
-        }
-        else if (anyR) node = cr.link;
-        else
-        {
-            if (sp == 0) break;
-            node = stack[--sp];
-        }
-    }
-}
-
-// Cooperative walk of ONE query box by a group of W lanes (W a power of two up
-// to 32; every lane of the group holds the same box), for queries with long
-// candidate lists: each step the group takes up to W entered nodes from its
-// stack, each lane tests both children of its node (one round trip), and the
-// entered internal children are pushed as a new group. Only the top group is
-// ever popped, so group g holds nodes of depth g exactly: at most depth groups
-// of at most 2W entries, the bound the caller sizes the stack (node indices)
-// by. f(a, b) is called by all lanes of the group once per step with the lane's
-// overlapping leaves (-1 for none) and returns false to end the walk (uniformly
-// across the group). The leaf set is bvh_query2's.
-template <int W, typename F>
-__device__ __forceinline__ void bvh_query_coop(const DevBVH& t, const Box& q, int above, int root, int* stack, int cap,
-                                               int* groups, int gcap, int* status, F&& f)
-{
-    const int lane = threadIdx.x & 31, sl = lane & (W - 1);
-    const unsigned mask = W == 32 ? 0xffffffffu : (((1u << W) - 1u) << (lane & ~(W - 1)));
-    const unsigned lt = (1u << lane) - 1u;
-    const float4 rlo = __ldg(&t.lo[root]), rhi = __ldg(&t.hi[root]);
-    const bool rootHit = !(rhi.x < q.lo.x || rhi.y < q.lo.y || rhi.z < q.lo.z || q.hi.x < rlo.x || q.hi.y < rlo.y ||
-                           q.hi.z < rlo.z);
-    if (!rootHit || (above >= 0 && __ldg(&t.maxPrim[root]) <= above)) return;
-    const int rch = __float_as_int(rlo.w);
-    if (rch < 0) { f(sl == 0 ? ~rch : -1, -1); return; }
-    if (sl == 0) { stack[0] = root; groups[0] = 1; }
-    int sp = 1, m = 1;
-    __syncwarp(mask);
-    while (m > 0)
-    {
-        const int g = groups[m - 1];
-        const int take = min(g, W);
-        const int node = sl < take ? stack[sp - 1 - sl] : -1;
-        __syncwarp(mask);
-        sp -= take;
-        int leafA = -1, leafB = -1, linkL = 0, linkR = 0;
-        bool pushL = false, pushR = false;
-        if (node >= 0)
-        {
-            const ChildRec cl = ld_child(t.rec, node, 0), cr = ld_child(t.rec, node, 1);
-            const bool oL = overlaps(cl, q) && (above < 0 || cl.maxPrim > above);
-            const bool oR = overlaps(cr, q) && (above < 0 || cr.maxPrim > above);
-            linkL = cl.link;
-            linkR = cr.link;
-            if (oL) { if (linkL < 0) leafA = ~linkL; else pushL = true; }
-            if (oR) { if (linkR < 0) leafB = ~linkR; else pushR = true; }
-        }
-        if (!f(leafA, leafB)) break;
-        const unsigned bl = __ballot_sync(mask, pushL), br = __ballot_sync(mask, pushR);
-        const int nl = __popc(bl), cnt = nl + __popc(br);
-        if (g == take) m--;
-        else if (sl == 0) groups[m - 1] = g - take;
-        if (cnt > 0)
-        {
-            if (sp + cnt > cap || m >= gcap)
-            {
-                // unreachable for a tree of the stated depth; recorded, never written out of bounds
-                if (sl == 0) atomicOr(status, ST_CCD_OVERFLOW);
-                break;
-            }
-            if (pushL) stack[sp + __popc(bl & lt)] = linkL;
-            if (pushR) stack[sp + nl + __popc(br & lt)] = linkR;
-            if (sl == 0) groups[m] = cnt;
-            sp += cnt;
-            m++;
-        }
-        __syncwarp(mask);
-    }
-    __syncwarp(mask);
 }
 
 // tree root for a query on particle v: its instance's tree in a batch
@@ -1488,230 +1291,51 @@ __global__ void __launch_bounds__(128) k_self_ee(DevCloth c, SolverParams P, Buf
 // Broad phase: every (triangle, vertex) and (edge, edge) pair whose swept boxes
 // overlap, with the Midphase's filters (vertex not on the triangle and not
 // pinned; edges sharing no vertex), Physics/SelfCollisionDetector.cpp:60-135,
-// but over all pairs rather than same-leaf pairs only. Pairs are listed per
-// query: (vertex, triangle) and (edge, higher edge).
-// Two passes: the first walks one query per thread and keeps up to KCCD
-// candidates in the query's own slots; the queries that find more go to a list
-// that the second pass walks one query per warp, storing the full lists in a
-// shared pool. Lists stay in traversal order: only the (rare) hits are put in
-// candidate order.
-// A vertex query: its swept box and the triangles incident to it (held in
-// registers, so a reported leaf costs no load).
-struct VtQuery
+// but over all pairs rather than same-leaf pairs only: (vertex, triangle) and
+// (edge, higher edge).
+//
+// k_ccd_boxes builds a BoxSet: one block of threads a group, one warp a block.
+template <bool TRI>
+__global__ void __launch_bounds__(1024) k_ccd_boxes(DevCloth c, Buffers b, BoxSet t, float tol)
 {
-    int i, nInc;
-    bool pinned;
-    Box box;
-    int inc[KADJ];
-    __device__ __forceinline__ void init(const DevCloth& c, int v, float tol)
+    __shared__ float sBox[32][6];
+    const int place = blockIdx.x * 1024 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (place == 0)
     {
-        i = v;
-        const float4 p4 = c.pos[v];
-        pinned = p4.w == 0.f;
-        box = Box::empty(); box.add(ld3(c.prev, v)); box.add(mk(p4.x, p4.y, p4.z)); box.extrude(tol);
-        const int r0 = c.vTriStart[v];
-        nInc = c.vTriStart[v + 1] - r0;
-#pragma unroll
-        for (int k = 0; k < KADJ; k++) inc[k] = k < nInc ? c.vTri[r0 + k].x : -1;
+        *(TRI ? b.ccdVtPairCount : b.ccdEePairCount) = 0;
+        *(TRI ? b.ccdVtTestCount : b.ccdEeTestCount) = 0;
+        *(TRI ? b.ccdVtHitTotal : b.ccdEeHitTotal) = 0;
     }
-    __device__ __forceinline__ bool accept(const DevCloth& c, int t) const
+    const int prim = t.prim[place];
+    Box x;
+    x.lo = mk(FLT_MAX, FLT_MAX, FLT_MAX); x.hi = mk(-FLT_MAX, -FLT_MAX, -FLT_MAX);
+    if (prim >= 0) x = leaf_box(c, TRI ? 2 : 3, prim, tol);
+    t.lo[place] = f4(x.lo, __int_as_float(prim));
+    t.hi[place] = f4(x.hi, 0.f);
+    float v[6] = {x.lo.x, x.lo.y, x.lo.z, -x.hi.x, -x.hi.y, -x.hi.z};
+#pragma unroll
+    for (int k = 0; k < 6; k++)
+        for (int o = 16; o > 0; o >>= 1) v[k] = fminf(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+    if (lane == 0)
     {
-        if (nInc <= KADJ)
+        t.blo[place >> 5] = make_float4(v[0], v[1], v[2], 0.f);
+        t.bhi[place >> 5] = make_float4(-v[3], -v[4], -v[5], 0.f);
+        for (int k = 0; k < 6; k++) sBox[warp][k] = v[k];
+    }
+    __syncthreads();
+    if (warp == 0)
+    {
+#pragma unroll
+        for (int k = 0; k < 6; k++)
         {
-            bool adj = false;
-#pragma unroll
-            for (int k = 0; k < KADJ; k++) adj |= inc[k] == t;
-            return !adj;
+            v[k] = sBox[lane][k];
+            for (int o = 16; o > 0; o >>= 1) v[k] = fminf(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
         }
-        return !((int)c.tri[3 * t] == i || (int)c.tri[3 * t + 1] == i || (int)c.tri[3 * t + 2] == i);
-    }
-};
-
-// An edge query: its swept box and the edges sharing one of its vertices (both
-// vertices' edge rings, in registers when they fit).
-struct EeQuery
-{
-    int i;
-    int4 e1;
-    bool inRegs;
-    Box box;
-    int adjE[KADJ];
-    __device__ __forceinline__ void init(const DevCloth& c, int e, float tol)
-    {
-        i = e;
-        e1 = c.edge[e];
-        box = Box::empty();
-        box.add(ld3(c.pos, e1.x)); box.add(ld3(c.pos, e1.y)); box.add(ld3(c.prev, e1.x)); box.add(ld3(c.prev, e1.y));
-        box.extrude(tol);
-        const int a0 = c.eRingStart[e1.x], na = c.eRingStart[e1.x + 1] - a0;
-        const int b0 = c.eRingStart[e1.y], nb = c.eRingStart[e1.y + 1] - b0;
-        inRegs = na + nb <= KADJ;
-#pragma unroll
-        for (int k = 0; k < KADJ; k++)
-            adjE[k] = !inRegs ? -1 : k < na ? c.eRing[a0 + k] : k < na + nb ? c.eRing[b0 + k - na] : -1;
-    }
-    __device__ __forceinline__ bool accept(const DevCloth& c, int e) const
-    {
-        if (e <= i) return false;
-        if (inRegs)
-        {
-            bool adj = false;
-#pragma unroll
-            for (int k = 0; k < KADJ; k++) adj |= adjE[k] == e;
-            return !adj;
-        }
-        const int4 e2 = c.edge[e];
-        return !(e1.x == e2.x || e1.y == e2.y || e1.x == e2.y || e1.y == e2.x);
-    }
-};
-
-// First pass: one query per thread (or per lane of a warp packet), at most KCCD
-// candidates into the query's own slots. A query that finds more stops walking,
-// keeps a count above KCCD and joins the overflow list for the second pass.
-__global__ void __launch_bounds__(128) k_ccd_broad_vt(DevCloth c, SolverParams P, Buffers b, DevBVH tb, float tol)
-{
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g - (int)(threadIdx.x & 31) >= c.N) return;          // whole warp past the end
-    const int i = g < c.N ? c.vQuery[g] : 0;
-    bool active = g < c.N;
-    if (active) b.ccdVtCnt[i] = 0;
-    VtQuery Q;
-    Q.init(c, i, tol);
-    if (Q.pinned) active = false;
-    int* out = b.ccdVtCand + (size_t)i * KCCD;
-    int n = 0;
-    bool stop = false;
-    auto emitT = [&](int t) {
-        if (!Q.accept(c, t)) return;
-        if (n < KCCD) out[n] = t;
-        if (++n > KCCD) stop = true;
-    };
-    if (b.broadWalk == BROAD_PACKET) bvh_query2_warp(tb, Q.box, active, emitT, -1, tree_root(c, tb, i), &stop);
-    else bvh_query2(tb, Q.box, active, emitT, -1, tree_root(c, tb, i), &stop);
-    if (!active) return;
-    b.ccdVtCnt[i] = n;
-    if (n > KCCD) b.ccdVtOvf[atomicAdd(b.ccdOvfN, 1)] = i;
-}
-
-__global__ void __launch_bounds__(128) k_ccd_broad_ee(DevCloth c, SolverParams P, Buffers b, DevBVH eb, float tol)
-{
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g - (int)(threadIdx.x & 31) >= c.E) return;
-    const int i = g < c.E ? c.eQuery[g] : 0;
-    const bool active = g < c.E;
-    EeQuery Q;
-    Q.init(c, i, tol);
-    int* out = b.ccdEeCand + (size_t)i * KCCD;
-    int n = 0;
-    bool stop = false;
-    auto emitE = [&](int e) {
-        if (!Q.accept(c, e)) return;
-        if (n < KCCD) out[n] = e;
-        if (++n > KCCD) stop = true;
-    };
-    if (b.broadWalk == BROAD_PACKET) bvh_query2_warp(eb, Q.box, active, emitE, i, tree_root(c, eb, Q.e1.x), &stop);
-    else bvh_query2(eb, Q.box, active, emitE, i, tree_root(c, eb, Q.e1.x), &stop);
-    if (!active) return;
-    b.ccdEeCnt[i] = n;
-    if (n > KCCD) b.ccdEeOvf[atomicAdd(b.ccdOvfN + 1, 1)] = i;
-}
-
-// Second pass over the overflow list: one warp per query walks the tree
-// cooperatively (bvh_query_coop) twice, counting its candidates, then writing
-// them into a pool block of exactly that size. The lane order of a step and the
-// step order are fixed, so each list (and the pair list) is deterministic.
-template <bool VT>
-__global__ void __launch_bounds__(CCD_COOP_THREADS) k_ccd_broad_coop(DevCloth c, SolverParams P, Buffers b, DevBVH t, float tol)
-{
-    extern __shared__ int sCoop[];
-    const unsigned full = 0xffffffffu;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    const int cap = CCD_COOP_GROUP * (t.depth + 1), gcap = t.depth + 2;
-    int* stack = sCoop + warp * (cap + gcap);
-    int* groups = stack + cap;
-    const int nOvf = b.ccdOvfN[VT ? 0 : 1];
-    const int* ovf = VT ? b.ccdVtOvf : b.ccdEeOvf;
-    int* cnt = VT ? b.ccdVtCnt : b.ccdEeCnt;
-    int* poolOff = VT ? b.ccdVtPoolOff : b.ccdEePoolOff;
-    const int warps = gridDim.x * (blockDim.x >> 5);
-    for (int w = blockIdx.x * (blockDim.x >> 5) + warp; w < nOvf; w += warps)
-    {
-        const int i = ovf[w];
-        VtQuery qv;
-        EeQuery qe;
-        int root, above;
-        Box box;
-        if (VT) { qv.init(c, i, tol); box = qv.box; root = tree_root(c, t, i); above = -1; }
-        else { qe.init(c, i, tol); box = qe.box; root = tree_root(c, t, qe.e1.x); above = i; }
-        auto ok = [&](int leaf) { return leaf >= 0 && (VT ? qv.accept(c, leaf) : qe.accept(c, leaf)); };
-        int total = 0;
-        bvh_query_coop<32>(t, box, above, root, stack, cap, groups, gcap, c.status, [&](int la, int lb) {
-            total += __popc(__ballot_sync(full, ok(la))) + __popc(__ballot_sync(full, ok(lb)));
-            return true;
-        });
-        int base = 0;
         if (lane == 0)
         {
-            base = atomicAdd(b.ccdPoolUsed, total);
-            if (base + total > b.ccdPoolCap) { atomicOr(c.status, ST_CCD_OVERFLOW); base = -1; }
+            t.glo[blockIdx.x] = make_float4(v[0], v[1], v[2], 0.f);
+            t.ghi[blockIdx.x] = make_float4(-v[3], -v[4], -v[5], 0.f);
         }
-        base = __shfl_sync(full, base, 0);
-        if (base < 0)
-        {
-            if (lane == 0) cnt[i] = 0;
-            continue;
-        }
-        int* out = b.ccdPool + base;
-        int pos = 0;
-        bvh_query_coop<32>(t, box, above, root, stack, cap, groups, gcap, c.status, [&](int la, int lb) {
-            const bool ka = ok(la), kb = ok(lb);
-            const unsigned ba = __ballot_sync(full, ka), bb = __ballot_sync(full, kb);
-            if (ka) out[pos + __popc(ba & lt)] = la;
-            if (kb) out[pos + __popc(ba) + __popc(bb & lt)] = lb;
-            pos += __popc(ba) + __popc(bb);
-            return true;
-        });
-        if (lane == 0) { cnt[i] = total; poolOff[i] = base; }
-        __syncwarp();
-    }
-}
-
-size_t ccd_coop_smem(int depth)
-{
-    const int cap = CCD_COOP_GROUP * (depth + 1), gcap = depth + 2;
-    return sizeof(int) * (size_t)(cap + gcap) * (CCD_COOP_THREADS / 32);
-}
-
-void ccd_kernel_setup()
-{
-    cudaFuncSetAttribute(k_ccd_broad_coop<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ccd_coop_smem(40));
-    cudaFuncSetAttribute(k_ccd_broad_coop<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ccd_coop_smem(40));
-}
-
-// first pass in the walk the model uses (BROAD_* in launch.h)
-static void launch_broad_pass1(cudaStream_t s, bool vt, const DevCloth& c, const SolverParams& P, const Buffers& b,
-                               const DevBVH& t, float tol)
-{
-    const int n = vt ? c.N : c.E;
-    if (vt) k_ccd_broad_vt<<<blocks_for(n, 128), 128, 0, s>>>(c, P, b, t, tol);
-    else k_ccd_broad_ee<<<blocks_for(n, 128), 128, 0, s>>>(c, P, b, t, tol);
-}
-
-// expand per-query candidate lists (own slots, or the pool for long lists)
-// into the dense pair list; one warp per query, coalesced copies
-__global__ void k_ccd_pairs(const int* cnt, const int* off, const int* cand, const int* pool, const int* poolOff,
-                            int n, int2* pairs, int cap, int* status, int* hitCnt)
-{
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (i >= n) return;
-    if (lane == 0) hitCnt[i] = 0;                 // counted by the narrow phase
-    const int m = cnt[i], o = off[i];
-    const int* src = m > KCCD ? pool + poolOff[i] : cand + (size_t)i * KCCD;
-    for (int k = lane; k < m; k += 32)
-    {
-        if (o + k < cap) pairs[o + k] = make_int2(i, src[k]);
-        else atomicOr(status, ST_CCD_OVERFLOW);
     }
 }
 
@@ -1805,12 +1429,10 @@ __device__ bool solve_cubic(V3 x1, V3 x2, V3 x3, V3 x4, V3 v1, V3 v2, V3 v3, V3 
     return coplanar;
 }
 
-// VertexTriangleTest + VertexTriangleCCD (SelfCollisionDetector.cpp:171-277) for
-// pair k: 1 and the contact record on a hit, else 0
-__device__ int ccd_vt_test(const DevCloth& c, const SolverParams& P, const Buffers& b, int k, SCt& rec)
+// VertexTriangleTest + VertexTriangleCCD (SelfCollisionDetector.cpp:171-277) for a
+// (vertex, triangle) pair: 1 and the contact record on a hit, else 0
+__device__ int ccd_vt_test(const DevCloth& c, const SolverParams& P, int vtx, int t, SCt& rec)
 {
-    int2 pr = b.ccdVtPairs[k];
-    const int vtx = pr.x, t = pr.y;
     const uint32_t i1 = c.tri[3 * t], i2 = c.tri[3 * t + 1], i3 = c.tri[3 * t + 2];
     V3 x1 = ld3(c.prev, i1), x2 = ld3(c.prev, i2), x3 = ld3(c.prev, i3), x4 = ld3(c.prev, vtx);
     V3 v1 = ld3(c.pos, i1) - x1, v2 = ld3(c.pos, i2) - x2, v3 = ld3(c.pos, i3) - x3, v4 = ld3(c.pos, vtx) - x4;
@@ -1835,11 +1457,10 @@ __device__ int ccd_vt_test(const DevCloth& c, const SolverParams& P, const Buffe
     return 1;
 }
 
-// EdgeEdgeTest + EdgeEdgeCCD (SelfCollisionDetector.cpp:491-606) for pair k
-__device__ int ccd_ee_test(const DevCloth& c, const SolverParams& P, const Buffers& b, int k, SCt& rec)
+// EdgeEdgeTest + EdgeEdgeCCD (SelfCollisionDetector.cpp:491-606) for a pair of edges
+__device__ int ccd_ee_test(const DevCloth& c, const SolverParams& P, int ea, int eb, SCt& rec)
 {
-    int2 pr = b.ccdEePairs[k];
-    const int4 A = c.edge[pr.x], B = c.edge[pr.y];
+    const int4 A = c.edge[ea], B = c.edge[eb];
     const int i1 = A.x, i2 = A.y, j1 = B.x, j2 = B.y;
     if (i1 == j1 || i1 == j2 || i2 == j1 || i2 == j2) return 0;
     V3 x1 = ld3(c.prev, i1), x2 = ld3(c.prev, i2), x3 = ld3(c.prev, j1), x4 = ld3(c.prev, j2);
@@ -1864,75 +1485,264 @@ __device__ int ccd_ee_test(const DevCloth& c, const SolverParams& P, const Buffe
     return 1;
 }
 
-// narrow phase over the device-counted pair lists (grid-stride; every pair
-// gets its hit flag, so no clearing is needed)
-// per pair: hit flag, and the query's hit count (zeroed by k_ccd_pairs; hits
-// are rare, so the atomics are too)
-__global__ void k_ccd_narrow_vt(DevCloth c, SolverParams P, Buffers b)
+// Broad phase and the first part of the narrow phase in one pass: JOIN_WARPS warps
+// per block of 32 queries that are neighbours in the rest shape, each with its
+// share of the candidate blocks. A warp carries the union of the queries' boxes down
+// the three levels, 32 boxes a step (one per lane, coalesced); the primitives of a
+// block that meet the union are laid out in shared memory and every lane tests its
+// own query against each (two broadcast loads, six compares, a bit of a mask: no
+// branch and no vote, so the loads overlap). An edge block meets itself and the
+// blocks after it only: each pair once. Accepted pairs go to a small buffer in
+// shared memory, which is written out 32 pairs at a time together with the test that
+// rules most of them out (four points coplanar at the start): the positions are
+// still in L1 there. What is left is listed for k_ccd_test.
+//
+// What bounds it: instruction issue and the latency of the block loads, which
+// JOIN_WARPS warps a query block hide on clothes of a few hundred blocks. The stack
+// walks it replaces took 29,000 warp instructions per 32 edge queries with 12 of 32
+// lanes active and two dependent loads a step, and their lists six more passes
+// (count, scan, copy, test, count and gather hits). The edge-edge half of a substep,
+// boxes included: 207 -> 78 us on a 128 x 128 drape (2 M pairs), 510 -> 253 us on a
+// 256 x 256 one (11.5 M pairs). Four warps a query block measured 98, one 205.
+constexpr int JOIN_WARPS = 8, JOIN_BUF = 128;
+constexpr unsigned JOIN_SHARE = 0x01010101u;        // every JOIN_WARPS-th bit
+
+struct JoinSmem
 {
-    int n = *b.ccdVtPairCount;
-    if (n > b.ccdVtCap) n = b.ccdVtCap;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    {
-        SCt rec;
-        const bool hit = ccd_vt_test(c, P, b, k, rec);
-        b.ccdVtHit[k] = (uint8_t)hit;
-        if (hit) atomicAdd(&b.ccdVtHitCnt[b.ccdVtPairs[k].x], 1);
-    }
+    float4 lo[32], hi[32];       // candidates of the current block; w: primitive, place
+    int4 ends[32];               // and their particles
+    int2 pair[JOIN_BUF];
+};
+
+// the first part of solve_cubic: the four points are (nearly) coplanar at the start
+// of the step, which rules the pair out; needs the start positions alone
+__device__ __forceinline__ bool coplanar_at_start(V3 x1, V3 x2, V3 x3, V3 x4)
+{
+    return fabsf(dot(cross(x2 - x1, x3 - x1), x4 - x1)) < 0.001f;
 }
 
-__global__ void k_ccd_narrow_ee(DevCloth c, SolverParams P, Buffers b)
-{
-    int n = *b.ccdEePairCount;
-    if (n > b.ccdEeCap) n = b.ccdEeCap;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    {
-        SCt rec;
-        const bool hit = ccd_ee_test(c, P, b, k, rec);
-        b.ccdEeHit[k] = (uint8_t)hit;
-        if (hit) atomicAdd(&b.ccdEeHitCnt[b.ccdEePairs[k].x], 1);
-    }
-}
-
-// append the hit records after the list's current count, per query in ascending
-// candidate order (the order of an all-pairs sweep); one warp per query picks its
-// hits smallest candidate first. A hit's record is recomputed by the same
-// deterministic test rather than stored per pair.
 template <bool VT>
-__global__ void k_ccd_gather(DevCloth c, SolverParams P, Buffers b, const int* hoff, SCt* list, const int* listCount, int listCap)
+__device__ __forceinline__ void join_flush(const DevCloth& c, const Buffers& b, const JoinSmem& s, int n, int lane)
 {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    const int n = VT ? c.N : c.E;
-    if (i >= n) return;
-    const int h = (VT ? b.ccdVtHitCnt : b.ccdEeHitCnt)[i];
-    if (h == 0) return;
-    const int* cnt = VT ? b.ccdVtCnt : b.ccdEeCnt;
-    const int* off = VT ? b.ccdVtOff : b.ccdEeOff;
-    const uint8_t* hit = VT ? b.ccdVtHit : b.ccdEeHit;
-    const int2* pairs = VT ? b.ccdVtPairs : b.ccdEePairs;
+    const unsigned full = 0xffffffffu;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(VT ? b.ccdVtPairCount : b.ccdEePairCount, n);
+    base = __shfl_sync(full, base, 0);
+    int2* pairs = VT ? b.ccdVtPairs : b.ccdEePairs;
     const int cap = VT ? b.ccdVtCap : b.ccdEeCap;
-    const int o = off[i], e = min(cap, o + cnt[i]);
-    const int d0 = *listCount + hoff[i];
-    int last = -1;
-    for (int r = 0; r < h; r++)
+    for (int i0 = 0; i0 < n; i0 += 32)
     {
-        int best = INT_MAX, bestK = -1;
-        for (int k = o + lane; k < e; k += 32)
-            if (hit[k])
-            {
-                const int id = pairs[k].y;
-                if (id > last && id < best) { best = id; bestK = k; }
-            }
-        const int m = __reduce_min_sync(0xffffffffu, best);
-        if (best == m && bestK >= 0)
+        const int i = i0 + lane;
+        bool left = false;
+        int2 pr = make_int2(0, 0);
+        if (i < n)
         {
-            SCt rec;
-            if (VT) ccd_vt_test(c, P, b, bestK, rec); else ccd_ee_test(c, P, b, bestK, rec);
-            if (d0 + r < listCap) list[d0 + r] = rec;
+            pr = s.pair[i];
+            if (base + i < cap && base + i >= 0) pairs[base + i] = pr;
+            else atomicOr(c.status, ST_CCD_OVERFLOW);
+            if (VT)
+                left = !coplanar_at_start(ld3(c.prev, c.tri[3 * pr.y]), ld3(c.prev, c.tri[3 * pr.y + 1]), ld3(c.prev, c.tri[3 * pr.y + 2]),
+                                          ld3(c.prev, pr.x));
+            else
+            {
+                const int4 A = c.edge[pr.x], B = c.edge[pr.y];
+                left = !coplanar_at_start(ld3(c.prev, A.x), ld3(c.prev, A.y), ld3(c.prev, B.x), ld3(c.prev, B.y));
+            }
+        }
+        const unsigned m = __ballot_sync(full, left);
+        if (m == 0u) continue;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(VT ? b.ccdVtTestCount : b.ccdEeTestCount, __popc(m));
+        at = __shfl_sync(full, at, 0) + __popc(m & ((1u << lane) - 1u));
+        if (left)
+        {
+            if (at < cap && at >= 0) (VT ? b.ccdVtTest : b.ccdEeTest)[at] = pr;
             else atomicOr(c.status, ST_CCD_OVERFLOW);
         }
-        last = m;
     }
+    __syncwarp();
+}
+
+__device__ __forceinline__ bool meet(float4 lo, float4 hi, const Box& q)
+{
+    return !(hi.x < q.lo.x || hi.y < q.lo.y || hi.z < q.lo.z || q.hi.x < lo.x || q.hi.y < lo.y || q.hi.z < lo.z);
+}
+
+template <bool VT>
+__global__ void __launch_bounds__(32 * JOIN_WARPS, 5) k_ccd_join(DevCloth c, Buffers b, BoxSet t, VertexBlocks vb, float tol)
+{
+    __shared__ JoinSmem sAll[JOIN_WARPS];
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, block = blockIdx.x;
+    JoinSmem& s = sAll[warp];
+    const int q = VT ? vb.vertex[32 * block + lane] : t.prim[32 * block + lane];
+    if (__ballot_sync(full, q >= 0) == 0u) return;          // an unused block of a group
+    if (warp == 0 && q >= 0) (VT ? b.ccdVtHitCnt : b.ccdEeHitCnt)[q] = 0;
+    Box box;
+    box.lo = mk(FLT_MAX, FLT_MAX, FLT_MAX); box.hi = mk(-FLT_MAX, -FLT_MAX, -FLT_MAX);
+    bool active = q >= 0;
+    int qa = -1, qb = -1;                  // the query's particles
+    if (VT && active)
+    {
+        const float4 p4 = c.pos[q];
+        box = Box::empty(); box.add(ld3(c.prev, q)); box.add(mk(p4.x, p4.y, p4.z)); box.extrude(tol);
+        active = p4.w != 0.f;
+        qa = q;
+    }
+    if (!VT && active)
+    {
+        box.lo = mk(t.lo[32 * block + lane]); box.hi = mk(t.hi[32 * block + lane]);
+        const int4 e = t.ends[32 * block + lane];
+        qa = e.x; qb = e.y;
+    }
+    // the union of the lanes' boxes
+    float v[6];
+    if (active) { v[0] = box.lo.x; v[1] = box.lo.y; v[2] = box.lo.z; v[3] = -box.hi.x; v[4] = -box.hi.y; v[5] = -box.hi.z; }
+    else for (int k = 0; k < 6; k++) v[k] = FLT_MAX;
+#pragma unroll
+    for (int k = 0; k < 6; k++)
+        for (int o = 16; o > 0; o >>= 1) v[k] = fminf(v[k], __shfl_xor_sync(full, v[k], o));
+    Box all;
+    all.lo = mk(v[0], v[1], v[2]); all.hi = mk(-v[3], -v[4], -v[5]);
+    int g0 = 0, g1 = t.nGroups;
+    if (t.inst)
+    {
+        const int2 r = t.inst[VT ? vb.blockInst[block] : t.groupInst[block >> 5]];
+        g0 = r.x; g1 = r.x + r.y;
+    }
+    if (!VT) g0 = block >> 5;
+    if (!__any_sync(full, active)) g1 = g0;
+    const unsigned lt = (1u << lane) - 1u;
+    int n = 0;
+    for (int gb = g0; gb < g1; gb += 32)
+    {
+        const int g = gb + lane;
+        unsigned mg = __ballot_sync(full, g < g1 && meet(t.glo[min(g, g1 - 1)], t.ghi[min(g, g1 - 1)], all));
+        for (; mg; mg &= mg - 1)
+        {
+            const int bl = 32 * (gb + __ffs(mg) - 1);
+            // this warp's share: every JOIN_WARPS-th block
+            unsigned mb = __ballot_sync(full, (VT || bl + lane >= block) && meet(t.blo[bl + lane], t.bhi[bl + lane], all)) & (JOIN_SHARE << warp);
+            for (; mb; mb &= mb - 1)
+            {
+                const int place = 32 * (bl + __ffs(mb) - 1) + lane;
+                const float4 lo = t.lo[place];
+                float4 hi = t.hi[place];
+                const bool in = __float_as_int(lo.w) >= 0 && meet(lo, hi, all);
+                const unsigned m = __ballot_sync(full, in);
+                hi.w = __int_as_float(place);
+                __syncwarp();
+                if (in) { const int k = __popc(m & lt); s.lo[k] = lo; s.hi[k] = hi; s.ends[k] = t.ends[place]; }
+                __syncwarp();
+                const int cnt = __popc(m);
+                unsigned met = 0u;
+#pragma unroll 4
+                for (int k = 0; k < cnt; k++) met |= meet(s.lo[k], s.hi[k], box) ? 1u << k : 0u;
+                if (!active) met = 0u;
+                while (__any_sync(full, met != 0u))
+                {
+                    bool ok = met != 0u;
+                    const int k = ok ? __ffs(met) - 1 : 0;
+                    const int p = __float_as_int(s.lo[k].w);
+                    met &= met - 1;
+                    // the Midphase's filters: the vertex not on the triangle, no shared particle
+                    const int4 e = s.ends[k];
+                    if (VT) ok = ok && e.x != qa && e.y != qa && e.z != qa;
+                    else ok = ok && __float_as_int(s.hi[k].w) > 32 * block + lane && e.x != qa && e.x != qb && e.y != qa && e.y != qb;
+                    const unsigned mo = __ballot_sync(full, ok);
+                    if (ok) s.pair[n + __popc(mo & lt)] = VT ? make_int2(q, p) : make_int2(min(q, p), max(q, p));
+                    n += __popc(mo);
+                    if (n > JOIN_BUF - 32) { __syncwarp(); join_flush<VT>(c, b, s, n, lane); n = 0; }
+                }
+            }
+        }
+    }
+    __syncwarp();
+    if (n > 0) join_flush<VT>(c, b, s, n, lane);
+}
+
+// the rest of the continuous test, for the pairs that were not coplanar at the start
+__global__ void __launch_bounds__(128) k_ccd_test(DevCloth c, SolverParams P, Buffers b)
+{
+    const bool vt = blockIdx.x < gridDim.x / 2;
+    const int blocks = gridDim.x / 2, n = vt ? min(*b.ccdVtTestCount, b.ccdVtCap) : min(*b.ccdEeTestCount, b.ccdEeCap);
+    const int2* list = vt ? b.ccdVtTest : b.ccdEeTest;
+    for (int k = (blockIdx.x % blocks) * blockDim.x + threadIdx.x; k < n; k += blocks * blockDim.x)
+    {
+        const int2 p = list[k];
+        SCt rec;
+        if (!(vt ? ccd_vt_test(c, P, p.x, p.y, rec) : ccd_ee_test(c, P, p.x, p.y, rec))) continue;
+        atomicAdd(&(vt ? b.ccdVtHitCnt : b.ccdEeHitCnt)[p.x], 1);
+        const int h = atomicAdd(vt ? b.ccdVtHitTotal : b.ccdEeHitTotal, 1);
+        if (h < (vt ? b.ccdVtHitCap : b.ccdEeHitCap)) (vt ? b.ccdVtHits : b.ccdEeHits)[h] = p;
+        else atomicOr(c.status, ST_CCD_OVERFLOW);
+    }
+}
+
+// The hits appended after the list's current count, in (query, candidate) order
+// (the order of an all-pairs sweep); a block of threads per kind. There are none in
+// most substeps. A hit's record is recomputed by the same deterministic test.
+template <bool VT>
+__device__ void append_hits(const DevCloth& c, const SolverParams& P, const Buffers& b, int* off)
+{
+    __shared__ int sWarp[32];
+    int* listCount = VT ? b.stCount : b.seCount;
+    SCt* list = VT ? b.stList : b.seList;
+    const int listCap = VT ? b.stCap : b.seCap;
+    const int base = *listCount, h = min(VT ? *b.ccdVtHitTotal : *b.ccdEeHitTotal, VT ? b.ccdVtHitCap : b.ccdEeHitCap);
+    __syncthreads();
+    if (threadIdx.x == 0) *listCount = min(listCap, base + h);
+    if (h == 0) return;
+    const int n = VT ? c.N : c.E;
+    int* cnt = VT ? b.ccdVtHitCnt : b.ccdEeHitCnt;
+    const int2* hits = VT ? b.ccdVtHits : b.ccdEeHits;
+    int2* sorted = VT ? b.ccdVtSorted : b.ccdEeSorted;
+    int carry = 0;
+    for (int i0 = 0; i0 < n; i0 += blockDim.x)
+    {
+        const int i = i0 + threadIdx.x;
+        int total;
+        const int ex = block_exclusive_scan(i < n ? cnt[i] : 0, sWarp, total);
+        if (i < n) off[i] = carry + ex;
+        carry += total;
+    }
+    if (threadIdx.x == 0) off[n] = carry;
+    __syncthreads();
+    if (carry > h)
+    {
+        // hits beyond the store (recorded in the status): the counts do not match it
+        for (int k = threadIdx.x; k < h; k += blockDim.x)
+        {
+            SCt rec;
+            const int2 p = hits[k];
+            if (VT) ccd_vt_test(c, P, p.x, p.y, rec); else ccd_ee_test(c, P, p.x, p.y, rec);
+            if (base + k < listCap) list[base + k] = rec;
+        }
+        return;
+    }
+    for (int k = threadIdx.x; k < h; k += blockDim.x)
+    {
+        const int2 p = hits[k];
+        sorted[off[p.x] + atomicSub(&cnt[p.x], 1) - 1] = p;
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < h; k += blockDim.x)
+    {
+        const int2 p = sorted[k];
+        const int a = off[p.x], e = off[p.x + 1];
+        int r = a;
+        for (int j = a; j < e; j++) r += sorted[j].y < p.y;
+        SCt rec;
+        if (VT) ccd_vt_test(c, P, p.x, p.y, rec); else ccd_ee_test(c, P, p.x, p.y, rec);
+        if (base + r < listCap) list[base + r] = rec;
+        else atomicOr(c.status, ST_CCD_OVERFLOW);
+    }
+}
+
+__global__ void __launch_bounds__(1024) k_ccd_hits(DevCloth c, SolverParams P, Buffers b)
+{
+    if (blockIdx.x == 0) append_hits<true>(c, P, b, b.scanOff);
+    else append_hits<false>(c, P, b, b.scanOff2);
 }
 
 // Constraint residual: max |C| over the warp, weft and shear constraints of every
@@ -2153,8 +1963,7 @@ void launch_self_proximity(cudaStream_t s, const DevCloth& c, const SolverParams
     k_self_ee<<<blocks_for(c.E, 128), 128, 0, s>>>(c, P, b, edgeBvh);
 }
 
-void launch_compact_self(cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, const DevCloth& c,
-                         const SolverParams& P, const Buffers& b, bool self, bool ccd)
+void launch_compact_self(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, bool self, bool ccd)
 {
     if (self)
     {
@@ -2165,24 +1974,10 @@ void launch_compact_self(cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cu
         k_compact<SCt><<<blocks_for(c.E), 256, 0, s>>>(b.seFlag, off, b.seSlot, 1, b.seList, c.E, nullptr, b.seCap, c.status, ST_SELF_EE_OVERFLOW);
     }
     else cudaMemsetAsync(b.stCount, 0, 2 * sizeof(int), s);     // no proximity contacts (stCount, seCount)
-    if (ccd)
-    {
-        // continuous hits go after the proximity contacts, as the detector's
-        // AddSelfTriangle / AddSelfEdge would append them (in pair order); the
-        // vertex-triangle list is assembled on the side stream beside the
-        // edge-edge one (own offsets, block sums and total)
-        cudaEventRecord(fork, s);
-        cudaStreamWaitEvent(side, fork, 0);
-        scan_ints(side, b.ccdVtHitCnt, b.scanOff2, c.N, b.scanTot + 1, b.scanBlock2);
-        k_ccd_gather<true><<<blocks_for(32 * c.N), 256, 0, side>>>(c, P, b, b.scanOff2, b.stList, b.stCount, b.stCap);
-        k_add_counts<<<1, 32, 0, side>>>(b.stCount, b.stCount, b.scanTot + 1, b.stCap);
-        cudaEventRecord(join, side);
-        scan_ints(s, b.ccdEeHitCnt, b.scanOff, c.E, b.scanTot, b.scanBlock);
-        k_ccd_gather<false><<<blocks_for(32 * c.E), 256, 0, s>>>(c, P, b, b.scanOff, b.seList, b.seCount, b.seCap);
-        k_add_counts<<<1, 32, 0, s>>>(b.seCount, b.seCount, b.scanTot, b.seCap);
-        cudaStreamWaitEvent(s, join, 0);
-    }
-    if (self)
+    // continuous hits go after the proximity contacts, as the detector's
+    // AddSelfTriangle / AddSelfEdge would append them (in pair order)
+    if (ccd) k_ccd_hits<<<2, 1024, 0, s>>>(c, P, b);
+    else if (self)
     {
         k_add_counts<<<1, 32, 0, s>>>(b.stCount, b.stCount, nullptr, b.stCap);
         k_add_counts<<<1, 32, 0, s>>>(b.seCount, b.seCount, nullptr, b.seCap);
@@ -2190,42 +1985,28 @@ void launch_compact_self(cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cu
 }
 
 void launch_ccd(cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, const DevCloth& c,
-                const SolverParams& P, const Buffers& b, const DevBVH& triBvh, const DevBVH& edgeBvh,
+                const SolverParams& P, const Buffers& b, const BoxSet& tris, const BoxSet& edges, const VertexBlocks& verts,
                 const cudaEvent_t* marks)
 {
     auto mark = [&](int k, cudaStream_t st) {
         if (marks && marks[k]) cudaEventRecordWithFlags(marks[k], st, cudaEventRecordExternal);
     };
-    // The vertex-triangle chain (refit, broad phase, pairs, narrow phase) runs on
-    // the side stream beside the edge-edge chain; each is latency bound and fills
-    // only part of the GPU. They share nothing but the pool counter (atomic).
+    // the vertex-triangle half runs on the side stream beside the edge-edge half:
+    // they share nothing
     const float tol = P.thickness + P.tolerance * 0.5f;
-    cudaMemsetAsync(b.ccdPoolUsed, 0, sizeof(int), s);
-    cudaMemsetAsync(b.ccdOvfN, 0, 2 * sizeof(int), s);
     cudaEventRecord(fork, s);
     cudaStreamWaitEvent(side, fork, 0);
-    launch_bvh_refit(side, triBvh, c, 2, tol);
     mark(2, side);
-    launch_broad_pass1(side, true, c, P, b, triBvh, tol);
-    k_ccd_broad_coop<true><<<CCD_COOP_BLOCKS, CCD_COOP_THREADS, ccd_coop_smem(triBvh.depth), side>>>(c, P, b, triBvh, tol);
+    k_ccd_boxes<true><<<tris.nGroups, 1024, 0, side>>>(c, b, tris, tol);
+    k_ccd_join<true><<<verts.nBlocks, 32 * JOIN_WARPS, 0, side>>>(c, b, tris, verts, tol);
     mark(3, side);
-    scan_ints(side, b.ccdVtCnt, b.ccdVtOff, c.N, b.ccdVtPairCount, b.scanBlock2);
-    k_ccd_pairs<<<blocks_for(32 * c.N), 256, 0, side>>>(b.ccdVtCnt, b.ccdVtOff, b.ccdVtCand, b.ccdPool, b.ccdVtPoolOff, c.N,
-                                                   b.ccdVtPairs, b.ccdVtCap, c.status, b.ccdVtHitCnt);
-    k_ccd_narrow_vt<<<4 * 148, 128, 0, side>>>(c, P, b);
     cudaEventRecord(join, side);
-
-    launch_bvh_refit(s, edgeBvh, c, 3, tol);
     mark(0, s);
-    launch_broad_pass1(s, false, c, P, b, edgeBvh, tol);
-    k_ccd_broad_coop<false><<<CCD_COOP_BLOCKS, CCD_COOP_THREADS, ccd_coop_smem(edgeBvh.depth), s>>>(c, P, b, edgeBvh, tol);
+    k_ccd_boxes<false><<<edges.nGroups, 1024, 0, s>>>(c, b, edges, tol);
+    k_ccd_join<false><<<32 * edges.nGroups, 32 * JOIN_WARPS, 0, s>>>(c, b, edges, verts, tol);
     mark(1, s);
-    scan_ints(s, b.ccdEeCnt, b.ccdEeOff, c.E, b.ccdEePairCount, b.scanBlock);
-    k_ccd_pairs<<<blocks_for(32 * c.E), 256, 0, s>>>(b.ccdEeCnt, b.ccdEeOff, b.ccdEeCand, b.ccdPool, b.ccdEePoolOff, c.E,
-                                                b.ccdEePairs, b.ccdEeCap, c.status, b.ccdEeHitCnt);
-    // narrow phase: a fixed grid strides over the device-side pair counts
-    k_ccd_narrow_ee<<<8 * 148, 128, 0, s>>>(c, P, b);
     cudaStreamWaitEvent(s, join, 0);
+    k_ccd_test<<<4 * 148, 128, 0, s>>>(c, P, b);
 }
 
 // largest displacement since the snapshot (scaled), into scal[11]; new snapshot
