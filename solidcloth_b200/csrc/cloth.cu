@@ -1886,8 +1886,17 @@ bool ClothModel::ensure_buffers(const CollisionWorld& world, cudaStream_t s)
     buf.ccdVtHitCnt = (int*)dalloc(sizeof(int) * N, true);
     buf.ccdEeHitCnt = (int*)dalloc(sizeof(int) * E, true);
     // colouring
-    buf.vmin = (unsigned long long*)dalloc(sizeof(unsigned long long) * N, true);
-    SC_CUDA(cudaMemset(buf.vmin, 0xff, sizeof(unsigned long long) * N));
+    for (int k = 0; k < 2; k++)
+    {
+        ColourScratch& w = buf.colouring[k];
+        const size_t cap = k == 0 ? buf.stCap : buf.seCap;
+        w.deg = (int*)dalloc(sizeof(int) * N, true);
+        w.cur = (int*)dalloc(sizeof(int) * N, true);
+        w.key = (unsigned long long*)dalloc(sizeof(unsigned long long) * 4 * cap, true);
+        w.sorted = (int*)dalloc(sizeof(int) * 4 * cap, true);
+        w.next = (int4*)dalloc(sizeof(int4) * cap, true);
+        w.rem = (int*)dalloc(sizeof(int) * cap, true);
+    }
     buf.colourCap = buf.ecCap + buf.tcCap + buf.stCap + buf.seCap;
     buf.colour = (int*)dalloc(sizeof(int) * (size_t)buf.colourCap, true);
     buf.order = (int*)dalloc(sizeof(int) * (size_t)buf.colourCap, true);

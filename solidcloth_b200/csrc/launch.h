@@ -37,6 +37,16 @@ struct VColl
     int4 sdfCells;
 };
 
+// scratch of one class's contact colouring: per particle its number of contacts (zero
+// between substeps) and its list's end; per list entry the key and, sorted, the
+// contact; per contact its successors' entries and how many particles hold it back
+struct ColourScratch
+{
+    int* deg; int* cur;
+    unsigned long long* key; int* sorted;
+    int4* next; int* rem;
+};
+
 struct Buffers
 {
     // vertex contacts: counts[coll][N] (uint8), slots[slotBase + i*kmax + k]
@@ -59,7 +69,7 @@ struct Buffers
     int* ccdVtHitCnt; int* ccdEeHitCnt;
     int2* ccdVtSorted; int2* ccdEeSorted;
     // colouring scratch
-    unsigned long long* vmin;  // N, kept at ~0
+    ColourScratch colouring[2];  // self vertex-triangle, self edge-edge
     int* colour; int* order; int* colourStart; int colourCap;
     // scan scratch: block sums, per-item offsets, totals
     int* scanBlock; int* scanOff; int* scanTot;

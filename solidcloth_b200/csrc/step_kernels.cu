@@ -708,6 +708,13 @@ __global__ void k_edge_colliders(DevCloth c, SolverParams P, Buffers b, VColl g,
 // colour. Contacts of one colour share no particle, so a colour is one
 // parallel sweep and the result equals the sequential sweep in
 // (colour, index) order, which is what the oracle's check mode runs.
+//
+// The rounds are run as a queue: every particle's contacts are ranked by key, and a
+// contact joins the next round when it has become the first uncoloured one on all
+// of its particles, so each contact is handled once and not once a round. The queue
+// is the colour order. What bounds it: the chain of rounds (one L2 round trip each)
+// on one block of threads per class; 10,081 + 5,171 contacts took 2,656 us when every
+// round visited every contact, 440 us here.
 
 __device__ __forceinline__ int contact_verts(const Buffers& b, int kind, int i, uint32_t* v)
 {
@@ -731,59 +738,109 @@ __device__ __forceinline__ unsigned long long contact_key(const DevCloth& c, con
 
 __device__ void place_by_colour(const ClassView& cv, int n);
 
-__device__ void colour_class(const DevCloth& c, const Buffers& b, const ClassView& cv, int* status)
+// self contacts (kind 2, 3); w: the class's scratch
+__device__ void colour_class(const DevCloth& c, const Buffers& b, const ClassView& cv, const ColourScratch& w, int* status)
 {
-    __shared__ int sRemaining;
-    const int n = *cv.count;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) cv.colour[i] = -1;
-    if (threadIdx.x == 0) sRemaining = n;
+    __shared__ int sTotal, sTail;
+    const int n = *cv.count, tid = threadIdx.x, nt = blockDim.x;
+    if (tid == 0) { sTotal = 0; sTail = 0; }
     __syncthreads();
-    int round = 0;
-    while (sRemaining > 0 && round < MAX_COLOURS - 1)
+    // contacts per particle; whoever counts first reserves the particle's list
+    auto particle = [&](const uint32_t* v, int nv, int k) {
+        for (int j = 0; j < k; j++) if (v[j] == v[k]) return false;      // a particle named twice counts once
+        return k < nv;
+    };
+    for (int i = tid; i < n; i += nt)
     {
-        for (int i = threadIdx.x; i < n; i += blockDim.x)
+        uint32_t v[4];
+        const int nv = contact_verts(b, cv.kind, i, v);
+        int first = 0;
+        for (int k = 0; k < nv; k++)
+            if (particle(v, nv, k) && atomicAdd(&w.deg[v[k]], 1) == 0) first |= 1 << k;
+        w.rem[i] = first;
+        cv.colour[i] = MAX_COLOURS - 1;
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += nt)
+    {
+        const int first = w.rem[i];
+        if (!first) continue;
+        uint32_t v[4];
+        contact_verts(b, cv.kind, i, v);
+        for (int k = 0; k < 4; k++) if (first >> k & 1) w.cur[v[k]] = atomicAdd(&sTotal, w.deg[v[k]]);
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += nt)
+    {
+        uint32_t v[4];
+        const int nv = contact_verts(b, cv.kind, i, v);
+        const unsigned long long key = contact_key(c, v, nv, i);
+        for (int k = 0; k < nv; k++) if (particle(v, nv, k)) w.key[atomicAdd(&w.cur[v[k]], 1)] = key;
+    }
+    __syncthreads();
+    // each contact's place in its particles' lists (cur is the list's end now): the
+    // sorted lists hold the contact, and the contact how many of its particles still
+    // have an earlier one
+    for (int i = tid; i < n; i += nt)
+    {
+        uint32_t v[4];
+        const int nv = contact_verts(b, cv.kind, i, v);
+        const unsigned long long key = contact_key(c, v, nv, i);
+        int rem = 0;
+        int at[4] = {-1, -1, -1, -1};
+        for (int k = 0; k < nv; k++)
         {
-            if (cv.colour[i] >= 0) continue;
-            uint32_t v[4]; int nv = contact_verts(b, cv.kind, i, v);
-            const unsigned long long key = contact_key(c, v, nv, i);
-            for (int k = 0; k < nv; k++) atomicMin(&b.vmin[v[k]], key);
+            if (!particle(v, nv, k)) continue;
+            const int e = w.cur[v[k]], d = w.deg[v[k]];
+            int r = 0;
+            for (int j = e - d; j < e; j++) r += w.key[j] < key;
+            w.sorted[e - d + r] = i;
+            at[k] = e - d + r + 1 < e ? e - d + r + 1 : -1;          // who comes after it
+            rem += r > 0;
+        }
+        w.rem[i] = rem;
+        w.next[i] = make_int4(at[0], at[1], at[2], at[3]);
+        if (rem == 0) cv.order[atomicAdd(&sTail, 1)] = i;
+    }
+    __syncthreads();
+    // clear the counts for the next substep (every particle is named by some contact)
+    for (int i = tid; i < n; i += nt)
+    {
+        uint32_t v[4];
+        const int nv = contact_verts(b, cv.kind, i, v);
+        for (int k = 0; k < nv; k++) w.deg[v[k]] = 0;
+    }
+    int head = 0, tail = sTail, round = 0;
+    while (head < tail && round < MAX_COLOURS - 1)
+    {
+        if (tid == 0) cv.start[round] = head;
+        __syncthreads();                                              // sTail has been read by all
+        for (int q = head + tid; q < tail; q += nt)
+        {
+            const int i = cv.order[q];
+            cv.colour[i] = round;
+            const int4 a = w.next[i];
+            const int at[4] = {a.x, a.y, a.z, a.w};
+            int j[4];
+            for (int k = 0; k < 4; k++) j[k] = at[k] >= 0 ? w.sorted[at[k]] : -1;
+            for (int k = 0; k < 4; k++)
+                if (j[k] >= 0 && atomicSub(&w.rem[j[k]], 1) == 1) cv.order[atomicAdd(&sTail, 1)] = j[k];
         }
         __syncthreads();
-        int mine = 0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x)
-        {
-            if (cv.colour[i] >= 0) continue;
-            uint32_t v[4]; int nv = contact_verts(b, cv.kind, i, v);
-            const unsigned long long key = contact_key(c, v, nv, i);
-            bool ok = true;
-            for (int k = 0; k < nv; k++) ok = ok && (b.vmin[v[k]] == key);
-            if (ok) { cv.colour[i] = MAX_COLOURS + round; mine++; }   // tentative mark
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x)
-        {
-            int col = cv.colour[i];
-            if (col >= 0 && col != MAX_COLOURS + round) continue;
-            uint32_t v[4]; int nv = contact_verts(b, cv.kind, i, v);
-            for (int k = 0; k < nv; k++) b.vmin[v[k]] = ~0ull;
-            if (col == MAX_COLOURS + round) cv.colour[i] = round;
-        }
-        __shared__ int sCount;
-        if (threadIdx.x == 0) sCount = 0;
-        __syncthreads();
-        if (mine) atomicAdd(&sCount, mine);
-        __syncthreads();
-        if (threadIdx.x == 0) sRemaining -= sCount;
-        __syncthreads();
+        head = tail;
+        tail = sTail;
         round++;
     }
-    if (sRemaining > 0)
+    for (int k = round + tid; k <= MAX_COLOURS; k += nt) cv.start[k] = k < MAX_COLOURS ? head : n;
+    if (head < n)
     {
         // not expected for contact graphs of bounded degree: the rest go to the
         // last colour, which the solver runs on a single thread in list order
-        if (threadIdx.x == 0) atomicOr(status, ST_COLOUR_OVERFLOW);
+        __syncthreads();
+        if (tid == 0) { atomicOr(status, ST_COLOUR_OVERFLOW); sTail = head; }
+        __syncthreads();
+        for (int i = tid; i < n; i += nt) if (cv.colour[i] == MAX_COLOURS - 1) cv.order[atomicAdd(&sTail, 1)] = i;
     }
-    place_by_colour(cv, n);
 }
 
 // Triangle (class 1) and edge (class 0) collider contacts: the static colour of
@@ -843,13 +900,17 @@ __device__ void place_by_colour(const ClassView& cv, int n)
 }
 
 
+// one block of threads per class
 __global__ void __launch_bounds__(1024) k_colour(DevCloth c, Buffers b, ColourArgs a)
 {
-    for (int k = 0; k < 4; k++)
+    const ClassView& cv = a.cls[blockIdx.x];
+    if (*cv.count == 0)
     {
-        if (a.cls[k].kind <= 1) static_colour_class(c, b, a.cls[k]);
-        else colour_class(c, b, a.cls[k], c.status);
+        if (threadIdx.x <= MAX_COLOURS) cv.start[threadIdx.x] = 0;
+        return;
     }
+    if (cv.kind <= 1) static_colour_class(c, b, cv);
+    else colour_class(c, b, cv, b.colouring[cv.kind - 2], c.status);
 }
 
 // residual-target mode, per-colour path: after iteration `iter` the residual
@@ -1947,7 +2008,7 @@ void launch_tri_edge_colliders(cudaStream_t s, const DevCloth& c, const SolverPa
 
 void launch_colour_contacts(cudaStream_t s, const DevCloth& c, const Buffers& b)
 {
-    k_colour<<<1, 1024, 0, s>>>(c, b, colour_args(b));
+    k_colour<<<4, 1024, 0, s>>>(c, b, colour_args(b));
 }
 
 
