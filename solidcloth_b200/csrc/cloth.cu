@@ -465,6 +465,8 @@ void ClothModel::release_device()
     for (void* p : allocs) cudaFree(p);
     allocs.clear();
     dc = DevCloth{};
+    if (stageRead) { cudaEventSynchronize(stageRead); cudaEventDestroy(stageRead); }
+    stageRead = nullptr;
     if (stageHost) cudaFreeHost(stageHost);
     stageHost = nullptr;
     stageDev = nullptr;          // one of allocs
@@ -478,6 +480,12 @@ bool ClothModel::ensure_stage()
     {
         cudaGetLastError();
         stageHost = nullptr;
+        return false;
+    }
+    if (!stageRead && cudaEventCreateWithFlags(&stageRead, cudaEventDisableTiming) != cudaSuccess)
+    {
+        cudaGetLastError();
+        stageRead = nullptr;
         return false;
     }
     stageDev = (float*)dalloc(sizeof(float) * 10 * (size_t)N);
@@ -1736,13 +1744,14 @@ void ClothModel::set_state(const float* pos, const float* prev, const float* vel
     memcpy(hprev.data(), prev, sizeof(float) * 3 * n);
     memcpy(hvel.data(), vel, sizeof(float) * 3 * n);
     if (!ensure_stage()) { upload_state(s); return; }
+    cudaEventSynchronize(stageRead);     // the staging buffer's last upload
     memcpy(stageHost, pos, sizeof(float) * 3 * n);
     memcpy(stageHost + 3 * n, vel, sizeof(float) * 3 * n);
     memcpy(stageHost + 6 * n, prev, sizeof(float) * 3 * n);
     memcpy(stageHost + 9 * n, invMass.data(), sizeof(float) * n);
     cudaMemcpyAsync(stageDev, stageHost, sizeof(float) * 10 * n, cudaMemcpyHostToDevice, s);
+    cudaEventRecord(stageRead, s);
     launch_unpack_state(s, dc, stageDev);
-    cudaStreamSynchronize(s);            // the staging buffer is reused by the next transfer
 }
 
 // Contact buffers depend on the world's colliders, the collision flags and the
@@ -2313,7 +2322,8 @@ void ClothPatch::record_substep(float h)
     const DevCloth& c = m.dc;
     Buffers& b = m.buf;
     cudaStream_t s = stream;
-    launch_predict(s, c, P);
+    const TileView* tiles = m.choice.kind == SOLVE_TILE && m.tilePlan.valid && m.prm.solverType == 1 ? &m.tilePlan.view : nullptr;
+    launch_predict(s, c, P, tiles, recordingSubstep == 0);
     const bool self = (m.prm.flags & CF_SELF) != 0, ccd = m.prm.ccd;
     // ClothModel::DetectCollisions (Physics/ClothCollision.cpp:17-48)
     if (ccd)
@@ -2356,8 +2366,9 @@ void ClothPatch::record_substep(float h)
         launch_ccd(s, side, evFork, evJoin, c, P, b, m.sweptTris, m.sweptEdges, m.sweptVerts, marks);
     }
     if (self || ccd) launch_compact_self(s, c, P, b, self, ccd);
-    else cudaMemsetAsync(b.stCount, 0, 2 * sizeof(int), s);
-    launch_colour_contacts(s, c, b);
+    // no contact class can have entries: their counts and colours stay zero, as allocated
+    const bool features = (m.prm.flags & (CF_TRIANGLES | CF_EDGES)) && m.feature_colliders() > 0;
+    if (self || ccd || features) launch_colour_contacts(s, c, b);
     // learned warm start (no reference counterpart): record the features and the
     // predicted positions, and / or move the particles by the network's correction
     const size_t sub = (size_t)recordingSubstep;
@@ -2365,7 +2376,7 @@ void ClothPatch::record_substep(float h)
     if (learn) launch_mlp_features(s, c, b, m.sampleFeat ? m.sampleFeat + sub * m.N * MLP_IN : nullptr);
     if (m.warmStart && m.mlpPrm) launch_mlp_warm(s, c, b, m.mlpPrm, m.mlpPrm + MLP_NPARAM);
     // ClothModelPBD::SolveGS (Physics/ClothPBD.cpp:324-369)
-    launch_reset_gs(s, c, m.choice.kind == SOLVE_TILE ? &m.tilePlan.view : nullptr);
+    if (!tiles) launch_reset_gs(s, c);
     timing_mark(SEC_GS, false, s);
     record_solve(s, P, m.choice);
     timing_mark(SEC_GS, true, s);

@@ -179,6 +179,7 @@ public:
     // pinned host / device staging of the packed state (10 N floats), made on first use
     float* stageHost = nullptr;
     float* stageDev = nullptr;
+    cudaEvent_t stageRead = nullptr;            // the staging buffer's last upload has read it
     bool ensure_stage();
     SolverParams solver_params(float h) const;
     // batch of independent clothes (empty: one cloth): first particle / triangle /

@@ -79,7 +79,9 @@ struct Buffers
     int numMeshes;
 };
 
-void launch_predict(cudaStream_t s, const DevCloth& c, const SolverParams& P);
+struct TileView;
+// tv: the tile solver's view when it runs this substep; first: of its frame
+void launch_predict(cudaStream_t s, const DevCloth& c, const SolverParams& P, const TileView* tv, bool first);
 // state <-> 10 N floats: positions, velocities, previous positions (xyz), inverse masses
 void launch_pack_state(cudaStream_t s, const DevCloth& c, float* out);
 void launch_unpack_state(cudaStream_t s, const DevCloth& c, const float* in);
@@ -112,7 +114,6 @@ void launch_ccd(cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t
 // self-contact lists: proximity contacts (self) compacted, then the continuous
 // hits appended (ccd)
 void launch_compact_self(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, bool self, bool ccd);
-struct TileView;
 // clears the solver's error and exit words; with a tile plan also its exchange tags
 void launch_reset_gs(cudaStream_t s, const DevCloth& c, const TileView* tv = nullptr);
 

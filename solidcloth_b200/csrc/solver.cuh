@@ -1666,6 +1666,7 @@ __global__ void __launch_bounds__(NT, 1) k_gs_tile(DevCloth c, SolverParams P, B
     __shared__ int sOff[3][65];
     __shared__ unsigned sRes;
     __shared__ int sCnt[2][MAX_COLOURS];
+    if (blockIdx.x == 0 && threadIdx.x == 0) c.scal[0] = 0.f;      // for the next prediction; the detection is done
     if (!guard_open(guard, ca)) return;
     const int tid = (int)threadIdx.x;
     const bool track = !P.fixedIterations;

@@ -28,10 +28,16 @@ namespace sc {
 // ClothModelPBD::Step, symplectic Euler part (Physics/ClothPBD.cpp:257-266);
 // also the max |pos - prev| used by the collision thresholds
 // (Physics/ClothCollision.cpp:91-100).
-__global__ void k_predict(DevCloth c, SolverParams P)
+// With a tile plan it also clears the solver's words and its exchange tags (no
+// exchange of an earlier substep may satisfy a wait of this one): on small clothes a
+// substep is bound by its launches, and these were two of four.
+__global__ void k_predict(DevCloth c, SolverParams P, float4* xch, unsigned long long* xred, int words, bool clear)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (clear && i < 9) c.scal[1 + i] = 0.f;
+    if (i < words) xred[i] = 0ull;
     if (i >= c.N) return;
+    if (xch) { xch[i].w = 0.f; xch[c.N + i].w = 0.f; }
     float4 p = c.pos[i];
     c.prev[i] = make_float4(p.x, p.y, p.z, 0.f);
     if (p.w == 0.f) return;
@@ -1944,10 +1950,12 @@ void launch_unpack_state(cudaStream_t s, const DevCloth& c, const float* in)
     k_unpack_state<<<blocks_for(c.N), 256, 0, s>>>(c, in);
 }
 
-void launch_predict(cudaStream_t s, const DevCloth& c, const SolverParams& P)
+void launch_predict(cudaStream_t s, const DevCloth& c, const SolverParams& P, const TileView* tv, bool first)
 {
-    cudaMemsetAsync(c.scal, 0, sizeof(float), s);
-    k_predict<<<blocks_for(c.N), 256, 0, s>>>(c, P);
+    // the travel maximum: cleared by the tile solver once the detection has read it
+    if (!tv || first) cudaMemsetAsync(c.scal, 0, sizeof(float), s);
+    const int words = tv && tv->xch ? 2 * tv->nTiles : 0;
+    k_predict<<<blocks_for(std::max(c.N, words)), 256, 0, s>>>(c, P, tv ? tv->xch : nullptr, tv ? tv->xred : nullptr, words, tv != nullptr);
 }
 
 void launch_velocity(cudaStream_t s, const DevCloth& c, const SolverParams& P)
@@ -1985,7 +1993,8 @@ void launch_tri_edge_colliders(cudaStream_t s, const DevCloth& c, const SolverPa
         if (flags & CF_EDGES) { k_edge_colliders<<<blocks_for(c.E, 128), 128, 0, s>>>(c, P, b, g, ei); ei++; }
         if (flags & CF_TRIANGLES) { k_tri_colliders<<<blocks_for(c.T, 128), 128, 0, s>>>(c, P, b, g, ti); ti++; }
     }
-    // compaction in (collider, item) order
+    // compaction in (collider, item) order (without such contacts the counts stay zero,
+    // as they were allocated)
     if (ti > 0)
     {
         int n = ti * c.T;
@@ -1993,7 +2002,6 @@ void launch_tri_edge_colliders(cudaStream_t s, const DevCloth& c, const SolverPa
         k_compact<TC><<<blocks_for(n), 256, 0, s>>>(b.tcFlag, b.scanOff, b.tcSlot, 1, b.tcList, n, nullptr, b.tcCap, c.status, ST_CONTACT_OVERFLOW, b.tcFlag);
         k_add_counts<<<1, 32, 0, s>>>(b.tcCount, b.tcCount, nullptr, b.tcCap);
     }
-    else cudaMemsetAsync(b.tcCount, 0, sizeof(int), s);
     if (ei > 0)
     {
         int n = ei * c.E;
@@ -2001,7 +2009,6 @@ void launch_tri_edge_colliders(cudaStream_t s, const DevCloth& c, const SolverPa
         k_compact<EC><<<blocks_for(n), 256, 0, s>>>(b.ecFlag, b.scanOff, b.ecSlot, 1, b.ecList, n, nullptr, b.ecCap, c.status, ST_CONTACT_OVERFLOW, b.ecFlag);
         k_add_counts<<<1, 32, 0, s>>>(b.ecCount, b.ecCount, nullptr, b.ecCap);
     }
-    else cudaMemsetAsync(b.ecCount, 0, sizeof(int), s);
 }
 
 
@@ -2111,19 +2118,19 @@ void launch_residual(cudaStream_t s, const DevCloth& c, unsigned* out)
     k_residual<<<2 * 148, 256, 0, s>>>(c, out);
 }
 
-// one launch in the place of the memset: no exchange of an earlier substep may
-// satisfy a wait of this one
+// what k_predict clears for the tile solver, for a solve that is timed by itself
 __global__ void k_tile_reset(DevCloth c, TileView tv)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < 9) c.scal[1 + i] = 0.f;
+    if (!tv.xch) return;
     if (i < 2 * tv.nTiles) tv.xred[i] = 0ull;
     if (i < 2 * tv.N) tv.xch[i].w = 0.f;
 }
 
 void launch_reset_gs(cudaStream_t s, const DevCloth& c, const TileView* tv)
 {
-    if (tv && tv->xch) k_tile_reset<<<blocks_for(std::max(2 * tv->N, 2 * tv->nTiles)), 256, 0, s>>>(c, *tv);
+    if (tv) k_tile_reset<<<blocks_for(std::max(2 * tv->N, 2 * tv->nTiles)), 256, 0, s>>>(c, *tv);
     else cudaMemsetAsync(c.scal + 1, 0, sizeof(float) * 9, s);
 }
 
