@@ -7,9 +7,17 @@
 // Every contraction runs on the fifth-generation tensor cores (tc05.cuh): tiles
 // of 128 particles (rows) per CTA, BF16 operands staged in shared memory, FP32
 // accumulators in tensor memory, one thread issuing tcgen05.mma and the CTA
-// waiting on an mbarrier that tcgen05.commit arrives on; the four warps read
-// their 32 rows back with tcgen05.ld for the bias / GELU epilogue, which writes
-// the next layer's BF16 operand tile. Training runs the same forward, then the
+// waiting on an mbarrier that tcgen05.commit arrives on; the eight warps read
+// 32 rows by 32 columns each back with tcgen05.ld for the bias / GELU epilogue,
+// which writes the next layer's BF16 operand tile.
+//
+// What bounds it: the GELU's tanhf (192 a row, about 30 instructions each, against
+// 2 x 9,200 multiply-adds that the tensor cores do in passing) and the chain of
+// layers of a tile. Eight warps instead of four a tile halve the epilogue of every
+// layer; the weights of layers 2 to 4 are staged, eight at a time, behind layer 1's
+// product. The training pass keeps the GELU's derivative from the forward epilogue
+// in shared memory instead of taking tanhf again. 65,536 rows: forward 31 ->
+// 25 us, gradients and Adam 175 -> 115 us. Training runs the same forward, then the
 // backward on the tensor cores too: dH = dZ W (K-major operands, transposed
 // weights in shared memory) and dW = dZ^T H (the activation tiles read
 // MN-major, summed over the CTA's tiles in tensor memory before one atomic
@@ -30,6 +38,7 @@ constexpr int ML_W4 = ML_B3 + ML_H, ML_B4 = ML_W4 + ML_OUT * ML_H;
 constexpr int ML_NPARAM = ML_B4 + ML_OUT;     // 9347
 constexpr int ML_NNORM = 2 * ML_IN + ML_OUT;  // feature mean, feature 1/std, output scale
 constexpr int ML_ROWS = 128;                  // rows (particles / samples) per tile = MMA M
+constexpr int ML_THREADS = 256;               // row threadIdx.x & 127, columns 32 (threadIdx.x >> 7) onwards
 
 // instruction descriptors: M = 128 rows, N = 64 hidden units or 16 (padded outputs
 // / padded inputs); forward and dH operands K-major, weight-gradient operands MN-major
@@ -62,24 +71,64 @@ __device__ __forceinline__ void put_bf16(unsigned char* tile, int r, int k, int 
     *reinterpret_cast<__nv_bfloat16*>(tile + core_off(r, k, K)) = __float2bfloat16_rn(v);
 }
 
-__device__ __forceinline__ void mlp_tc_load(MlpTcWeights& s, MlpTcTrans* t, const float* prm, const float* norm)
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
+{
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);   // .x = lo (lower 16 bits)
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ void put_chunk8(unsigned char* tile, int r, int k, int K, const float* x)
+{
+    uint4 q;
+    q.x = pack_bf16(x[0], x[1]); q.y = pack_bf16(x[2], x[3]); q.z = pack_bf16(x[4], x[5]); q.w = pack_bf16(x[6], x[7]);
+    *reinterpret_cast<uint4*>(tile + core_off(r, k, K)) = q;
+}
+// eight consecutive floats; the caller's vector may start at any float
+__device__ __forceinline__ void ld8(const float* p, float* x)
+{
+    if ((reinterpret_cast<unsigned long long>(p) & 15ull) == 0ull)
+    {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+    }
+    else
+        for (int k = 0; k < 8; k++) x[k] = __ldg(p + k);
+}
+
+// what layer 1 needs, and the rest: 64 x 64 matrices in chunks of eight along a row
+__device__ __forceinline__ void mlp_tc_load_first(MlpTcWeights& s, const float* prm, const float* norm)
 {
     for (int k = threadIdx.x; k < 64 * 16; k += blockDim.x)
     {
         const int o = k / 16, i = k % 16;
         put_bf16(s.w1, o, i, 16, i < ML_IN ? prm[ML_W1 + o * ML_IN + i] : 0.f);
     }
-    for (int k = threadIdx.x; k < 64 * 64; k += blockDim.x)
+    if (threadIdx.x < ML_IN) { s.mean[threadIdx.x] = norm[threadIdx.x]; s.istd[threadIdx.x] = norm[ML_IN + threadIdx.x]; }
+    if (threadIdx.x < ML_OUT) s.oscale[threadIdx.x] = norm[2 * ML_IN + threadIdx.x];
+}
+
+__device__ __forceinline__ void mlp_tc_load_rest(MlpTcWeights& s, MlpTcTrans* t, const float* prm)
+{
+#pragma unroll
+    for (int k = threadIdx.x; k < 512; k += ML_THREADS)
     {
-        const int o = k / 64, i = k % 64;
-        put_bf16(s.w2, o, i, 64, prm[ML_W2 + k]);
-        put_bf16(s.w3, o, i, 64, prm[ML_W3 + k]);
-        if (t)
-        {
-            put_bf16(t->w2t, i, o, 64, prm[ML_W2 + k]);
-            put_bf16(t->w3t, i, o, 64, prm[ML_W3 + k]);
-        }
+        const int o = k >> 3, i = (k & 7) * 8;
+        float a[8], b[8];
+        ld8(prm + ML_W2 + o * 64 + i, a);
+        ld8(prm + ML_W3 + o * 64 + i, b);
+        put_chunk8(s.w2, o, i, 64, a);
+        put_chunk8(s.w3, o, i, 64, b);
     }
+    if (t)
+#pragma unroll
+        for (int k = threadIdx.x; k < 512; k += ML_THREADS)
+        {
+            // the transposes: eight outputs of one input (neighbouring threads: neighbouring inputs)
+            const int i = k & 63, o = (k >> 6) * 8;
+            float a[8], b[8];
+            for (int j = 0; j < 8; j++) { a[j] = __ldg(prm + ML_W2 + (o + j) * 64 + i); b[j] = __ldg(prm + ML_W3 + (o + j) * 64 + i); }
+            put_chunk8(t->w2t, i, o, 64, a);
+            put_chunk8(t->w3t, i, o, 64, b);
+        }
     for (int k = threadIdx.x; k < 16 * 64; k += blockDim.x)
     {
         const int o = k / 64, i = k % 64;
@@ -92,8 +141,6 @@ __device__ __forceinline__ void mlp_tc_load(MlpTcWeights& s, MlpTcTrans* t, cons
         s.b1[k] = prm[ML_B1 + k]; s.b2[k] = prm[ML_B2 + k]; s.b3[k] = prm[ML_B3 + k];
     }
     if (threadIdx.x < 16) s.b4[threadIdx.x] = threadIdx.x < ML_OUT ? prm[ML_B4 + threadIdx.x] : 0.f;
-    if (threadIdx.x < ML_IN) { s.mean[threadIdx.x] = norm[threadIdx.x]; s.istd[threadIdx.x] = norm[ML_IN + threadIdx.x]; }
-    if (threadIdx.x < ML_OUT) s.oscale[threadIdx.x] = norm[2 * ML_IN + threadIdx.x];
 }
 
 // GELU, tanh form, and its derivative
@@ -102,19 +149,14 @@ __device__ __forceinline__ float gelu(float x)
     const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
     return 0.5f * x * (1.f + tanhf(u));
 }
-__device__ __forceinline__ float gelu_grad(float x)
+// the value and the derivative, of one tanhf
+__device__ __forceinline__ float gelu_and_grad(float x, float& grad)
 {
     const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
     const float t = tanhf(u);
-    return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * 0.7978845608028654f * (1.f + 3.f * 0.044715f * x * x);
+    grad = 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * 0.7978845608028654f * (1.f + 3.f * 0.044715f * x * x);
+    return 0.5f * x * (1.f + t);
 }
-
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
-{
-    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);   // .x = lo (lower 16 bits)
-    return *reinterpret_cast<const uint32_t*>(&v);
-}
-
 
 // this thread's row of a 16-column operand tile (K = 16) from 16 floats
 __device__ __forceinline__ void put_row16(unsigned char* tile, int r, const float* x)
@@ -127,8 +169,9 @@ __device__ __forceinline__ void put_row16(unsigned char* tile, int r, const floa
 }
 
 // 32 accumulator columns of this thread's row (tensor memory at taddr) plus bias,
-// through GELU, into columns [c0, c0 + 32) of row r of a K-column operand tile
-__device__ __forceinline__ void epilogue_gelu32(uint32_t taddr, const float* bias, unsigned char* tile, int r, int c0, int K)
+// through GELU, into columns [c0, c0 + 32) of row r of a K-column operand tile;
+// grad (optional): the derivatives, [column][row]
+__device__ __forceinline__ void epilogue_gelu32(uint32_t taddr, const float* bias, unsigned char* tile, int r, int c0, int K, float* grad)
 {
     uint32_t v[32];
     tc_ld32(taddr, v);
@@ -138,10 +181,14 @@ __device__ __forceinline__ void epilogue_gelu32(uint32_t taddr, const float* bia
     {
         float h[8];
 #pragma unroll
-        for (int j = 0; j < 8; j++) h[j] = gelu(__uint_as_float(v[8 * c + j]) + bias[c0 + 8 * c + j]);
-        uint4 q;
-        q.x = pack_bf16(h[0], h[1]); q.y = pack_bf16(h[2], h[3]); q.z = pack_bf16(h[4], h[5]); q.w = pack_bf16(h[6], h[7]);
-        *reinterpret_cast<uint4*>(tile + core_off(r, c0 + 8 * c, K)) = q;
+        for (int j = 0; j < 8; j++)
+        {
+            const int col = c0 + 8 * c + j;
+            const float x = __uint_as_float(v[8 * c + j]) + bias[col];
+            if (grad) { float g; h[j] = gelu_and_grad(x, g); grad[col * ML_ROWS + r] = g; }
+            else h[j] = gelu(x);
+        }
+        put_chunk8(tile, r, c0 + 8 * c, K, h);
     }
 }
 
@@ -163,28 +210,31 @@ struct TcCtx
 // Forward of the CTA's 128-row tile whose normalised inputs (BF16, K = 16) are
 // already in x: hidden layers into tensor-memory columns zcol[0..2] (pre-
 // activations, no bias), their GELU outputs as operand tiles h[0..2] (each may be
-// the same buffer when they need not survive), outputs into column ycol. Returns
-// false if a wait gave up.
-__device__ __forceinline__ bool mlp_tc_forward(TcCtx& t, const MlpTcWeights& s, unsigned char* x,
-                                               unsigned char* const* h, const uint32_t* zcol, uint32_t ycol)
+// the same buffer when they need not survive), outputs into column ycol; grad
+// (optional): the three layers' GELU derivatives. `behind` runs between layer 1's
+// issue and its wait. Returns false if a wait gave up.
+template <class F>
+__device__ __forceinline__ bool mlp_tc_forward(TcCtx& t, const MlpTcWeights& s, unsigned char* x, unsigned char* const* h,
+                                               const uint32_t* zcol, uint32_t ycol, float* grad, F&& behind)
 {
-    const int r = threadIdx.x;
+    const int r = threadIdx.x & (ML_ROWS - 1), c0 = 32 * (threadIdx.x >> 7);
     const uint32_t lanes = tmem_lane_base(t.tmem);
     tc_sync_for_mma();
-    if (r == 0)
+    if (threadIdx.x == 0)
     {
         umma_bf16(t.tmem + zcol[0], desc_kmajor(smem_addr(x), 16), desc_kmajor(smem_addr(s.w1), 16), IDESC_N64, 0);
         umma_commit(t.mbar);
     }
+    behind();
     if (!t.wait()) return false;
     const float* bias[3] = {s.b1, s.b2, s.b3};
     const unsigned char* w[3] = {s.w2, s.w3, s.w4};
+#pragma unroll
     for (int l = 0; l < 3; l++)
     {
-        epilogue_gelu32(lanes + zcol[l], bias[l], h[l], r, 0, 64);
-        epilogue_gelu32(lanes + zcol[l] + 32, bias[l], h[l], r, 32, 64);
+        epilogue_gelu32(lanes + zcol[l] + c0, bias[l], h[l], r, c0, 64, grad ? grad + l * ML_H * ML_ROWS : nullptr);
         tc_sync_for_mma();
-        if (r == 0)
+        if (threadIdx.x == 0)
         {
             const uint32_t dst = l < 2 ? zcol[l + 1] : ycol;
             for (int ks = 0; ks < 4; ks++)
@@ -276,38 +326,45 @@ struct MlpArgs
 // warm start: features -> MLP -> position correction, tiles of 128 particles
 // (one per thread), CTAs persistent over the tiles; pinned particles are left
 // alone. A wait that gives up sets ST_TC_TIMEOUT and ends the CTA's work.
-__global__ void __launch_bounds__(128) k_mlp_warm(DevCloth c, Buffers b, MlpArgs ml)
+__global__ void __launch_bounds__(ML_THREADS, 4) k_mlp_warm(DevCloth c, Buffers b, MlpArgs ml)
 {
     __shared__ MlpTcInferSmem s;
-    mlp_tc_load(s.w, nullptr, ml.prm, ml.norm);
+    mlp_tc_load_first(s.w, ml.prm, ml.norm);
     TcCtx t = mlp_tc_begin(s, 128);
     unsigned char* hs[3] = {s.h, s.h, s.h};
     const uint32_t zc[3] = {0, 64, 0};
     const int tiles = (c.N + ML_ROWS - 1) / ML_ROWS;
+    bool loaded = false;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
     {
-        const int i = tile * ML_ROWS + (int)threadIdx.x;
-        float f[16];
-        if (i < c.N) ml_features(c, b, i, f);
+        const int i = tile * ML_ROWS + (int)(threadIdx.x & (ML_ROWS - 1));
+        if (threadIdx.x < ML_ROWS)
+        {
+            float f[16];
+            if (i < c.N) ml_features(c, b, i, f);
 #pragma unroll
-        for (int k = 0; k < 16; k++) f[k] = (i < c.N && k < ML_IN) ? (f[k] - s.w.mean[k]) * s.w.istd[k] : 0.f;
-        put_row16(s.x, threadIdx.x, f);
-        if (!mlp_tc_forward(t, s.w, s.x, hs, zc, 64))
+            for (int k = 0; k < 16; k++) f[k] = (i < c.N && k < ML_IN) ? (f[k] - s.w.mean[k]) * s.w.istd[k] : 0.f;
+            put_row16(s.x, threadIdx.x, f);
+        }
+        if (!mlp_tc_forward(t, s.w, s.x, hs, zc, 64, nullptr, [&] { if (!loaded) mlp_tc_load_rest(s.w, nullptr, ml.prm); loaded = true; }))
         {
             if (threadIdx.x == 0) atomicOr(c.status, ST_TC_TIMEOUT);
             break;
         }
-        float y[ML_OUT];
-        mlp_tc_outputs(t, s.w, 64, y);
-        if (i < c.N)
+        if (threadIdx.x < ML_ROWS)
         {
-            float4 p = c.pos[i];
-            if (p.w > 0.f)
+            float y[ML_OUT];
+            mlp_tc_outputs(t, s.w, 64, y);
+            if (i < c.N)
             {
-                p.x += y[0] * s.w.oscale[0];
-                p.y += y[1] * s.w.oscale[1];
-                p.z += y[2] * s.w.oscale[2];
-                c.pos[i] = p;
+                float4 p = c.pos[i];
+                if (p.w > 0.f)
+                {
+                    p.x += y[0] * s.w.oscale[0];
+                    p.y += y[1] * s.w.oscale[1];
+                    p.z += y[2] * s.w.oscale[2];
+                    c.pos[i] = p;
+                }
             }
         }
     }
@@ -340,124 +397,103 @@ __global__ void k_mlp_targets(DevCloth c, float* target)
     if (target) { target[3 * (size_t)i] = dx; target[3 * (size_t)i + 1] = dy; target[3 * (size_t)i + 2] = dz; }
 }
 
+// one raw feature row; the caller's array may start at any float
+__device__ __forceinline__ void ld_row12(const float* p, float* f)
+{
+    if ((reinterpret_cast<unsigned long long>(p) & 15ull) == 0ull)
+    {
+        const float4* q = reinterpret_cast<const float4*>(p);
+        const float4 a = __ldg(q), b = __ldg(q + 1), d = __ldg(q + 2);
+        f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+        f[8] = d.x; f[9] = d.y; f[10] = d.z; f[11] = d.w;
+    }
+    else
+        for (int k = 0; k < ML_IN; k++) f[k] = __ldg(p + k);
+}
+
+// this tile's normalised inputs into x (rows past S: zero)
+__device__ __forceinline__ void put_inputs(const MlpTcWeights& w, unsigned char* x, const float* X, int row, int S)
+{
+    float f[16];
+    if (row < S) ld_row12(X + (size_t)row * ML_IN, f);
+#pragma unroll
+    for (int k = 0; k < 16; k++) f[k] = (row < S && k < ML_IN) ? (f[k] - w.mean[k]) * w.istd[k] : 0.f;
+    put_row16(x, threadIdx.x, f);
+}
+
 // forward over raw feature rows (S x 12) -> outputs (S x 3, output scale applied)
-__global__ void __launch_bounds__(128) k_mlp_forward(const float* X, int S, MlpArgs ml, float* Y, int* status)
+__global__ void __launch_bounds__(ML_THREADS, 4) k_mlp_forward(const float* X, int S, MlpArgs ml, float* Y, int* status)
 {
     __shared__ MlpTcInferSmem s;
-    mlp_tc_load(s.w, nullptr, ml.prm, ml.norm);
+    mlp_tc_load_first(s.w, ml.prm, ml.norm);
     TcCtx t = mlp_tc_begin(s, 128);
     unsigned char* hs[3] = {s.h, s.h, s.h};
     const uint32_t zc[3] = {0, 64, 0};
     const int tiles = (S + ML_ROWS - 1) / ML_ROWS;
+    bool loaded = false;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
     {
-        const int r = tile * ML_ROWS + (int)threadIdx.x;
-        float f[16];
-#pragma unroll
-        for (int k = 0; k < 16; k++) f[k] = (r < S && k < ML_IN) ? (X[(size_t)r * ML_IN + k] - s.w.mean[k]) * s.w.istd[k] : 0.f;
-        put_row16(s.x, threadIdx.x, f);
-        if (!mlp_tc_forward(t, s.w, s.x, hs, zc, 64))
+        const int r = tile * ML_ROWS + (int)(threadIdx.x & (ML_ROWS - 1));
+        if (threadIdx.x < ML_ROWS) put_inputs(s.w, s.x, X, r, S);
+        if (!mlp_tc_forward(t, s.w, s.x, hs, zc, 64, nullptr, [&] { if (!loaded) mlp_tc_load_rest(s.w, nullptr, ml.prm); loaded = true; }))
         {
             if (threadIdx.x == 0 && status) atomicOr(status, 1);
             break;
         }
-        float y[ML_OUT];
-        mlp_tc_outputs(t, s.w, 64, y);
-        if (r < S)
-            for (int k = 0; k < ML_OUT; k++) Y[(size_t)r * ML_OUT + k] = y[k] * s.w.oscale[k];
+        if (threadIdx.x < ML_ROWS)
+        {
+            float y[ML_OUT];
+            mlp_tc_outputs(t, s.w, 64, y);
+            if (r < S)
+                for (int k = 0; k < ML_OUT; k++) Y[(size_t)r * ML_OUT + k] = y[k] * s.w.oscale[k];
+        }
     }
     tmem_free(t.tmem, 128);
 }
 
 // ------------------------------------------------------------ training
-// Sum over a warp of 64 per-lane values: a butterfly in which each step halves
-// the columns a lane keeps, so that lane l ends with the sums of columns 2l and
-// 2l + 1 (62 shuffles instead of 64 x 5).
-__device__ __forceinline__ float2 warp_colsum64(const float (&v)[64])
+// Sum over a warp of 32 per-lane values: a butterfly in which each step halves the
+// columns a lane keeps, so that lane l ends with the sum of column l (31 shuffles
+// instead of 32 x 5).
+__device__ __forceinline__ float warp_colsum32(const float (&v)[32])
 {
     const int lane = threadIdx.x & 31;
-    float a[32];
+    float a[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++)
     {
         const bool hi = lane & 16;
-#pragma unroll
-        for (int j = 0; j < 32; j++)
-        {
-            const float keep = hi ? v[j + 32] : v[j], send = hi ? v[j] : v[j + 32];
-            a[j] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-        }
+        a[j] = (hi ? v[j + 16] : v[j]) + __shfl_xor_sync(0xffffffffu, hi ? v[j] : v[j + 16], 16);
     }
-    float b16[16];
-    {
-        const bool hi = lane & 8;
 #pragma unroll
-        for (int j = 0; j < 16; j++)
-        {
-            const float keep = hi ? a[j + 16] : a[j], send = hi ? a[j] : a[j + 16];
-            b16[j] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-        }
-    }
-    float c8[8];
+    for (int o = 8; o > 0; o >>= 1)
     {
-        const bool hi = lane & 4;
+        const bool hi = lane & o;
 #pragma unroll
         for (int j = 0; j < 8; j++)
-        {
-            const float keep = hi ? b16[j + 8] : b16[j], send = hi ? b16[j] : b16[j + 8];
-            c8[j] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-        }
+            if (j < o)
+            {
+                const float keep = hi ? a[j + o] : a[j], send = hi ? a[j] : a[j + o];
+                a[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
     }
-    float d4[4];
-    {
-        const bool hi = lane & 2;
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-        {
-            const float keep = hi ? c8[j + 4] : c8[j], send = hi ? c8[j] : c8[j + 4];
-            d4[j] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-        }
-    }
-    float e2[2];
-    {
-        const bool hi = lane & 1;
-#pragma unroll
-        for (int j = 0; j < 2; j++)
-        {
-            const float keep = hi ? d4[j + 2] : d4[j], send = hi ? d4[j] : d4[j + 2];
-            e2[j] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
-        }
-    }
-    return make_float2(e2[0], e2[1]);
+    return a[0];
 }
 
-// dZ = dH * gelu'(Z + b) for this thread's row: dH and Z (no bias) from tensor
-// memory, dZ as BF16 into columns 0..63 of row r of the 128-column tile d, and
-// its per-column sums over the warp into bsum (lane l: columns 2l, 2l + 1)
-__device__ __forceinline__ void epilogue_dz(uint32_t lanes, uint32_t dhCol, uint32_t zCol, const float* bias,
-                                            unsigned char* d, int r, float2& bsum)
+// dZ = dH * gelu'(Z + b) for 32 columns from c0 of this thread's row: dH from tensor
+// memory, the derivatives kept by the forward epilogue; dZ as BF16 into row r of the
+// 128-column tile d, and its column sums over the warp into bsum (lane l: column c0 + l)
+__device__ __forceinline__ void epilogue_dz(uint32_t lanes, uint32_t dhCol, const float* grad, unsigned char* d, int r, int c0, float& bsum)
 {
-    float dz[64];
+    float dz[32];
+    uint32_t vh[32];
+    tc_ld32(lanes + dhCol + c0, vh);
+    tc_wait_ld();
 #pragma unroll
-    for (int half = 0; half < 2; half++)
-    {
-        uint32_t vh[32], vz[32];
-        tc_ld32(lanes + dhCol + 32 * half, vh);
-        tc_ld32(lanes + zCol + 32 * half, vz);
-        tc_wait_ld();
+    for (int j = 0; j < 32; j++) dz[j] = __uint_as_float(vh[j]) * grad[(c0 + j) * ML_ROWS + r];
 #pragma unroll
-        for (int j = 0; j < 32; j++)
-            dz[32 * half + j] = __uint_as_float(vh[j]) * gelu_grad(__uint_as_float(vz[j]) + bias[32 * half + j]);
-    }
-#pragma unroll
-    for (int c = 0; c < 8; c++)
-    {
-        uint4 q;
-        q.x = pack_bf16(dz[8 * c], dz[8 * c + 1]); q.y = pack_bf16(dz[8 * c + 2], dz[8 * c + 3]);
-        q.z = pack_bf16(dz[8 * c + 4], dz[8 * c + 5]); q.w = pack_bf16(dz[8 * c + 6], dz[8 * c + 7]);
-        *reinterpret_cast<uint4*>(d + core_off(r, 8 * c, 128)) = q;
-    }
-    const float2 s2 = warp_colsum64(dz);
-    bsum.x += s2.x;
-    bsum.y += s2.y;
+    for (int c = 0; c < 4; c++) put_chunk8(d, r, c0 + 8 * c, 128, dz + 8 * c);
+    bsum += warp_colsum32(dz);
 }
 
 // Tensor-memory columns of the training kernel (512 allocated)
@@ -473,6 +509,7 @@ struct __align__(128) MlpTcTrainSmem
     // dY / dZ tile, 128 columns: 0..63 in use, 64..127 zero (the padded rows of
     // the M = 128 weight-gradient products)
     unsigned char d[ML_ROWS * 128 * 2];
+    float grad[3 * ML_H * ML_ROWS];       // GELU derivatives of the three hidden layers, [layer][column][row]
     unsigned long long mbar;
     uint32_t tmemSlot;
 };
@@ -482,12 +519,12 @@ struct __align__(128) MlpTcTrainSmem
 // loss[0] (both zeroed by the caller). CTAs are persistent over 128-row tiles;
 // the weight gradients of all their tiles are summed in tensor memory and added
 // to grad[] once per CTA. A wait that gives up sets *status (if given).
-__global__ void __launch_bounds__(128) k_mlp_grad(const float* X, const float* T, int S, MlpArgs ml, float* grad,
-                                                  float* loss, int* status)
+__global__ void __launch_bounds__(ML_THREADS) k_mlp_grad(const float* X, const float* T, int S, MlpArgs ml, float* grad,
+                                                         float* loss, int* status)
 {
     extern __shared__ __align__(1024) unsigned char dyn[];
     MlpTcTrainSmem& s = *reinterpret_cast<MlpTcTrainSmem*>(dyn);
-    mlp_tc_load(s.w, &s.t, ml.prm, ml.norm);
+    mlp_tc_load_first(s.w, ml.prm, ml.norm);
     for (int k = threadIdx.x; k < ML_ROWS * 128 * 2 / 16; k += blockDim.x)
         reinterpret_cast<uint4*>(s.d)[k] = make_uint4(0u, 0u, 0u, 0u);
     TcCtx t;
@@ -495,10 +532,10 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const float* X, const float* T
     t.tmem = tmem_alloc(&s.tmemSlot, 512);
     t.mbar = smem_addr(&s.mbar);
     t.phase = 0;
-    const int r = threadIdx.x, lane = r & 31;
+    const int r = threadIdx.x & (ML_ROWS - 1), lane = threadIdx.x & 31, half = threadIdx.x >> 7, c0 = 32 * half;
     const uint32_t lanes = tmem_lane_base(t.tmem);
     const float inv = 1.f / (float)(S * ML_OUT);
-    float2 db1 = make_float2(0.f, 0.f), db2 = db1, db3 = db1;
+    float db[3] = {0.f, 0.f, 0.f};
     float db4[ML_OUT] = {0.f, 0.f, 0.f}, lsum = 0.f;
     unsigned char* hs[3] = {s.h1, s.h2, s.h3};
     const uint32_t zc[3] = {TM_Z1, TM_Z2, TM_Z3};
@@ -508,39 +545,34 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const float* X, const float* T
     {
         const int row = tile * ML_ROWS + r;
         const bool live = row < S;
-        float f[16];
-#pragma unroll
-        for (int k = 0; k < 16; k++) f[k] = (live && k < ML_IN) ? (X[(size_t)row * ML_IN + k] - s.w.mean[k]) * s.w.istd[k] : 0.f;
-        put_row16(s.x, r, f);
-        if (!(ok = mlp_tc_forward(t, s.w, s.x, hs, zc, TM_Y))) break;
+        if (half == 0) put_inputs(s.w, s.x, X, row, S);
+        if (!(ok = mlp_tc_forward(t, s.w, s.x, hs, zc, TM_Y, s.grad, [&] { if (first) mlp_tc_load_rest(s.w, &s.t, ml.prm); }))) break;
         // output layer: dL/dy (zero for rows past S) into dY columns 0..2
-        float y[ML_OUT], dy[16];
-        mlp_tc_outputs(t, s.w, TM_Y, y);
-#pragma unroll
-        for (int k = 0; k < 16; k++) dy[k] = 0.f;
-        for (int k = 0; k < ML_OUT; k++)
-            if (live)
+        uint4 q0 = make_uint4(0u, 0u, 0u, 0u);
+        if (half == 0)
+        {
+            float y[ML_OUT], dy[ML_OUT] = {0.f, 0.f, 0.f};
+            mlp_tc_outputs(t, s.w, TM_Y, y);
+            for (int k = 0; k < ML_OUT; k++)
+                if (live)
+                {
+                    const float e = y[k] - T[(size_t)row * ML_OUT + k] / s.w.oscale[k];
+                    lsum += e * e * inv;
+                    dy[k] = 2.f * e * inv;
+                }
+            for (int k = 0; k < ML_OUT; k++)
             {
-                const float e = y[k] - T[(size_t)row * ML_OUT + k] / s.w.oscale[k];
-                lsum += e * e * inv;
-                dy[k] = 2.f * e * inv;
+                float v = dy[k];
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                db4[k] += v;
             }
-        for (int k = 0; k < ML_OUT; k++)
-        {
-            float v = dy[k];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            db4[k] += v;
+            q0.x = pack_bf16(dy[0], dy[1]); q0.y = pack_bf16(dy[2], 0.f);
         }
-        {
-            uint4 q0, q1;
-            q0.x = pack_bf16(dy[0], dy[1]); q0.y = pack_bf16(dy[2], 0.f); q0.z = 0u; q0.w = 0u;
-            q1 = make_uint4(0u, 0u, 0u, 0u);
-            *reinterpret_cast<uint4*>(s.d + core_off(r, 0, 128)) = q0;
-            for (int c = 1; c < 8; c++) *reinterpret_cast<uint4*>(s.d + core_off(r, 8 * c, 128)) = q1;
-        }
+        for (int c = 0; c < 4; c++)
+            *reinterpret_cast<uint4*>(s.d + core_off(r, c0 + 8 * c, 128)) = c == 0 ? q0 : make_uint4(0u, 0u, 0u, 0u);
         // dH3 = dY W4 (K = 16) and dW4 += dY^T H3 (sum over the tile's rows)
         tc_sync_for_mma();
-        if (r == 0)
+        if (threadIdx.x == 0)
         {
             umma_bf16(t.tmem + TM_DH, desc_kmajor(smem_addr(s.d), 128), desc_kmajor(smem_addr(s.t.w4t), 16), IDESC_N64, 0);
             for (int ks = 0; ks < ML_ROWS / 16; ks++)
@@ -550,15 +582,15 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const float* X, const float* T
         }
         if (!(ok = t.wait())) break;
         // hidden layers 3, 2, 1: dZ, then dH of the layer below and dW += dZ^T H
-        const float* bias[3] = {s.w.b1, s.w.b2, s.w.b3};
-        float2* dbs[3] = {&db1, &db2, &db3};
         const unsigned char* wt[3] = {nullptr, s.t.w2t, s.t.w3t};
         const uint32_t dwc[3] = {TM_DW1, TM_DW2, TM_DW3};
-        for (int l = 2; l >= 0 && ok; l--)
+#pragma unroll
+        for (int l = 2; l >= 0; l--)
         {
-            epilogue_dz(lanes, TM_DH, zc[l], bias[l], s.d, r, *dbs[l]);
+            if (!ok) break;
+            epilogue_dz(lanes, TM_DH, s.grad + l * ML_H * ML_ROWS, s.d, r, c0, db[l]);
             tc_sync_for_mma();
-            if (r == 0)
+            if (threadIdx.x == 0)
             {
                 if (l > 0)
                     for (int ks = 0; ks < 4; ks++)
@@ -577,40 +609,39 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const float* X, const float* T
         first = false;
     }
     if (!ok && threadIdx.x == 0 && status) atomicOr(status, 1);
-    // this CTA's sums: weight gradients (rows 0..63 = output units: warps 0, 1),
-    // bias gradients (lane l of each warp: units 2l, 2l + 1), loss
+    // this CTA's sums: weight gradients (rows 0..63 = output units), bias gradients
+    // (lane l: unit c0 + l), loss. Tensor-memory loads are warp-collective: every warp
+    // loads its half of the columns, the warps holding rows 0..63 add them.
     if (ok && !first)
     {
-        // tensor-memory loads are warp-collective: every warp loads, the warps
-        // holding rows 0..63 (output units) add them
         const bool mine = r < 64;
         uint32_t v[32];
-        for (int half = 0; half < 2; half++)
-        {
-            tc_ld32(lanes + TM_DW3 + 32 * half, v);
-            tc_wait_ld();
-            if (mine) for (int j = 0; j < 32; j++) atomicAdd(&grad[ML_W3 + r * ML_H + 32 * half + j], __uint_as_float(v[j]));
-            tc_ld32(lanes + TM_DW2 + 32 * half, v);
-            tc_wait_ld();
-            if (mine) for (int j = 0; j < 32; j++) atomicAdd(&grad[ML_W2 + r * ML_H + 32 * half + j], __uint_as_float(v[j]));
-            tc_ld32(lanes + TM_DW4 + 32 * half, v);
-            tc_wait_ld();
-            if (r < ML_OUT) for (int j = 0; j < 32; j++) atomicAdd(&grad[ML_W4 + r * ML_H + 32 * half + j], __uint_as_float(v[j]));
-        }
-        uint32_t v16[16];
-        tc_ld16(lanes + TM_DW1, v16);
+        tc_ld32(lanes + TM_DW3 + c0, v);
         tc_wait_ld();
-        if (mine) for (int j = 0; j < ML_IN; j++) atomicAdd(&grad[ML_W1 + r * ML_IN + j], __uint_as_float(v16[j]));
-    }
-    if (ok && !first)
-    {
-        atomicAdd(&grad[ML_B1 + 2 * lane], db1.x); atomicAdd(&grad[ML_B1 + 2 * lane + 1], db1.y);
-        atomicAdd(&grad[ML_B2 + 2 * lane], db2.x); atomicAdd(&grad[ML_B2 + 2 * lane + 1], db2.y);
-        atomicAdd(&grad[ML_B3 + 2 * lane], db3.x); atomicAdd(&grad[ML_B3 + 2 * lane + 1], db3.y);
-        if (lane == 0)
-            for (int k = 0; k < ML_OUT; k++) atomicAdd(&grad[ML_B4 + k], db4[k]);
-        for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-        if (lane == 0) atomicAdd(loss, lsum);
+        if (mine) for (int j = 0; j < 32; j++) atomicAdd(&grad[ML_W3 + r * ML_H + c0 + j], __uint_as_float(v[j]));
+        tc_ld32(lanes + TM_DW2 + c0, v);
+        tc_wait_ld();
+        if (mine) for (int j = 0; j < 32; j++) atomicAdd(&grad[ML_W2 + r * ML_H + c0 + j], __uint_as_float(v[j]));
+        tc_ld32(lanes + TM_DW4 + c0, v);
+        tc_wait_ld();
+        if (r < ML_OUT) for (int j = 0; j < 32; j++) atomicAdd(&grad[ML_W4 + r * ML_H + c0 + j], __uint_as_float(v[j]));
+        if (half == 0)
+        {
+            uint32_t v16[16];
+            tc_ld16(lanes + TM_DW1, v16);
+            tc_wait_ld();
+            if (mine) for (int j = 0; j < ML_IN; j++) atomicAdd(&grad[ML_W1 + r * ML_IN + j], __uint_as_float(v16[j]));
+        }
+        atomicAdd(&grad[ML_B1 + c0 + lane], db[0]);
+        atomicAdd(&grad[ML_B2 + c0 + lane], db[1]);
+        atomicAdd(&grad[ML_B3 + c0 + lane], db[2]);
+        if (half == 0)
+        {
+            if (lane == 0)
+                for (int k = 0; k < ML_OUT; k++) atomicAdd(&grad[ML_B4 + k], db4[k]);
+            for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+            if (lane == 0) atomicAdd(loss, lsum);
+        }
     }
     tmem_free(t.tmem, 512);
 }

@@ -2197,7 +2197,7 @@ static int mlp_infer_grid(int rows) { return std::max(1, std::min((rows + ML_ROW
 
 void launch_mlp_warm(cudaStream_t s, const DevCloth& c, const Buffers& b, const float* prm, const float* norm)
 {
-    k_mlp_warm<<<mlp_infer_grid(c.N), 128, 0, s>>>(c, b, MlpArgs{prm, norm});
+    k_mlp_warm<<<mlp_infer_grid(c.N), ML_THREADS, 0, s>>>(c, b, MlpArgs{prm, norm});
 }
 
 void launch_mlp_features(cudaStream_t s, const DevCloth& c, const Buffers& b, float* feat)
@@ -2212,7 +2212,7 @@ void launch_mlp_targets(cudaStream_t s, const DevCloth& c, float* target)
 
 void launch_mlp_forward(cudaStream_t s, const float* X, int S, const float* prm, const float* norm, float* Y)
 {
-    k_mlp_forward<<<mlp_infer_grid(S), 128, 0, s>>>(X, S, MlpArgs{prm, norm}, Y, nullptr);
+    k_mlp_forward<<<mlp_infer_grid(S), ML_THREADS, 0, s>>>(X, S, MlpArgs{prm, norm}, Y, nullptr);
 }
 
 size_t mlp_grad_smem() { return sizeof(MlpTcTrainSmem); }
@@ -2231,7 +2231,7 @@ bool launch_mlp_grad(cudaStream_t s, const float* X, const float* T, int S, cons
     cudaMemsetAsync(loss, 0, sizeof(float), s);
     // training CTAs hold all 512 tensor-memory columns of their SM: one per SM
     const int grid = std::max(1, std::min((S + ML_ROWS - 1) / ML_ROWS, mlp_sm_count()));
-    k_mlp_grad<<<grid, 128, smem, s>>>(X, T, S, MlpArgs{prm, norm}, grad, loss, nullptr);
+    k_mlp_grad<<<grid, ML_THREADS, smem, s>>>(X, T, S, MlpArgs{prm, norm}, grad, loss, nullptr);
     return cudaGetLastError() == cudaSuccess;
 }
 

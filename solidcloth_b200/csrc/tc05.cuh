@@ -120,9 +120,9 @@ __device__ __forceinline__ void tmem_free(uint32_t base, uint32_t cols)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(base), "r"(cols) : "memory");
 }
 
-// this warp's 32 lanes (rows 32 w .. 32 w + 31 of an M = 128 accumulator): lane
-// field of the tensor-memory address
-__device__ __forceinline__ uint32_t tmem_lane_base(uint32_t base) { return base + ((uint32_t)((threadIdx.x >> 5) * 32) << 16); }
+// this warp's 32 lanes (rows 32 w .. 32 w + 31 of an M = 128 accumulator, w the
+// warp's number modulo 4): lane field of the tensor-memory address
+__device__ __forceinline__ uint32_t tmem_lane_base(uint32_t base) { return base + ((uint32_t)(((threadIdx.x >> 5) & 3) * 32) << 16); }
 
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32])
 {
