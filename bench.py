@@ -497,8 +497,8 @@ def run_ours(args):
     kernel_names = {"gs_solve": solver,
                     "ccd_broad_ee": "k_ccd_boxes + k_ccd_join (edge-edge swept boxes, their join in blocks of 32, and "
                                     "the first part of the narrow phase)",
-                    "colliders": "k_vertex_colliders (+ k_tri_colliders, k_edge_colliders when continuous collision is "
-                                 "off: with it on they run on another branch, untimed)"}
+                    "colliders": "k_vertex_colliders, k_tri_colliders, k_edge_colliders, k_mesh_query and the contact "
+                                 "lists (beside the edge-edge broad phase when continuous collision is on)"}
     per = {}
     for k in algo:
         tot, cnt = sections.get(k, (0.0, 0))

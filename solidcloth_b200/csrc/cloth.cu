@@ -315,12 +315,35 @@ bool MeshC::upload(int devId)
         verts.insert(verts.end(), t.verts.begin(), t.verts.end());
         edges.insert(edges.end(), t.edges.begin(), t.edges.end());
     }
+    std::vector<float4> rec(MESH_NODE_WORDS * (size_t)M);
+    for (int k = 0; k < M; k++)
+    {
+        const Box none = Box::empty();
+        const Box& l = tree[k].left >= 0 ? tree[tree[k].left].box : none;
+        const Box& r = tree[k].right >= 0 ? tree[tree[k].right].box : none;
+        float4* q = &rec[MESH_NODE_WORDS * (size_t)k];
+        q[0] = f4(l.lo, bits_f((uint32_t)tree[k].left)); q[1] = f4(l.hi, 0.f);
+        q[2] = f4(r.lo, bits_f((uint32_t)tree[k].right)); q[3] = f4(r.hi, 0.f);
+        q[4] = make_float4(bits_f((uint32_t)pr[k].x), bits_f((uint32_t)pr[k].y), bits_f((uint32_t)pr[k].z), bits_f((uint32_t)pr[k].w));
+        q[5] = make_float4(bits_f((uint32_t)er[k].x), bits_f((uint32_t)er[k].y), 0.f, 0.f);
+    }
+    // the leaves' primitives with their geometry, in list order
+    std::vector<float4> triV, vertV, edgeV;
+    for (uint32_t t : tris)
+        for (int k = 0; k < 3; k++) triV.push_back(f4(mesh.verts[mesh.idx[3 * t + k]], bits_f(t)));
+    for (uint32_t i : verts) vertV.push_back(f4(mesh.verts[i], bits_f(i)));
+    for (uint32_t e : edges)
+    {
+        edgeV.push_back(f4(mesh.verts[mesh.edges[e].i1], bits_f(e)));
+        edgeV.push_back(f4(mesh.verts[mesh.edges[e].i2], bits_f(e)));
+    }
     // one allocation, 256-byte aligned sub-buffers
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
     size_t oV = take(V * 16), oN = take(V * 16), oEN = take(E * 16), oT = take(T * 12), oE = take(E * 16);
     size_t oLo = take(M * 16), oHi = take(M * 16), oCh = take(M * 8), oPr = take(M * 16), oEr = take(M * 8);
     size_t oTr = take(tris.size() * 4 + 4), oVe = take(verts.size() * 4 + 4), oEd = take(edges.size() * 4 + 4);
+    size_t oTV = take(triV.size() * 16 + 16), oVV = take(vertV.size() * 16 + 16), oEV = take(edgeV.size() * 16 + 16), oRec = take(rec.size() * 16 + 16);
     SC_CUDA(cudaMalloc(&dmem, off));
     char* d = (char*)dmem;
     SC_CUDA(cudaMemcpy(d + oV, v.data(), V * 16, cudaMemcpyHostToDevice));
@@ -336,6 +359,12 @@ bool MeshC::upload(int devId)
     if (!tris.empty()) SC_CUDA(cudaMemcpy(d + oTr, tris.data(), tris.size() * 4, cudaMemcpyHostToDevice));
     if (!verts.empty()) SC_CUDA(cudaMemcpy(d + oVe, verts.data(), verts.size() * 4, cudaMemcpyHostToDevice));
     if (!edges.empty()) SC_CUDA(cudaMemcpy(d + oEd, edges.data(), edges.size() * 4, cudaMemcpyHostToDevice));
+    if (!triV.empty()) SC_CUDA(cudaMemcpy(d + oTV, triV.data(), triV.size() * 16, cudaMemcpyHostToDevice));
+    if (!vertV.empty()) SC_CUDA(cudaMemcpy(d + oVV, vertV.data(), vertV.size() * 16, cudaMemcpyHostToDevice));
+    if (!edgeV.empty()) SC_CUDA(cudaMemcpy(d + oEV, edgeV.data(), edgeV.size() * 16, cudaMemcpyHostToDevice));
+    SC_CUDA(cudaMemcpy(d + oRec, rec.data(), rec.size() * 16, cudaMemcpyHostToDevice));
+    dev.tree.rec = (const float4*)(d + oRec);
+    dev.tree.triV = (const float4*)(d + oTV); dev.tree.vertV = (const float4*)(d + oVV); dev.tree.edgeV = (const float4*)(d + oEV);
     dev.V = V; dev.T = T; dev.E = E;
     dev.v = (const float4*)(d + oV); dev.n = (const float4*)(d + oN); dev.en = (const float4*)(d + oEN);
     dev.tri = (const uint32_t*)(d + oT); dev.edge = (const int4*)(d + oE);
@@ -1847,6 +1876,17 @@ bool ClothModel::ensure_buffers(const CollisionWorld& world, cudaStream_t s)
     if (!meshes.empty()) SC_CUDA(cudaMemcpy(dmeshes, meshes.data(), sizeof(DevMesh) * meshes.size(), cudaMemcpyHostToDevice));
     buf.meshes = dmeshes;
     buf.numMeshes = (int)meshes.size();
+    // queries that reach a mesh collider: one entry per vertex, triangle and edge at most
+    size_t reach[3] = {0, 0, 0};
+    for (const VColl& g : vcollHost)
+    {
+        if (g.type != CT_MESH) continue;
+        reach[0] += (size_t)g.vCount;
+        reach[1] += (prm.flags & CF_TRIANGLES) ? T : 0;
+        reach[2] += (prm.flags & CF_EDGES) ? E : 0;
+    }
+    for (int k = 0; k < 3; k++) buf.meshQueryBase[k] = (int)(k == 0 ? 0 : k == 1 ? reach[0] : reach[0] + reach[1]);
+    buf.meshQuery = (int4*)dalloc(sizeof(int4) * std::max<size_t>(1, reach[0] + reach[1] + reach[2]), true);
     // triangle / edge contacts
     const int nTc = (prm.flags & CF_TRIANGLES) ? nTE : 0, nEc = (prm.flags & CF_EDGES) ? nTE : 0;
     buf.tcCap = std::max(1, nTc * T);
@@ -1858,6 +1898,7 @@ bool ClothModel::ensure_buffers(const CollisionWorld& world, cudaStream_t s)
     buf.ecFlag = (int*)dalloc(sizeof(int) * (size_t)buf.ecCap, true);
     buf.ecList = (EC*)dalloc(sizeof(EC) * (size_t)buf.ecCap, true);
     int* counts = (int*)dalloc(sizeof(int) * 16, true);
+    buf.meshQueryCount = counts + 11;
     buf.tcCount = counts; buf.ecCount = counts + 1; buf.stCount = counts + 2; buf.seCount = counts + 3;
     buf.ccdVtPairCount = counts + 4; buf.ccdEePairCount = counts + 5; buf.scanTot = counts + 8;
     // self contacts
@@ -2326,25 +2367,18 @@ void ClothPatch::record_substep(float h)
     launch_predict(s, c, P, tiles, recordingSubstep == 0);
     const bool self = (m.prm.flags & CF_SELF) != 0, ccd = m.prm.ccd;
     // ClothModel::DetectCollisions (Physics/ClothCollision.cpp:17-48)
+    // the collider contacts only read the predicted positions: with continuous collision
+    // they run on the side stream ahead of its half, which the main stream joins before
+    // anything reads them
+    const cudaStream_t cs = ccd ? side : s;
     if (ccd)
     {
-        // the vertex contacts only read the predicted positions: they run on the
-        // side stream ahead of its continuous-collision branch, which the main
-        // stream joins before anything reads them
         cudaEventRecord(evFork, s);
         cudaStreamWaitEvent(side, evFork, 0);
-        timing_mark(SEC_COLLIDERS, false, side);
-        launch_vertex_colliders(side, c, P, b, m.vcollHost.data());
-        timing_mark(SEC_COLLIDERS, true, side);
-        launch_tri_edge_colliders(s, c, P, b, m.vcollHost.data(), (int)m.vcollHost.size(), m.prm.flags);
     }
-    else
-    {
-        timing_mark(SEC_COLLIDERS, false, s);
-        launch_vertex_colliders(s, c, P, b, m.vcollHost.data());
-        launch_tri_edge_colliders(s, c, P, b, m.vcollHost.data(), (int)m.vcollHost.size(), m.prm.flags);
-        timing_mark(SEC_COLLIDERS, true, s);
-    }
+    timing_mark(SEC_COLLIDERS, false, cs);
+    launch_colliders(cs, c, P, b, m.vcollHost.data(), (int)m.vcollHost.size(), m.prm.flags);
+    timing_mark(SEC_COLLIDERS, true, cs);
     if (self)
     {
         launch_bvh_refit(s, m.triBvh, c, 0, 0.f);

@@ -77,6 +77,9 @@ struct Buffers
     int* scanOff2;             // second per-item offsets (side stream)
     const DevMesh* meshes;     // device array
     int numMeshes;
+    // this substep's queries that reach a mesh collider, by kind (vertices, triangles,
+    // edges): item, collider (index in vcoll), contact slot of the collider
+    int4* meshQuery; int meshQueryBase[3]; int* meshQueryCount;
 };
 
 struct TileView;
@@ -91,9 +94,9 @@ void launch_links(cudaStream_t s, const DevCloth& c, const SolverParams& P, int 
 void launch_reset_link_error(cudaStream_t s, const DevCloth& c);
 void launch_bends(cudaStream_t s, const DevCloth& c, const SolverParams& P, int first, int count, int resetErr);
 void launch_normals(cudaStream_t s, const DevCloth& c, bool prevMesh, const float4* verts);
-void launch_vertex_colliders(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, const VColl* hostColl);
-void launch_tri_edge_colliders(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b,
-                               const VColl* hostColl, int numColl, int flags);
+// vertex contacts of every collider, triangle and edge contacts with their dense lists
+void launch_colliders(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, const VColl* hostColl,
+                      int numColl, int flags);
 void launch_solve_vertex_contacts(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b);
 void launch_solve_multi_contacts(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, int iter);
 void launch_colour_contacts(cudaStream_t s, const DevCloth& c, const Buffers& b);

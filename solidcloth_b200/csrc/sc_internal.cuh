@@ -139,7 +139,16 @@ struct DevMeshTree
     const uint32_t* tris;
     const uint32_t* verts;
     const uint32_t* edges;
+    // the same lists with the geometry in place: index (as bits) in the first w
+    const float4* triV;      // three per triangle
+    const float4* vertV;     // one per vertex
+    const float4* edgeV;     // two per edge
+    // six words per node: per child its box and index, (left lo, left) (left hi, -)
+    // (right lo, right) (right hi, -), then (first triangle, triangles, first vertex,
+    // vertices) (first edge, edges); primitives are in nodes without children only
+    const float4* rec;
 };
+constexpr int MESH_NODE_WORDS = 6;
 
 struct DevMesh
 {

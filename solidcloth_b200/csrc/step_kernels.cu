@@ -373,63 +373,6 @@ __device__ PointHit mesh_point_query(const DevMesh& m, V3 p, int* status, float 
     return r;
 }
 
-struct VtxHit { float dist; int vertex; V3 cpMesh, cpTri, bary, normal; int region; };
-
-__device__ VtxHit mesh_triangle_query(const DevMesh& m, V3 a, V3 b, V3 cc, int* status, float bound)
-{
-    VtxHit r; r.dist = -FLT_MAX; r.vertex = -1; r.region = 0;
-    r.cpMesh = r.cpTri = r.bary = r.normal = mk(0.f, 0.f, 0.f);
-    float minDist = bound;
-    Box tb = Box::empty(); tb.add(a); tb.add(b); tb.add(cc);
-    const float slack = skip_slack(a);
-    int stNode[MESH_STACK]; float stDist[MESH_STACK];
-    int sp = 0, node = 0;
-    while (true)
-    {
-        if (node >= 0)
-        {
-            int4 pr = m.tree.primRange[node];
-            for (int k = 0; k < pr.w; k++)
-            {
-                uint32_t v = m.tree.verts[pr.z + k];
-                V3 pv = ld3(m.v, v);
-                if (cannot_improve(tb.dist(pv), minDist, slack)) continue;
-                V3 bary, cp;
-                int region = closest_point_triangle(pv, a, b, cc, cp, bary);
-                V3 delta = cp - pv;
-                float dist = len(delta);
-                if (dist == 0) continue;
-                if (dist < minDist)
-                {
-                    minDist = dist;
-                    r.vertex = (int)v; r.cpMesh = pv; r.cpTri = cp; r.bary = bary;
-                    r.normal = (1.f / dist) * delta; r.dist = dist; r.region = region;
-                }
-            }
-            int2 ch = m.tree.children[node];
-            if (ch.x >= 0 || ch.y >= 0)
-            {
-                Box bl, br;
-                float dl = FLT_MAX, dr = FLT_MAX;
-                if (ch.x >= 0) { bl.lo = ld3(m.tree.lo, ch.x); bl.hi = ld3(m.tree.hi, ch.x); dl = bl.dist(tb); }
-                if (ch.y >= 0) { br.lo = ld3(m.tree.lo, ch.y); br.hi = ld3(m.tree.hi, ch.y); dr = br.dist(tb); }
-                int nearN = ch.x, farN = ch.y; float nearD = dl, farD = dr;
-                if (!(dl < dr)) { nearN = ch.y; farN = ch.x; nearD = dr; farD = dl; }
-                if (sp < MESH_STACK) { stNode[sp] = farN; stDist[sp] = farD; sp++; }
-                else atomicOr(status, ST_MESH_STACK_OVERFLOW);
-                node = (nearD < minDist) ? nearN : -1;
-                continue;
-            }
-        }
-        node = -1;
-        while (sp > 0 && node < 0) { sp--; if (stDist[sp] < minDist) node = stNode[sp]; }
-        if (node < 0) break;
-    }
-    return r;
-}
-
-struct SegHit { float dist; int edge; V3 cpMesh, cpSegm, normal; float cs0, cs1, cm0, cm1; int region; };
-
 // ComputeEdgeNormal (Geometry/ClosestPointOnMesh.cpp:483-497)
 __device__ __forceinline__ V3 mesh_edge_normal(const DevMesh& m, int e, float param)
 {
@@ -440,63 +383,189 @@ __device__ __forceinline__ V3 mesh_edge_normal(const DevMesh& m, int e, float pa
     return n;
 }
 
-__device__ SegHit mesh_segment_query(const DevMesh& m, V3 p, V3 q, int* status, float bound)
+// ---- mesh queries
+// A cloth's queries against a collider mesh: every thread rules its item out against
+// the root's children (k_vertex_colliders, k_tri_colliders, k_edge_colliders); the
+// rest are listed, neighbours together and kinds apart, and k_mesh_query searches for
+// them: the recursion's depth-first order with an explicit stack, first down to a
+// leaf, then through its primitives, so that a warp's lanes do the same thing.
+//
+// What bounds it: instruction issue, most of it in the leaves' closest-point
+// computations. One thread per item of the whole cloth left warps waiting for the few
+// lanes that reached the mesh, and a primitive took three dependent loads (index,
+// vertices, positions; the leaves now carry the positions): on a 256 x 256 cloth on a
+// 20,480-triangle sphere, edges 335 us, vertices 292, triangles 141 a substep;
+// 267 us together (the listed queries of a warp differ in their leaves: 8 of 32 lanes
+// active). One warp per listed query, its lanes on a leaf's primitives, took 327 us:
+// 2,700 instructions a query, most of them the same in every lane.
+struct MeshHit
 {
-    SegHit r; r.dist = -FLT_MAX; r.edge = -1; r.region = -1;
-    r.cpMesh = r.cpSegm = r.normal = mk(0.f, 0.f, 0.f);
-    r.cs0 = r.cs1 = r.cm0 = r.cm1 = 0.f;
+    float dist, w0, w1, w2;
+    int feature;                 // -1: none
+    V3 cp, normal;
+};
+
+// the root's children in reach of the bound (or primitives in the root itself)
+template <int KIND, class Q>
+__device__ __forceinline__ bool mesh_in_reach(const DevMesh& m, const Q& q, float bound)
+{
+    const int4 pr = m.tree.primRange[0];
+    if ((KIND == 0 ? pr.y : KIND == 1 ? pr.w : m.tree.edgeRange[0].y) > 0) return true;
+    const int2 ch = m.tree.children[0];
+    for (int c : {ch.x, ch.y})
+    {
+        if (c < 0) continue;
+        Box b;
+        b.lo = ld3(m.tree.lo, c); b.hi = ld3(m.tree.hi, c);
+        if (b.dist(q) < bound) return true;
+    }
+    return false;
+}
+
+// a point (KIND 0: x), a triangle (1: x, y, z against the mesh's vertices) or a
+// segment (2: x, y). Primitives whose box is farther than the best distance plus the
+// slack are skipped (cannot_improve, on squares: the slack is far above either rounding).
+template <int KIND>
+__device__ __forceinline__ MeshHit mesh_query(const DevMesh& m, V3 x, V3 y, V3 z, float bound, int* status)
+{
+    MeshHit r;
+    r.feature = -1; r.dist = r.w0 = r.w1 = r.w2 = 0.f;
+    r.cp = r.normal = mk(0.f, 0.f, 0.f);
+    Box qb = Box::empty();
+    qb.add(x);
+    if (KIND >= 1) qb.add(y);
+    if (KIND == 1) qb.add(z);
+    const V3 ext = qb.hi - qb.lo;
+    const float slack = skip_slack(x);
     float minDist = bound;
-    Box eb = Box::empty(); eb.add(p); eb.add(q);
-    const float slack = skip_slack(p);
+    auto skip = [&](const Box& b, V3 v) {
+        const float dx = mx(0.f, mx(b.lo.x - v.x, v.x - b.hi.x)), dy = mx(0.f, mx(b.lo.y - v.y, v.y - b.hi.y)),
+                    dz = mx(0.f, mx(b.lo.z - v.z, v.z - b.hi.z));
+        return dx * dx + dy * dy + dz * dz > (minDist + slack) * (minDist + slack);
+    };
+    auto reach = [&](float4 lo, float4 hi) {
+        const Box b = {mk(lo), mk(hi)};
+        if (__float_as_int(lo.w) < 0) return FLT_MAX;
+        if constexpr (KIND == 0) return b.dist(x);
+        else return b.dist(qb);
+    };
     int stNode[MESH_STACK]; float stDist[MESH_STACK];
     int sp = 0, node = 0;
-    while (true)
-    {
-        if (node >= 0)
+    auto pop = [&] {
+        node = -1;
+        while (sp > 0 && node < 0)
         {
-            int2 er = m.tree.edgeRange[node];
-            for (int k = 0; k < er.y; k++)
+            sp--;
+            if (stDist[sp] < minDist) node = stNode[sp];
+        }
+    };
+    while (node >= 0)
+    {
+        const float4* rec = m.tree.rec + MESH_NODE_WORDS * (size_t)node;
+        // down to a leaf
+        while (true)
+        {
+            const float4 l0 = __ldg(rec), l1 = __ldg(rec + 1), r0 = __ldg(rec + 2), r1 = __ldg(rec + 3);
+            const int left = __float_as_int(l0.w), right = __float_as_int(r0.w);
+            if (left < 0 && right < 0) break;
+            const float dl = reach(l0, l1), dr = reach(r0, r1);
+            int nearN = left, farN = right; float nearD = dl, farD = dr;
+            if (!(dl < dr)) { nearN = right; farN = left; nearD = dr; farD = dl; }
+            // a far child that is out of reach now will be when its turn comes
+            if (farD < minDist)
             {
-                uint32_t e = m.tree.edges[er.x + k];
-                int4 ed = m.edge[e];
-                V3 a = ld3(m.v, ed.x), b = ld3(m.v, ed.y);
-                Box pb = Box::empty(); pb.add(a); pb.add(b);
-                if (cannot_improve(pb.dist(eb), minDist, slack)) continue;
-                float ps, pm;
-                V3 cs, cm;
-                int region = closest_segm_segm(p, q, a, b, ps, pm, cs, cm);
-                V3 delta = cm - cs;
-                float dist = len(delta);
-                if (dist == 0) continue;
-                if (dist < minDist)
-                {
-                    minDist = dist;
-                    r.dist = dist; r.edge = (int)e; r.cpMesh = cm; r.cpSegm = cs;
-                    r.cs0 = 1.0f - ps; r.cs1 = ps; r.cm0 = 1.0f - pm; r.cm1 = pm;
-                    r.normal = mesh_edge_normal(m, (int)e, pm);
-                    r.region = region;
-                }
-            }
-            int2 ch = m.tree.children[node];
-            if (ch.x >= 0 || ch.y >= 0)
-            {
-                Box bl, br;
-                float dl = FLT_MAX, dr = FLT_MAX;
-                if (ch.x >= 0) { bl.lo = ld3(m.tree.lo, ch.x); bl.hi = ld3(m.tree.hi, ch.x); dl = bl.dist(eb); }
-                if (ch.y >= 0) { br.lo = ld3(m.tree.lo, ch.y); br.hi = ld3(m.tree.hi, ch.y); dr = br.dist(eb); }
-                int nearN = ch.x, farN = ch.y; float nearD = dl, farD = dr;
-                if (!(dl < dr)) { nearN = ch.y; farN = ch.x; nearD = dr; farD = dl; }
                 if (sp < MESH_STACK) { stNode[sp] = farN; stDist[sp] = farD; sp++; }
                 else atomicOr(status, ST_MESH_STACK_OVERFLOW);
-                node = (nearD < minDist) ? nearN : -1;
-                continue;
+            }
+            if (nearD < minDist) node = nearN;
+            else pop();
+            if (node < 0) break;
+            rec = m.tree.rec + MESH_NODE_WORDS * (size_t)node;
+        }
+        if (node < 0) break;
+        // first mark the primitives that could improve the result, then compute those in
+        // order: the lanes of a warp are in the long computation together
+        const int2 range = __ldg(reinterpret_cast<const int2*>(rec + 4) + KIND);
+        auto far = [&](int k) {
+            if constexpr (KIND == 0)
+                return skip(prim_box(mk(__ldg(&m.tree.triV[3 * k])), mk(__ldg(&m.tree.triV[3 * k + 1])), mk(__ldg(&m.tree.triV[3 * k + 2]))), x);
+            else if constexpr (KIND == 1)
+                return skip(qb, mk(__ldg(&m.tree.vertV[k])));
+            else
+            {
+                // the segment's box against the query's, as the query's corner against the box of both extents
+                const V3 a = mk(__ldg(&m.tree.edgeV[2 * k])), b = mk(__ldg(&m.tree.edgeV[2 * k + 1]));
+                const Box pb = {vmin(a, b) - ext, vmax(a, b)};
+                return skip(pb, qb.lo);
+            }
+        };
+        for (int k0 = range.x; k0 < range.x + range.y; k0 += 32)
+        {
+            unsigned near = 0u;
+            const int cnt = min(32, range.x + range.y - k0);
+            for (int j = 0; j < cnt; j++) near |= far(k0 + j) ? 0u : 1u << j;
+            while (near)
+            {
+                const int k = k0 + __ffs(near) - 1;
+                near &= near - 1;
+                if (far(k)) continue;                // the best distance has come down since
+                if constexpr (KIND == 0)
+                {
+                    const float4 a4 = __ldg(&m.tree.triV[3 * k]);
+                    const V3 a = mk(a4), b = mk(__ldg(&m.tree.triV[3 * k + 1])), c = mk(__ldg(&m.tree.triV[3 * k + 2]));
+                    V3 coords, cp;
+                    closest_point_triangle(x, a, b, c, cp, coords);
+                    const V3 delta = x - cp;
+                    const float dist = len(delta);
+                    if (dist == 0 || !(dist < minDist)) continue;
+                    minDist = dist;
+                    r.dist = dist; r.feature = __float_as_int(a4.w); r.cp = cp; r.normal = (1.f / dist) * delta;
+                }
+                else if constexpr (KIND == 1)
+                {
+                    const float4 a4 = __ldg(&m.tree.vertV[k]);
+                    const V3 pv = mk(a4);
+                    V3 coords, ct;
+                    closest_point_triangle(pv, x, y, z, ct, coords);
+                    const V3 delta = ct - pv;
+                    const float dist = len(delta);
+                    if (dist == 0 || !(dist < minDist)) continue;
+                    minDist = dist;
+                    r.dist = dist; r.feature = __float_as_int(a4.w); r.cp = pv; r.normal = (1.f / dist) * delta;
+                    r.w0 = coords.x; r.w1 = coords.y; r.w2 = coords.z;
+                }
+                else
+                {
+                    const float4 a4 = __ldg(&m.tree.edgeV[2 * k]);
+                    const V3 a = mk(a4), b = mk(__ldg(&m.tree.edgeV[2 * k + 1]));
+                    float ps, pm;
+                    V3 cs, cp;
+                    closest_segm_segm(x, y, a, b, ps, pm, cs, cp);
+                    const V3 delta = cp - cs;
+                    const float dist = len(delta);
+                    if (dist == 0 || !(dist < minDist)) continue;
+                    minDist = dist;
+                    r.dist = dist; r.feature = __float_as_int(a4.w); r.cp = cp;
+                    r.w0 = 1.0f - ps; r.w1 = ps; r.w2 = pm;
+                }
             }
         }
-        node = -1;
-        while (sp > 0 && node < 0) { sp--; if (stDist[sp] < minDist) node = stNode[sp]; }
-        if (node < 0) break;
+        pop();
     }
+    if (KIND == 2 && r.feature >= 0) r.normal = mesh_edge_normal(m, r.feature, r.w2);
     return r;
+}
+
+// append an item to the mesh query list of its kind (any subset of a warp's lanes: one
+// reservation for all of them, so neighbours stay together)
+__device__ __forceinline__ void list_mesh_query(const Buffers& b, int kind, int item, int coll, int slot)
+{
+    const unsigned m = __activemask();
+    const int lane = threadIdx.x & 31;
+    int at = 0;
+    if (lane == __ffs(m) - 1) at = atomicAdd(&b.meshQueryCount[kind], __popc(m));
+    at = __shfl_sync(m, at, __ffs(m) - 1) + __popc(m & ((1u << lane) - 1u));
+    b.meshQuery[b.meshQueryBase[kind] + at] = make_int4(item, coll, slot, 0);
 }
 
 // ------------------------------------------------- vertex contact detection
@@ -548,11 +617,8 @@ __global__ void k_vertex_colliders(DevCloth c, SolverParams P, Buffers b)
         }
         else if (g.type == 4)
         {
-            if (P.flags & CF_VERTICES)
-            {
-                PointHit h = mesh_point_query(b.meshes[g.mesh], prev, c.status, radTolMesh);
-                if (h.dist < radTolMesh && h.dist >= 0) add(h.cp, h.normal, h.tri, g.mesh);
-            }
+            // k_mesh_query writes its contact
+            if ((P.flags & CF_VERTICES) && mesh_in_reach<0>(b.meshes[g.mesh], prev, radTolMesh)) list_mesh_query(b, 0, i, ci, 0);
         }
         b.vcCount[(size_t)g.countBase + (i - g.vBegin)] = (uint8_t)n;
     }
@@ -598,7 +664,7 @@ __device__ float sdf_query_triangle(const VColl& g, V3 a, V3 bb, V3 cc, V3& cpOu
 // (SDFCollisions edge + triangle parts, Physics/ClothCollision.cpp:472-579;
 // MeshCollisions triangle + edge parts, :137-196). One thread per cloth
 // triangle or edge per collider; results go to per-item slots.
-__global__ void k_tri_colliders(DevCloth c, SolverParams P, Buffers b, VColl g, int slotColl)
+__global__ void k_tri_colliders(DevCloth c, SolverParams P, Buffers b, VColl g, int coll, int slotColl)
 {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= c.T) return;
@@ -616,15 +682,9 @@ __global__ void k_tri_colliders(DevCloth c, SolverParams P, Buffers b, VColl g, 
     if (g.type == 4)
     {
         // MeshCollisions: per-triangle threshold with 1.2 x travel (ClothCollision.cpp:137-160)
-        float rt = P.thickness + mx(P.tolerance, tvm * 1.2f);
-        VtxHit h = mesh_triangle_query(b.meshes[g.mesh], a, bb, cc, c.status, rt);
-        if (h.dist < rt && h.dist >= 0)
-        {
-            rec.point = f4(h.cpMesh, 0.f); rec.normal = f4(h.normal, 0.f);
-            rec.w = make_float4(h.bary.x, h.bary.y, h.bary.z, 0.f);
-            rec.feature = h.vertex; rec.mesh = g.mesh;
-            b.tcSlot[slot] = rec; b.tcFlag[slot] = 1;
-        }
+        const float rt = P.thickness + mx(P.tolerance, tvm * 1.2f);
+        Box tb = Box::empty(); tb.add(a); tb.add(bb); tb.add(cc);
+        if (mesh_in_reach<1>(b.meshes[g.mesh], tb, rt)) list_mesh_query(b, 1, t, coll, slotColl);
         return;
     }
     const bool handleBorder = ((P.flags & CF_VERTICES) == 0) || ((P.flags & CF_EDGES) == 0);
@@ -653,7 +713,7 @@ __global__ void k_tri_colliders(DevCloth c, SolverParams P, Buffers b, VColl g, 
     }
 }
 
-__global__ void k_edge_colliders(DevCloth c, SolverParams P, Buffers b, VColl g, int slotColl)
+__global__ void k_edge_colliders(DevCloth c, SolverParams P, Buffers b, VColl g, int coll, int slotColl)
 {
     int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= c.E) return;
@@ -667,14 +727,8 @@ __global__ void k_edge_colliders(DevCloth c, SolverParams P, Buffers b, VColl g,
     if (g.type == 4)
     {
         const float radTol = P.thickness + mx(P.tolerance, c.scal[0] * 1.5f);
-        SegHit h = mesh_segment_query(b.meshes[g.mesh], p, q, c.status, radTol);
-        if (h.dist < radTol && h.dist >= 0)
-        {
-            rec.point = f4(h.cpMesh, 0.f); rec.normal = f4(h.normal, 0.f);
-            rec.w = make_float4(h.cs0, h.cs1, 0.f, 0.f);
-            rec.feature = h.edge; rec.mesh = g.mesh;
-            b.ecSlot[slot] = rec; b.ecFlag[slot] = 1;
-        }
+        Box eb = Box::empty(); eb.add(p); eb.add(q);
+        if (mesh_in_reach<2>(b.meshes[g.mesh], eb, radTol)) list_mesh_query(b, 2, e, coll, slotColl);
         return;
     }
     const bool handleBorder = (P.flags & CF_VERTICES) == 0;
@@ -704,6 +758,74 @@ __global__ void k_edge_colliders(DevCloth c, SolverParams P, Buffers b, VColl g,
         rec.w = make_float4(c0, c1, 0.f, 0.f);
         rec.feature = -1; rec.mesh = -1;
         b.ecSlot[slot] = rec; b.ecFlag[slot] = 1;
+    }
+}
+
+constexpr int MESH_QUERY_THREADS = 128;
+
+__global__ void __launch_bounds__(MESH_QUERY_THREADS) k_mesh_query(DevCloth c, SolverParams P, Buffers b)
+{
+    const int n0 = b.meshQueryCount[0], n1 = b.meshQueryCount[1], n2 = b.meshQueryCount[2];
+    const int w0 = (n0 + 31) / 32, w1 = (n1 + 31) / 32, w2 = (n2 + 31) / 32;
+    const int warps = gridDim.x * (MESH_QUERY_THREADS / 32), lane = threadIdx.x & 31;
+    const float travel = P.thickness + mx(P.tolerance, c.scal[0] * 1.5f);
+    for (int w = blockIdx.x * (MESH_QUERY_THREADS / 32) + (threadIdx.x >> 5); w < w0 + w1 + w2; w += warps)
+    {
+        // a warp's entries are of one kind
+        const int kind = w < w0 ? 0 : w < w0 + w1 ? 1 : 2;
+        const int k = 32 * (w - (kind > 0 ? w0 : 0) - (kind > 1 ? w1 : 0)) + lane;
+        if (k >= (kind == 0 ? n0 : kind == 1 ? n1 : n2)) continue;
+        const int4 e = b.meshQuery[b.meshQueryBase[kind] + k];      // item, collider, contact slot
+        const VColl& g = b.vcoll[e.y];
+        const DevMesh& m = b.meshes[g.mesh];
+        if (kind == 0)
+        {
+            // vertex part of MeshCollisions (Physics/ClothCollision.cpp:89-135)
+            const MeshHit h = mesh_query<0>(m, ld3(c.prev, e.x), mk(0, 0, 0), mk(0, 0, 0), travel, c.status);
+            if (h.feature >= 0 && h.dist < travel && h.dist >= 0)
+            {
+                VC v;
+                v.point = f4(h.cp, 0.f); v.normal = f4(h.normal, 0.f);
+                v.lam = make_float2(0.f, 0.f); v.feature = h.feature; v.mesh = g.mesh;
+                b.vc[g.slotBase + (size_t)(e.x - g.vBegin) * g.kmax] = v;
+                b.vcCount[(size_t)g.countBase + (e.x - g.vBegin)] = 1;
+            }
+        }
+        else if (kind == 1)
+        {
+            const uint32_t i1 = c.tri[3 * e.x], i2 = c.tri[3 * e.x + 1], i3 = c.tri[3 * e.x + 2];
+            const V3 x1 = ld3(c.prev, i1), x2 = ld3(c.prev, i2), x3 = ld3(c.prev, i3);
+            const float tvm = mx(len(x1 - ld3(c.pos, i1)), mx(len(x2 - ld3(c.pos, i2)), len(x3 - ld3(c.pos, i3))));
+            const float rt = P.thickness + mx(P.tolerance, tvm * 1.2f);
+            const MeshHit h = mesh_query<1>(m, x1, x2, x3, rt, c.status);
+            if (h.feature >= 0 && h.dist < rt && h.dist >= 0)
+            {
+                TC rec;
+                rec.idx = make_uint4(i1, i2, i3, (uint32_t)e.x | ((uint32_t)min(e.z, 255) << 24));   // .w: triangle, collider slot
+                rec.lam = make_float2(0.f, 0.f);
+                rec.point = f4(h.cp, 0.f); rec.normal = f4(h.normal, 0.f);
+                rec.w = make_float4(h.w0, h.w1, h.w2, 0.f);
+                rec.feature = h.feature; rec.mesh = g.mesh;
+                const size_t slot = (size_t)e.z * c.T + e.x;
+                b.tcSlot[slot] = rec; b.tcFlag[slot] = 1;
+            }
+        }
+        else
+        {
+            const int4 ed = c.edge[e.x];
+            const MeshHit h = mesh_query<2>(m, ld3(c.prev, ed.x), ld3(c.prev, ed.y), mk(0, 0, 0), travel, c.status);
+            if (h.feature >= 0 && h.dist < travel && h.dist >= 0)
+            {
+                EC rec;
+                rec.idx = make_uint4(ed.x, ed.y, (uint32_t)e.x, (uint32_t)e.z);   // .z: edge, .w: collider slot
+                rec.lam = make_float2(0.f, 0.f);
+                rec.point = f4(h.cp, 0.f); rec.normal = f4(h.normal, 0.f);
+                rec.w = make_float4(h.w0, h.w1, 0.f, 0.f);
+                rec.feature = h.feature; rec.mesh = g.mesh;
+                const size_t slot = (size_t)e.z * c.E + e.x;
+                b.ecSlot[slot] = rec; b.ecFlag[slot] = 1;
+            }
+        }
     }
 }
 
@@ -1975,14 +2097,11 @@ void launch_normals(cudaStream_t s, const DevCloth& c, bool prevMesh, const floa
     k_vertex_normals<<<blocks_for(c.N), 256, 0, s>>>(c.N, c.vTriStart, c.vTri, triN, c.triAngles, vn);
 }
 
-void launch_vertex_colliders(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, const VColl*)
+void launch_colliders(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, const VColl* hostColl,
+                      int numColl, int flags)
 {
+    if (b.numMeshes > 0) cudaMemsetAsync(b.meshQueryCount, 0, 3 * sizeof(int), s);
     if (b.numVColl > 0) k_vertex_colliders<<<blocks_for(c.N, 128), 128, 0, s>>>(c, P, b);
-}
-
-void launch_tri_edge_colliders(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b,
-                               const VColl* hostColl, int numColl, int flags)
-{
     // per-collider triangle / edge slots: collider slot index = order among
     // colliders that produce such contacts (world order)
     int ti = 0, ei = 0;
@@ -1990,9 +2109,10 @@ void launch_tri_edge_colliders(cudaStream_t s, const DevCloth& c, const SolverPa
     {
         const VColl& g = hostColl[k];
         if (g.type != 3 && g.type != 4 && g.type != 7) continue;
-        if (flags & CF_EDGES) { k_edge_colliders<<<blocks_for(c.E, 128), 128, 0, s>>>(c, P, b, g, ei); ei++; }
-        if (flags & CF_TRIANGLES) { k_tri_colliders<<<blocks_for(c.T, 128), 128, 0, s>>>(c, P, b, g, ti); ti++; }
+        if (flags & CF_EDGES) { k_edge_colliders<<<blocks_for(c.E, 128), 128, 0, s>>>(c, P, b, g, k, ei); ei++; }
+        if (flags & CF_TRIANGLES) { k_tri_colliders<<<blocks_for(c.T, 128), 128, 0, s>>>(c, P, b, g, k, ti); ti++; }
     }
+    if (b.numMeshes > 0) k_mesh_query<<<148 * 6, MESH_QUERY_THREADS, 0, s>>>(c, P, b);
     // compaction in (collider, item) order (without such contacts the counts stay zero,
     // as they were allocated)
     if (ti > 0)
