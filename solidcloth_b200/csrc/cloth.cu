@@ -2464,7 +2464,7 @@ bool ClothPatch::record_solve(cudaStream_t s, const SolverParams& P, const Solve
         plan.nLinkCol = (int)m.linkColourStart.size() - 1;
         for (size_t k = 0; k < m.linkColourStart.size(); k++) plan.linkStart[k] = m.linkColourStart[k];
     }
-    int shift = 0;
+    int vpc = 0;
     size_t smem = 0;
     if (ch.kind == SOLVE_TILE && m.tilePlan.valid)
     {
@@ -2474,18 +2474,18 @@ bool ClothPatch::record_solve(cudaStream_t s, const SolverParams& P, const Solve
             return false;
         if (!other) return true;
         plan.guard = GUARD_IF_SELF;
-        const int cs = ops.cluster_size(m.N, shift, smem);
-        plan.shift = shift;
+        const int cs = ops.cluster_size(m.N, vpc, smem);
+        plan.vpc = vpc;
         if (cs > 0) { ops.cluster(s, c, P, b, plan, cs, smem, 0); return true; }
         return ops.grid(s, c, P, b, plan, 0, 1);
     }
     if (ch.kind == SOLVE_BAND && m.band_active() &&
         ops.band(s, c, P, b, plan, m.bandPlan.view, m.bandPlan.clusterSize, m.band_smem(), ch.variant))
         return true;                                                 // includes the velocity update
-    const int cluster = (ch.kind == SOLVE_CLUSTER && planFits) ? ops.cluster_size(m.N, shift, smem) : 0;
+    const int cluster = (ch.kind == SOLVE_CLUSTER && planFits) ? ops.cluster_size(m.N, vpc, smem) : 0;
     if (cluster > 0)
     {
-        plan.shift = shift;
+        plan.vpc = vpc;
         // records each CTA handles: per colour a contiguous chunk of ceil(count / cluster)
         auto perCta = [&](const std::vector<int>& start) {
             int most = 0;

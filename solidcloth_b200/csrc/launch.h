@@ -148,7 +148,7 @@ constexpr int GS_THREADS = 512;
 constexpr int GS_SMEM_MAX = 200 * 1024; // dynamic shared memory per CTA: particles + staged records
 struct GsPlan
 {
-    int iterations, shift, nFemCol, nBendCol;
+    int iterations, vpc, nFemCol, nBendCol;   // vpc: particles per CTA (cluster solver)
     int stage;               // 1: each CTA copies its constraint records to shared memory first
     int femStage, bendStage; // records per CTA when staged (max over the cluster's CTAs)
     int femStart[65];
@@ -162,8 +162,8 @@ struct GsPlan
 // (the counts are known on the device alone).
 enum { GUARD_NONE = 0, GUARD_IF_SELF = 1, GUARD_IF_NO_SELF = 2 };
 // cluster size usable for N particles (0: too large or unsupported); sets the
-// log2 particles-per-CTA and the dynamic shared memory per CTA
-int gs_cluster_size(int N, int& shift, size_t& smem);
+// particles per CTA and the dynamic shared memory per CTA
+int gs_cluster_size(int N, int& vpc, size_t& smem);
 // variant 0: one constraint per thread; 1: two (their loads overlap)
 int gs_cluster_variants();
 void launch_gs_cluster(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, GsPlan plan,

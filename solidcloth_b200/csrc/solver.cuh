@@ -700,13 +700,19 @@ __device__ __forceinline__ bool guard_open(int guard, const ColourArgs& ca)
     return self == (guard == GUARD_IF_SELF);
 }
 
+// The cloth's particles in equal blocks over the cluster's CTAs. The block size is
+// N / CTAs, not the next power of two: the constraints are split evenly, and with
+// 1,024 particles a CTA a 91 x 91 cloth lay in 9 of 16 CTAs, away from most of its
+// constraints (516 -> 328 us a substep, fast build).
 struct ClusterPos
 {
     float4* local;
-    uint32_t shift, mask;
+    uint32_t vpc, inv;           // particles per CTA and ceil(2^32 / vpc): v / vpc = hi(v inv) for v vpc < 2^32
+    __device__ __forceinline__ ClusterPos(float4* p, uint32_t n) : local(p), vpc(n), inv(0xffffffffu / n + 1u) {}
     __device__ __forceinline__ float4* addr(uint32_t v) const
     {
-        return cg::this_cluster().map_shared_rank(local + (v & mask), v >> shift);
+        const uint32_t r = __umulhi(v, inv);
+        return cg::this_cluster().map_shared_rank(local + (v - r * vpc), r);
     }
     __device__ __forceinline__ float4 ld(uint32_t v) const { return *addr(v); }
     __device__ __forceinline__ void st(uint32_t v, float4 x) const { *addr(v) = x; }
@@ -950,7 +956,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_cluster(DevCloth c, SolverPar
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
     const int nRank = (int)cl.num_blocks();
-    const uint32_t vpc = 1u << plan.shift;
+    const uint32_t vpc = (uint32_t)plan.vpc;
     const int v0 = rank * (int)vpc;
     for (uint32_t v = threadIdx.x; v < vpc; v += blockDim.x)
     {
@@ -1006,7 +1012,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_cluster(DevCloth c, SolverPar
         }
     }
     cl.sync();
-    const ClusterPos pa{sPos, (uint32_t)plan.shift, vpc - 1};
+    const ClusterPos pa(sPos, vpc);
     const bool track = !P.fixedIterations;
     if (P.resTol > 0.f)
     {
@@ -1240,7 +1246,7 @@ __global__ void __launch_bounds__(NT) k_gs_band(DevCloth c, SolverParams P, Buff
     if (threadIdx.x < 8) sErr[threadIdx.x] = 0.f;
     cl.sync();
     const BandPos pa{sPos, sHalo, (uint32_t)v0, (uint32_t)v0 + vpc};
-    const ClusterPos cpa{sPos, (uint32_t)bv.shift, vpc - 1};
+    const ClusterPos cpa(sPos, vpc);
     const bool track = !P.fixedIterations;
     if (P.resTol > 0.f)
     {
@@ -2069,7 +2075,7 @@ bool launch_gs_grid(cudaStream_t s, const DevCloth& c, const SolverParams& P, co
 static const GridKernel kClusterVariants[] = {k_gs_cluster<1>, k_gs_cluster<2>};
 int gs_cluster_variants() { return 2; }
 
-int gs_cluster_size(int N, int& shift, size_t& smem)
+int gs_cluster_size(int N, int& vpc, size_t& smem)
 {
     static int supported = -1;
     if (supported < 0)
@@ -2101,10 +2107,8 @@ int gs_cluster_size(int N, int& shift, size_t& smem)
     }
     if (supported == 0) return 0;
     const int cs = supported;
-    int vpc = 1, sh = 0;
-    while (vpc * cs < N) { vpc <<= 1; sh++; }
+    vpc = std::max(8, ((N + cs - 1) / cs + 7) & ~7);
     if ((size_t)vpc * sizeof(float4) > 128 * 1024) return 0;
-    shift = sh;
     smem = (size_t)vpc * sizeof(float4);
     return cs;
 }

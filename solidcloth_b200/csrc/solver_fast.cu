@@ -10,6 +10,7 @@
 // stays bit-exact.
 #include "step_common.cuh"
 #include <cooperative_groups.h>
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
 
