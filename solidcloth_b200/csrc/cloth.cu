@@ -1032,7 +1032,8 @@ bool ClothModel::ensure_tile_plan()
     const bool selfProx = (prm.flags & CF_SELF) != 0;
     const int edgeSlots = (prm.flags & CF_EDGES) && instV.empty() ? feature_colliders() : 0;
     const int triSlots = (prm.flags & CF_TRIANGLES) && instV.empty() ? feature_colliders() : 0;
-    const std::vector<int> key = {N, prm.fem, prm.dihedral, selfProx, prm.ccd, edgeSlots, triSlots, (int)tris.size(), (int)bends.size(), (int)links.size()};
+    const std::vector<int> key = {N, prm.fem, prm.dihedral, selfProx, prm.ccd, edgeSlots, triSlots, (int)tris.size(), (int)bends.size(), (int)links.size(),
+                                  buf.stCap, buf.seCap};
     if (tilePlan.key == key) return tilePlan.valid;
     release_tile_plan();
     tilePlan.key = key;
@@ -1318,7 +1319,7 @@ bool ClothModel::ensure_tile_plan()
     // issue slots (a 17 x 17 cloth, 64 records a colour: 107 us a substep with 512
     // threads, 95 with 128)
     const int threads = mostRec <= 128 && !selfProx ? 128 : mostRec <= 256 && !selfProx ? 256 : 512;
-    if (gs_tile_max_blocks_per_sm(threads, tilePlan.smem) < 1) return false;
+    if (gs_tile_max_blocks_per_sm(threads, identity, tilePlan.smem) < 1) return false;
     // ---- device copies
     bool ok = true;
     auto put = [&](const void* h, size_t bytes) -> void* {
@@ -1355,6 +1356,7 @@ bool ClothModel::ensure_tile_plan()
         tc.entry = (int4*)put(entry[k].data(), sizeof(int4) * entry[k].size());
         tc.rec = (float4*)put(nullptr, sizeof(float4) * TILE_CT_WORDS * (size_t)tc.nSlot * (size_t)tc.nEntry);
     }
+    if (identity) v.selfRec = (float4*)put(nullptr, sizeof(float4) * 2 * ((size_t)buf.stCap + (size_t)buf.seCap));
     if (open)
     {
         v.xch = (float4*)put(nullptr, sizeof(float4) * 2 * (size_t)N);

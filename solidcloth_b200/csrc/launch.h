@@ -204,7 +204,7 @@ constexpr int BAND_SMEM_MAX = 220 * 1024;  // dynamic shared memory per CTA of t
 int gs_band_variants();
 int gs_band_threads(int variant);
 // resident CTAs of the tile solver per SM with smem bytes each (0: none)
-int gs_tile_max_blocks_per_sm(int threads, size_t smem);
+int gs_tile_max_blocks_per_sm(int threads, bool whole, size_t smem);
 // true if a cluster of clusterSize CTAs with smem bytes each can run the band solver
 bool gs_band_fits(int clusterSize, size_t smem);
 
@@ -251,6 +251,7 @@ struct TileView
     const float4* linkRec;
     float4* xch;                 // 2 N: exchanged positions, w = exchange number (as bits)
     unsigned long long* xred;    // 2 nTiles: exchanged iteration-end words (number << 32 | value)
+    float4* selfRec;             // identity: 2 words per self contact (stCap, then seCap of them), in colour order
 };
 
 // The solver's entry points as one table per build of solver.cuh: IEEE division

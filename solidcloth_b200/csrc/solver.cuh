@@ -1626,18 +1626,101 @@ __device__ __forceinline__ float tile_contact_sweep(const TilePos& pa, const Til
     return err;
 }
 
-// The contact classes of a cloth in one closed tile (local indices are the
-// particle indices), colour by colour with CTA barriers.
+// ---- self contacts of a cloth in one closed tile (local indices are the particle indices)
+// A folded cloth has some hundred colours of self contacts an iteration. Solved from the
+// contact lists, a colour was a chain of three dependent global loads (its start, the
+// order, the 64-byte contact) ahead of the projection. The contacts are copied once a
+// substep, in colour order, into 32-byte records of what the solve reads: two 16-bit
+// pairs of particles, the side, the list index; the normal and the multiplier. A
+// thread's record of the next colour is loaded before this colour's projections. A
+// thread has the same records in every iteration, so its multipliers need no barrier.
+// 48 x 48 folded cloth, 15,000 contacts: 4.1 -> 3.3 ms a substep, the frame 39.3 -> 32.8.
+template <int KIND, int NT>
+__device__ __forceinline__ void tile_self_records(float4* rec, const ClassView& cv, const SCt* list, const int* start)
+{
+    for (int j = (int)threadIdx.x; j < start[MAX_COLOURS - 1]; j += NT)
+    {
+        const int i = cv.order[j];
+        const SCt& k = list[i];
+        rec[2 * (size_t)j] = make_float4(__uint_as_float(k.idx.x | (k.idx.y << 16)), __uint_as_float(k.idx.z | (k.idx.w << 16)), k.side, __int_as_float(i));
+        rec[2 * (size_t)j + 1] = make_float4(k.normal.x, k.normal.y, k.normal.z, k.lam.x);
+    }
+}
+
+struct SelfRec { float4 a, b; };
+// volatile: a prefetch stays where it is written
+__device__ __forceinline__ SelfRec ld_self(const float4* rec, int j)
+{
+    SelfRec r;
+    const float4* p = rec + 2 * (size_t)j;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w) : "l"(p) : "memory");
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w) : "l"(p + 1) : "memory");
+    return r;
+}
+
+// one sweep of class KIND (2 vertex-triangle, 3 edge-edge) over the colours ahead of the serial one
+template <int KIND, int NT>
+__device__ __forceinline__ float tile_self_sweep(const TilePos& pa, const DevCloth& c, const SolverParams& P, SCt* list, float4* rec, const int* start)
+{
+    float err = 0.f;
+    int j = (int)threadIdx.x, e = start[1];
+    SelfRec cur;
+    if (j < e) cur = ld_self(rec, j);
+    for (int col = 0; col < MAX_COLOURS - 1 && start[col] < start[MAX_COLOURS - 1]; col++)
+    {
+        const int jn = e + (int)threadIdx.x, en = start[min(col + 2, MAX_COLOURS - 1)];
+        SelfRec nxt;
+        if (jn < en) nxt = ld_self(rec, jn);
+        while (j < e)
+        {
+            const unsigned u = __float_as_uint(cur.a.x), v = __float_as_uint(cur.a.y);
+            SCt k;
+            k.idx = make_uint4(u & 0xffffu, u >> 16, v & 0xffffu, v >> 16);
+            k.normal = cur.b; k.side = cur.a.z; k.lam = make_float2(cur.b.w, 0.f);
+            k.w = make_float4(0.f, 0.f, 0.f, 0.f); k.error = 0.f;
+            const float r = KIND == 2 ? solve_self_tri(pa, c, P, k) : solve_self_edge(pa, c, P, k);
+            err = fmaxf(err, r);
+            // the list, which the getters read
+            SCt& o = list[__float_as_int(cur.a.w)];
+            *reinterpret_cast<float2*>(&o.w) = make_float2(k.w.x, k.w.y);
+            if (KIND == 2) o.w.z = k.w.z;
+            if (!(r < 0.f))
+            {
+                o.lam.x = k.lam.x;
+                o.error = k.error;
+                rec[2 * (size_t)j + 1].w = k.lam.x;
+            }
+            j += NT;
+            if (j < e) cur = ld_self(rec, j);
+        }
+        __syncthreads();
+        cur = nxt;
+        j = jn; e = en;
+    }
+    return err;
+}
+
+// The contact classes of a cloth in one closed tile, colour by colour with CTA barriers.
 template <int NT>
-__device__ __forceinline__ void tile_contact_classes(const TilePos& pa, const DevCloth& c, const SolverParams& P,
-                                                     const Buffers& b, const ColourArgs& ca, bool track, float* sErr)
+__device__ __forceinline__ void tile_contact_classes(const TilePos& pa, const DevCloth& c, const SolverParams& P, const Buffers& b,
+                                                     const ColourArgs& ca, float4* const* rec, const int (*start)[MAX_COLOURS + 1],
+                                                     bool track, float* sErr)
 {
     for (int cls = 0; cls < 4; cls++)
     {
         const ClassView& cv = ca.cls[cls];
         const int n = *cv.count;
         if (n == 0) continue;
-        for (int col = 0; col < MAX_COLOURS; col++)
+        int first = 0;
+        if (cls >= 2)
+        {
+            const float e = cls == 2 ? tile_self_sweep<2, NT>(pa, c, P, b.stList, rec[0], start[0])
+                                     : tile_self_sweep<3, NT>(pa, c, P, b.seList, rec[1], start[1]);
+            if (track && e > 0.f) atomicMax((int*)&sErr[4 + cls], __float_as_int(e));
+            if (start[cls - 2][MAX_COLOURS - 1] == n) continue;
+            first = MAX_COLOURS - 1;
+        }
+        for (int col = first; col < MAX_COLOURS; col++)
         {
             const int s0 = cv.start[col], s1 = cv.start[col + 1];
             if (s0 == s1) continue;
@@ -1663,7 +1746,9 @@ __device__ __forceinline__ void tile_contact_classes(const TilePos& pa, const De
     }
 }
 
-template <int NT>
+// WHOLE: the one closed tile of a cloth with contact classes (TileView::identity); a
+// kernel of its own, because its contact solves cost the other one registers
+template <int NT, bool WHOLE>
 __global__ void __launch_bounds__(NT, 1) k_gs_tile(DevCloth c, SolverParams P, Buffers b, ColourArgs ca,
                                                               __grid_constant__ const TileView tv, int iterations, int guard)
 {
@@ -1672,17 +1757,18 @@ __global__ void __launch_bounds__(NT, 1) k_gs_tile(DevCloth c, SolverParams P, B
     __shared__ int sOff[3][65];
     __shared__ unsigned sRes;
     __shared__ int sCnt[2][MAX_COLOURS];
+    __shared__ int sStart[WHOLE ? 2 : 1][MAX_COLOURS + 1];
     if (blockIdx.x == 0 && threadIdx.x == 0) c.scal[0] = 0.f;      // for the next prediction; the detection is done
     if (!guard_open(guard, ca)) return;
     const int tid = (int)threadIdx.x;
     const bool track = !P.fixedIterations;
     // collider contacts of this substep (the same answer in every tile)
-    const bool edges = tv.edgeCt.nSlot > 0 && *ca.cls[0].count > 0, triangles = tv.triCt.nSlot > 0 && *ca.cls[1].count > 0;
+    const bool edges = !WHOLE && tv.edgeCt.nSlot > 0 && *ca.cls[0].count > 0, triangles = !WHOLE && tv.triCt.nSlot > 0 && *ca.cls[1].count > 0;
     for (int item = tv.ctaStart[blockIdx.x]; item < tv.ctaStart[blockIdx.x + 1]; item++)
     {
         const int t = tv.ctaTile[item];
         const TileDesc d = tv.tile[t];
-        TileLink<NT> lk{tv, sPos, tv.ids + d.idBase, t, d.nOwn, d.nLoc, d.peers, d.peerFirst, 0u, 0u, c.status};
+        TileLink<NT> lk{tv, sPos, tv.ids + d.idBase, t, d.nOwn, d.nLoc, WHOLE ? 1 : d.peers, d.peerFirst, 0u, 0u, c.status};
         for (int i = tid; i < d.nLoc; i += NT) sPos[i] = c.pos[__ldg(&lk.ids[i])];
         for (int j = tid; j <= tv.fem.nCol; j += NT) sOff[0][j] = __ldg(&tv.fem.off[t * (tv.fem.nCol + 1) + j]);
         for (int j = tid; j <= tv.bend.nCol; j += NT) sOff[1][j] = __ldg(&tv.bend.off[t * (tv.bend.nCol + 1) + j]);
@@ -1694,6 +1780,14 @@ __global__ void __launch_bounds__(NT, 1) k_gs_tile(DevCloth c, SolverParams P, B
             __syncthreads();
             if (edges) tile_contact_records<0, NT>(tv, c, b, d, t, sCnt[0]);
             if (triangles) tile_contact_records<1, NT>(tv, c, b, d, t, sCnt[1]);
+        }
+        float4* const selfRec[2] = {tv.selfRec, tv.selfRec + 2 * (size_t)b.stCap};
+        if constexpr (WHOLE)
+        {
+            for (int j = tid; j <= MAX_COLOURS; j += NT) { sStart[0][j] = ca.cls[2].start[j]; sStart[1][j] = ca.cls[3].start[j]; }
+            __syncthreads();
+            if (*ca.cls[2].count > 0) tile_self_records<2, NT>(selfRec[0], ca.cls[2], b.stList, sStart[0]);
+            if (*ca.cls[3].count > 0) tile_self_records<3, NT>(selfRec[1], ca.cls[3], b.seList, sStart[1]);
         }
         if (P.resTol > 0.f)
             for (int i = tid; i < d.nOwn; i += NT) c.xsnap[__ldg(&lk.ids[i])] = sPos[i];
@@ -1738,7 +1832,7 @@ __global__ void __launch_bounds__(NT, 1) k_gs_tile(DevCloth c, SolverParams P, B
                 err = tile_contact_sweep<1, NT>(TilePos{sPos}, tv, P, b, t, sCnt[1]);
                 if (track && err > 0.f) atomicMax((int*)&sErr[5], __float_as_int(err));
             }
-            if (tv.identity) tile_contact_classes<NT>(TilePos{sPos}, c, P, b, ca, track, sErr);
+            if constexpr (WHOLE) tile_contact_classes<NT>(TilePos{sPos}, c, P, b, ca, selfRec, sStart, track, sErr);
             // the last exchange of a launch is needed only if there was none before it:
             // no tile may write its particles back before its neighbours have loaded them
             if (lk.peers > 1 && (k + 1 < iterations || lk.seq == 0) && !(ok = lk.exchange())) break;
@@ -2192,22 +2286,27 @@ bool launch_gs_band(cudaStream_t s, const DevCloth& c, const SolverParams& P, co
 
 // ---------------------------------------------- tile solver launcher
 using TileKernel = void (*)(DevCloth, SolverParams, Buffers, ColourArgs, const TileView, int, int);
-static TileKernel tile_kernel(int threads) { return threads == 128 ? k_gs_tile<128> : threads == 256 ? k_gs_tile<256> : k_gs_tile<512>; }
+static TileKernel tile_kernel(int threads, bool whole)
+{
+    if (whole) return threads == 128 ? k_gs_tile<128, true> : threads == 256 ? k_gs_tile<256, true> : k_gs_tile<512, true>;
+    return threads == 128 ? k_gs_tile<128, false> : threads == 256 ? k_gs_tile<256, false> : k_gs_tile<512, false>;
+}
 
 static void tile_attributes()
 {
     static std::once_flag once;
     std::call_once(once, [] {
-        for (int t : {128, 256, 512}) cudaFuncSetAttribute(tile_kernel(t), cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM_MAX);
+        for (int t : {128, 256, 512})
+            for (bool whole : {false, true}) cudaFuncSetAttribute(tile_kernel(t, whole), cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM_MAX);
         cudaGetLastError();
     });
 }
 
-int gs_tile_max_blocks_per_sm(int threads, size_t smem)
+int gs_tile_max_blocks_per_sm(int threads, bool whole, size_t smem)
 {
     tile_attributes();
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_kernel(threads), threads, smem) != cudaSuccess) n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_kernel(threads, whole), threads, smem) != cudaSuccess) n = 0;
     cudaGetLastError();
     return n;
 }
@@ -2226,7 +2325,7 @@ bool launch_gs_tile(cudaStream_t s, const DevCloth& c, const SolverParams& P, co
     at.id = cudaLaunchAttributeCooperative;
     at.val.cooperative = tv.xch ? 1 : 0;
     cfg.attrs = &at; cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, tile_kernel(tv.threads), c, P, b, colour_args(b), tv, iterations, guard) == cudaSuccess;
+    return cudaLaunchKernelEx(&cfg, tile_kernel(tv.threads, tv.identity != 0), c, P, b, colour_args(b), tv, iterations, guard) == cudaSuccess;
 }
 
 // ---------------------------------------------- per-colour path launchers
