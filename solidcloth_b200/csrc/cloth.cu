@@ -1076,12 +1076,14 @@ bool ClothModel::ensure_tile_plan()
     std::vector<int> parts(G, 1);
     if (G == 1)
     {
-        // One tile up to 1,500 particles: a colour of it is a quarter of a microsecond
-        // on one SM, less than a split saves (32 x 32, 10 iterations: see the kernel's
-        // comment). With live self-proximity a cloth that fits stays in one tile as
-        // well: its contacts take a hundred colours an iteration, each a CTA barrier
-        // there and a cluster or grid barrier otherwise.
-        if (N > 1500 && !(selfProx && N <= fit)) parts[0] = sms;
+        // One tile below 700 particles, 64 or more particles a tile above (us a frame, one
+        // tile / 64 a tile): 24 x 24 drop 519 / 548, 28 x 28 582 / 560, 32 x 32 603 / 569,
+        // 36 x 36 706 / 591; 32 x 32 SDF drape 2356 / 1970. Every SM where there are fewer
+        // than 64 particles for each: 45 x 45 links 145 / 134 with 64 a tile, 64 x 64 SDF
+        // drape 2123 / 2064. With live self-proximity a cloth that fits stays in one tile:
+        // its contacts take a hundred colours an iteration, each a CTA barrier there and a
+        // cluster or grid barrier otherwise.
+        if (N >= 700 && !(selfProx && N <= fit)) parts[0] = std::min(sms, N / 64);
     }
     else
     {
