@@ -274,9 +274,9 @@ SCEXP int scMlpAdamStep(float* params, const float* grad, float* m, float* v, in
    (up to 131,072 particles); false: one kernel per colour. Same results. */
 SCEXP void scSetClusterSolver(scModel model, bool val);
 /* Solver for the Gauss-Seidel loop (additions, no reference counterpart).
-   0 = autotuned at the first step (default: the fastest of the cluster kernel,
-   the grid-resident cooperative kernel's variants and the per-colour kernels,
-   timed on this cloth), 1 = cluster kernel (clothes up to 131,072 particles),
+   0 = automatic (default: the tile kernel where the cloth has a tile plan, else
+   the fastest of the cluster kernel, the grid-resident cooperative kernel's
+   variants and the per-colour kernels, timed on this cloth at the first step), 1 = cluster kernel (clothes up to 131,072 particles),
    2 = grid kernel (tuned variant), 3 = per-colour kernels, 4 = band-parallel
    kernel (clothes with a band plan, scGetBandPlan; its thread count timed at
    the first step). Modes 0-3 give identical results (the colour order); the
