@@ -41,9 +41,9 @@ def _compare(build, frames, dt=1.0 / 60.0, tile=True):
         assert a[2] == b[2], (f, a[2], b[2])
 
 
-# 2 x 2 and 3 x 50: a handful of records a colour; 38 / 39 columns: the last size in
-# one closed tile (1,500 particles) and the first split one; 151: ragged tiles
-@pytest.mark.parametrize("shape", [(2, 2), (3, 50), (38, 39), (39, 39), (151, 20), (100, 100)])
+# 2 x 2 and 3 x 50: a handful of records a colour; 27 x 25 / 28 x 25: the last size in
+# one closed tile (below 700 particles) and the first split one; 151: ragged tiles
+@pytest.mark.parametrize("shape", [(2, 2), (3, 50), (27, 25), (28, 25), (38, 39), (39, 39), (151, 20), (100, 100)])
 @pytest.mark.parametrize("kind", ["fem", "bends", "links", "exit", "residual"])
 def test_grids(shape, kind):
     from solidcloth_b200 import api
