@@ -1021,6 +1021,8 @@ bool ClothModel::tile_eligible() const
     if (triColourStart.size() > 65 || bendColourStart.size() > 65 || linkColourStart.size() > 65) return false;
     if (!instV.empty() && (!prm.fixedIterations || prm.resTol > 0.f)) return false;
     const int slots = feature_colliders();
+    // a batch's plan has no records for them (scSetCollisionFlags on a batch asks for them)
+    if (!instV.empty() && slots > 0 && (prm.flags & (CF_TRIANGLES | CF_EDGES))) return false;
     if ((prm.flags & CF_TRIANGLES) && slots * dc.nTriColours >= MAX_COLOURS - 1) return false;
     if ((prm.flags & CF_EDGES) && slots * dc.nEdgeColours >= MAX_COLOURS - 1) return false;
     return dc.nTriColours <= 64 && dc.nEdgeColours <= 64;
