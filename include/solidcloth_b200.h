@@ -413,11 +413,13 @@ SCEXP int scGetKernelTiming(scClothPatch patch, float* ms, int* counts);
    Every triangle index is checked on the device: a triangle with an index
    >= numVertices is skipped (nothing is written for it) and the call returns
    SC_ERR_ARG; to report that, the call waits for its work on `stream` to finish.
-   Every call shares that scratch and leaves its contents behind; a call clears
-   what it uses first, but calls that overlap on the GPU race and must be
-   serialised by the caller. The first call on a device looks the scratch's
-   device address up, so make it before any stream capture that includes later
-   calls; later calls on a stream that is not capturing look it up again.
+   Every call on a device shares that scratch and puts zeros back for the next one;
+   calls that overlap on one GPU race and must be serialised by the caller (calls on
+   different GPUs share nothing). The first call registers 4 KiB of the library's own
+   host memory with the driver (cudaHostRegister; the check's outcome is written
+   there) and looks the scratch's device address up, so make it, on every device,
+   before any stream capture that includes later calls; later calls on a stream that
+   is not capturing look the address up again.
    Work is enqueued on `stream` (a cudaStream_t, NULL = legacy default).
    Returns 0 or an error code (details from scGetLastErrorString). */
 #define SC_NOALLOC_MAX_VERTICES 65536

@@ -19,8 +19,10 @@
 //     until the process exits;
 //   * every call shares that array; the normalisation puts zeros back for the next
 //     call (after a failed launch the next call clears the array first). Calls that
-//     overlap on the GPU (different streams, or another thread) race on it and must
-//     be serialised by the caller;
+//     overlap on one GPU (different streams, or another thread) race on it and must
+//     be serialised by the caller; calls on different GPUs share nothing;
+//   * the first call registers 4 KiB of the library's own host memory with the driver
+//     (cudaHostRegister), where the index check's outcome is written;
 //   * the first call on a device looks the array's device address up
 //     (cudaGetSymbolAddress) with that device current; make that first call
 //     before any stream capture that would include later calls. Later calls
@@ -29,6 +31,7 @@
 //   * the per-vertex sums use atomic adds, so the order of additions (and the
 //     last bits of the result) can differ from scUpdateClothMesh's ordered sum.
 #include "cloth.h"
+#include "host_words.h"
 #include "../../include/solidcloth_b200.h"
 #include <mutex>
 
@@ -39,10 +42,10 @@ static __device__ __align__(256) float4 g_noalloc_normal_acc[SC_NOALLOC_MAX_VERT
 // and of the last call
 static __device__ int g_noalloc_bad_triangles;
 static __device__ int g_noalloc_last_bad;
-// the same word in this library's own host memory, registered with the driver on the
-// first call: the kernel writes it and the call only waits for the stream (a copy of
-// four bytes to pageable memory cost 8 us of a call's 34)
-alignas(4096) static int g_noalloc_host[1024];
+// the same word, one per device, in this library's own host memory, registered with
+// the driver on the first call: the kernel writes it and the call only waits for the
+// stream (a copy of four bytes to pageable memory cost 8 us of a call's 34)
+static HostWords g_noalloc_host;
 
 // only after a call whose second kernel did not run
 __global__ void k_noalloc_clear(float4* acc)
@@ -102,26 +105,26 @@ __global__ void k_noalloc_normalise(float4* acc, int n, float* out, int* host)
 
 // device address of the scratch array, looked up once per device
 static std::mutex g_noalloc_mutex;
-static float4* g_noalloc_ptr[64] = {nullptr};
-static bool g_noalloc_dirty[64] = {false};      // a call ended between its kernels
+static float4* g_noalloc_ptr[HostWords::DEVICES] = {nullptr};
+static bool g_noalloc_dirty[HostWords::DEVICES] = {false};      // a call ended between its kernels
 
-// device address of g_noalloc_host, or null if it cannot be mapped (the word is then copied)
-static int* noalloc_host_word(bool capturing)
+// device address of the current device's word, or null if it cannot be mapped (the word is then copied)
+static int* noalloc_host_word(int dev, bool capturing)
 {
     std::lock_guard<std::mutex> lock(g_noalloc_mutex);
     static int state = 0;                       // 0 not tried, 1 registered, -1 not possible
     if (state == 0 && capturing) return nullptr;
     if (state == 0)
-        state = cudaHostRegister(g_noalloc_host, sizeof(g_noalloc_host), cudaHostRegisterPortable | cudaHostRegisterMapped) == cudaSuccess ? 1 : -1;
+        state = cudaHostRegister(g_noalloc_host.word, sizeof(g_noalloc_host.word), cudaHostRegisterPortable | cudaHostRegisterMapped) == cudaSuccess ? 1 : -1;
     void* d = nullptr;
-    if (state != 1 || cudaHostGetDevicePointer(&d, g_noalloc_host, 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    if (state != 1 || cudaHostGetDevicePointer(&d, g_noalloc_host.of(dev), 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }
     return (int*)d;
 }
 
 static float4* noalloc_scratch(int dev, bool capturing)
 {
     std::lock_guard<std::mutex> lock(g_noalloc_mutex);
-    if (dev < 0 || dev >= 64) return nullptr;
+    if (!HostWords::has(dev)) return nullptr;
     if (!g_noalloc_ptr[dev] || !capturing)
     {
         float4* p = nullptr;
@@ -168,7 +171,7 @@ extern "C" int scComputeVertexNormalsNoAlloc(const float* vertices, int numVerti
     if (e != cudaSuccess) { set_error(SC_ERR_CUDA, std::string("cudaStreamIsCapturing: ") + cudaGetErrorString(e)); return SC_ERR_CUDA; }
     float4* acc = noalloc_scratch(dev, cap != cudaStreamCaptureStatusNone);
     if (!acc) return SC_ERR_CUDA;
-    int* host = noalloc_host_word(cap != cudaStreamCaptureStatusNone);
+    int* host = noalloc_host_word(dev, cap != cudaStreamCaptureStatusNone);
     const int nb = (numVertices + 255) / 256;
     if (g_noalloc_dirty[dev]) k_noalloc_clear<<<(SC_NOALLOC_MAX_VERTICES + 255) / 256, 256, 0, s>>>(acc);
     if (numTriangles > 0)
@@ -177,11 +180,11 @@ extern "C" int scComputeVertexNormalsNoAlloc(const float* vertices, int numVerti
     e = cudaGetLastError();
     g_noalloc_dirty[dev] = e != cudaSuccess;
     if (e != cudaSuccess) { set_error(SC_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e)); return SC_ERR_CUDA; }
-    // the index check's outcome: read the device counter once the work is done
+    // the index check's outcome: this device's word, or a copy of its counter, once the work is done
     int bad = 0;
     if (!host) e = cudaMemcpyFromSymbolAsync(&bad, g_noalloc_last_bad, sizeof(int), 0, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (host) bad = *reinterpret_cast<volatile int*>(g_noalloc_host);
+    if (host) bad = *static_cast<volatile int*>(g_noalloc_host.of(dev));
     if (e != cudaSuccess) { set_error(SC_ERR_CUDA, std::string("status read: ") + cudaGetErrorString(e)); return SC_ERR_CUDA; }
     if (bad > 0)
     {
