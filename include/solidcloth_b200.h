@@ -304,6 +304,11 @@ SCEXP int scGetBandPlan(scModel model, int* out4);
    returns the mode asked for (1 by default) and zeros in ms2: nothing is tuned. */
 SCEXP void scSetBroadPhaseMode(scModel model, int mode);
 SCEXP int scGetBroadPhaseMode(scModel model, float* ms2);
+/* For tests of the error path: launches of these solver kinds (bit k: mode k; bit 5:
+   the tile kernel) are refused as if the driver had refused them. A solver that
+   cannot be launched leaves the substep to the per-colour kernels; where nothing can
+   take its place scStepCloth reports SC_ERR_CUDA. 0 (default): none. */
+SCEXP void scSetLaunchFault(scModel model, int kinds);
 /* info3 = {threads per CTA, FEM constraints per thread, bends per thread} per variant */
 SCEXP int scGetGridVariants(int* info3, int cap);
 /* true (default): the cluster solver copies each CTA's FEM and bend records to

@@ -138,6 +138,7 @@ SIGNATURES = {
     "scSetSelfCCD": ([scModel, C.c_bool], None),
     "scSetClusterSolver": ([scModel, C.c_bool], None),
     "scSetClusterStaging": ([scModel, C.c_bool], None),
+    "scSetLaunchFault": ([scModel, C.c_int], None),
     "scSetSolverPrecision": ([scModel, C.c_int], None),
     "scSetResidualUnit": ([scModel, C.c_int], None),
     "scSetClusterVariant": ([scModel, C.c_int], None),
@@ -386,6 +387,12 @@ class ClothModel:
         ms = np.zeros(2, np.float32)
         mode = lib().scGetBroadPhaseMode(self.h, ms.ctypes.data_as(_f))
         return int(mode), ms.copy()
+
+    def set_launch_fault(self, *kinds: int):
+        """for tests: launches of these solver kinds (0..4 as set_solver_mode, 5 the
+        tile kernel) are refused; none: as usual"""
+        lib().scSetLaunchFault(self.h, sum(1 << k for k in kinds))
+        _check("scSetLaunchFault")
 
     def set_cluster_staging(self, on: bool):
         lib().scSetClusterStaging(self.h, bool(on))

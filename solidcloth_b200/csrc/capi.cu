@@ -739,6 +739,12 @@ int scGetGridVariants(int* info3, int cap)
     for (int v = 0; info3 && v < n && v < cap; v++) gs_grid_variant_info(v, info3[3 * v], info3[3 * v + 1], info3[3 * v + 2]);
     return n;
 }
+void scSetLaunchFault(scModel m, int kinds)
+{
+    if (!M(m)) { set_error(SC_ERR_ARG, "null model"); return; }
+    M(m)->launchFault = kinds;
+    M(m)->touch();
+}
 void scSetClusterStaging(scModel m, bool v) { if (M(m)) { M(m)->prm.stageRecords = v; M(m)->touch(); } }
 void scSetSolverPrecision(scModel m, int mode)
 {

@@ -2362,7 +2362,8 @@ void ClothPatch::sync()
 }
 
 // One substep (ClothModelPBD::Step) recorded into the capture stream.
-void ClothPatch::record_substep(float h)
+// False (and an error) if its solve could not be launched.
+bool ClothPatch::record_substep(float h)
 {
     ClothModel& m = model;
     const SolverParams P = m.solver_params(h);
@@ -2418,17 +2419,24 @@ void ClothPatch::record_substep(float h)
     // ClothModelPBD::SolveGS (Physics/ClothPBD.cpp:324-369)
     if (!tiles) launch_reset_gs(s, c);
     timing_mark(SEC_GS, false, s);
-    record_solve(s, P, m.choice);
+    if (!record_solve(s, P, m.choice))
+    {
+        const cudaError_t e = cudaGetLastError();
+        set_error(SC_ERR_CUDA, std::string("solver launch failed: ") + cudaGetErrorString(e));
+        return false;
+    }
     timing_mark(SEC_GS, true, s);
     if (learn) launch_mlp_targets(s, c, m.sampleTarget ? m.sampleTarget + sub * m.N * MLP_OUT : nullptr);
     recordingSubstep++;
+    return true;
 }
 
 
 // One substep's Gauss-Seidel loop and velocity update, by the chosen solver:
 // the cluster-resident kernel, the grid-resident cooperative kernel (a tuned
 // variant), or one kernel per colour. The three are the same algorithm in the
-// same order (bit-identical results).
+// same order (bit-identical results). A solver whose launch fails leaves the work
+// to the kernels per colour; false: nothing solves this substep.
 bool ClothPatch::record_solve(cudaStream_t s, const SolverParams& P, const SolverChoice& ch)
 {
     ClothModel& m = model;
@@ -2470,23 +2478,34 @@ bool ClothPatch::record_solve(cudaStream_t s, const SolverParams& P, const Solve
         plan.nLinkCol = (int)m.linkColourStart.size() - 1;
         for (size_t k = 0; k < m.linkColourStart.size(); k++) plan.linkStart[k] = m.linkColourStart[k];
     }
+    // a launch, unless the model refuses its kind (scSetLaunchFault); a failed one's error is taken
+    auto launched = [&](int kind, auto&& launch) {
+        if (!(m.launchFault >> kind & 1) && launch()) return true;
+        cudaGetLastError();
+        return false;
+    };
     int vpc = 0;
     size_t smem = 0;
     if (ch.kind == SOLVE_TILE && m.tilePlan.valid)
     {
         // self contacts across tiles go to the launch after it (GUARD_*)
         const bool other = !m.tilePlan.view.identity && ((m.prm.flags & CF_SELF) || m.prm.ccd);
-        if (!ops.tile(s, c, P, b, m.tilePlan.view, m.tilePlan.ctas, m.tilePlan.smem, iterations, other ? GUARD_IF_NO_SELF : GUARD_NONE))
-            return false;
-        if (!other) return true;
-        plan.guard = GUARD_IF_SELF;
-        const int cs = ops.cluster_size(m.N, vpc, smem);
-        plan.vpc = vpc;
-        if (cs > 0) { ops.cluster(s, c, P, b, plan, cs, smem, 0); return true; }
-        return ops.grid(s, c, P, b, plan, 0, 1);
+        if (launched(SOLVE_TILE, [&] {
+                return ops.tile(s, c, P, b, m.tilePlan.view, m.tilePlan.ctas, m.tilePlan.smem, iterations, other ? GUARD_IF_NO_SELF : GUARD_NONE);
+            }))
+        {
+            if (!other) return true;
+            plan.guard = GUARD_IF_SELF;
+            const int cs = ops.cluster_size(m.N, vpc, smem);
+            plan.vpc = vpc;
+            if (cs > 0 && launched(SOLVE_CLUSTER, [&] { return ops.cluster(s, c, P, b, plan, cs, smem, 0); })) return true;
+            return launched(SOLVE_GRID, [&] { return ops.grid(s, c, P, b, plan, 0, 1); });
+        }
+        cudaMemsetAsync(c.scal, 0, sizeof(float), s);                // what k_gs_tile clears for the next prediction
     }
-    if (ch.kind == SOLVE_BAND && m.band_active() &&
-        ops.band(s, c, P, b, plan, m.bandPlan.view, m.bandPlan.clusterSize, m.band_smem(), ch.variant))
+    if (ch.kind == SOLVE_BAND && m.band_active() && launched(SOLVE_BAND, [&] {
+            return ops.band(s, c, P, b, plan, m.bandPlan.view, m.bandPlan.clusterSize, m.band_smem(), ch.variant);
+        }))
         return true;                                                 // includes the velocity update
     const int cluster = (ch.kind == SOLVE_CLUSTER && planFits) ? ops.cluster_size(m.N, vpc, smem) : 0;
     if (cluster > 0)
@@ -2515,10 +2534,10 @@ bool ClothPatch::record_solve(cudaStream_t s, const SolverParams& P, const Solve
             plan.stage = 1;
             smem = staged;
         }
-        ops.cluster(s, c, P, b, plan, cluster, smem, ch.variant);   // includes the velocity update
-        return true;
+        if (launched(SOLVE_CLUSTER, [&] { return ops.cluster(s, c, P, b, plan, cluster, smem, ch.variant); }))
+            return true;                                             // includes the velocity update
     }
-    if (ch.kind == SOLVE_GRID && planFits && ops.grid(s, c, P, b, plan, ch.variant, ch.blocksPerSm))
+    if (ch.kind == SOLVE_GRID && planFits && launched(SOLVE_GRID, [&] { return ops.grid(s, c, P, b, plan, ch.variant, ch.blocksPerSm); }))
         return true;
     if (P.resTol > 0.f) launch_residual_exit(s, c, P, -1);
     for (int k = 0; k < iterations; k++)
@@ -2617,8 +2636,8 @@ bool ClothPatch::autotune(float h)
         cudaGraphExec_t ge = nullptr;
         if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) continue;
         launch_reset_gs(stream, m.dc, ch.kind == SOLVE_TILE ? &m.tilePlan.view : nullptr);
-        record_solve(stream, P, ch);
-        if (cudaStreamEndCapture(stream, &g) != cudaSuccess || cudaGraphInstantiate(&ge, g, 0) != cudaSuccess)
+        const bool recorded = record_solve(stream, P, ch);
+        if (cudaStreamEndCapture(stream, &g) != cudaSuccess || !recorded || cudaGraphInstantiate(&ge, g, 0) != cudaSuccess)
         {
             if (g) cudaGraphDestroy(g);
             cudaGetLastError();
@@ -2726,10 +2745,12 @@ bool ClothPatch::step(float dt)
         const int frames = timingFrames;
         timingFrames = 0;
         recordingSubstep = 0;
-        for (int i = 0; i < n; i++) record_substep(h);
-        timingFrames = frames;
-        SC_CUDA(cudaGetLastError());
+        bool ok = true;
         hostStateDirty = true;
+        for (int i = 0; i < n && ok; i++) ok = record_substep(h);
+        timingFrames = frames;
+        if (!ok) return false;
+        SC_CUDA(cudaGetLastError());
         return true;
     }
     if (!graph || graphDt != dt || graphSteps != n || graphParamVersion != m.paramVersion || graphWorldVersion != world.version)
@@ -2747,7 +2768,14 @@ bool ClothPatch::step(float dt)
         if (timingFrames && timingCapture.size() != (size_t)n * NSEC * 2) set_timing(timingFrames);
         recordingSubstep = 0;
         SC_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        for (int i = 0; i < n; i++) record_substep(h);
+        bool ok = true;
+        for (int i = 0; i < n && ok; i++) ok = record_substep(h);
+        if (!ok)
+        {
+            if (cudaStreamEndCapture(stream, &g) == cudaSuccess && g) cudaGraphDestroy(g);
+            cudaGetLastError();
+            return false;
+        }
         SC_CUDA(cudaStreamEndCapture(stream, &g));
         size_t numNodes = 0;
         cudaGraphGetNodes(g, nullptr, &numNodes);

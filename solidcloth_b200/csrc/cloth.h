@@ -197,6 +197,7 @@ public:
     SolverChoice choice{SOLVE_CLUSTER, 0, 0, 0.f};
     bool tuned = false;
     uint64_t tunedVersion = 0;
+    int launchFault = 0;                        // solver kinds whose launches are refused (scSetLaunchFault)
     std::vector<SolverChoice> tuneLog;          // candidates and their times of the last tuning
     int broadMode = -1;                         // what scSetBroadPhaseMode asked for
     void colour_constraints();
@@ -281,7 +282,7 @@ public:
     std::vector<int> meshMap;                  // mesh cloth: input vertex -> particle
     bool step(float dt);
     void update_mesh();
-    void record_substep(float h);
+    bool record_substep(float h);
     bool record_solve(cudaStream_t s, const SolverParams& P, const SolverChoice& ch);
     bool autotune(float h);
     void sync();

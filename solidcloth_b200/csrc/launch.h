@@ -166,7 +166,7 @@ enum { GUARD_NONE = 0, GUARD_IF_SELF = 1, GUARD_IF_NO_SELF = 2 };
 int gs_cluster_size(int N, int& vpc, size_t& smem);
 // variant 0: one constraint per thread; 1: two (their loads overlap)
 int gs_cluster_variants();
-void launch_gs_cluster(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, GsPlan plan,
+bool launch_gs_cluster(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, GsPlan plan,
                        int clusterSize, size_t smem, int variant);
 
 // grid-resident solver (cooperative launch, any cloth or batch size); variants
@@ -268,7 +268,7 @@ struct SolverOps
     void (*vertex_contacts)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&);
     void (*multi_contacts)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&, int);
     int (*cluster_size)(int, int&, size_t&);
-    void (*cluster)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&, GsPlan, int, size_t, int);
+    bool (*cluster)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&, GsPlan, int, size_t, int);
     int (*grid_max_blocks_per_sm)(int);
     bool (*grid)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&, GsPlan, int, int);
     bool (*band)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&, GsPlan, const BandView&, int, size_t,

@@ -2207,7 +2207,7 @@ int gs_cluster_size(int N, int& vpc, size_t& smem)
     return cs;
 }
 
-void launch_gs_cluster(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, GsPlan plan,
+bool launch_gs_cluster(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, GsPlan plan,
                        int clusterSize, size_t smem, int variant)
 {
     cudaLaunchConfig_t cfg = {};
@@ -2219,7 +2219,7 @@ void launch_gs_cluster(cudaStream_t s, const DevCloth& c, const SolverParams& P,
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = clusterSize; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
     cfg.attrs = &at; cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kClusterVariants[variant == 1 ? 1 : 0], c, P, b, colour_args(b), plan);
+    return cudaLaunchKernelEx(&cfg, kClusterVariants[variant == 1 ? 1 : 0], c, P, b, colour_args(b), plan) == cudaSuccess;
 }
 
 // ---------------------------------------------- band solver launchers
