@@ -1932,12 +1932,12 @@ bool ClothModel::ensure_buffers(const CollisionWorld& world, cudaStream_t s)
     buf.ccdVtTest = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdVtCap, true);
     buf.ccdEeTest = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdEeCap, true);
     buf.ccdVtTestCount = counts + 9; buf.ccdEeTestCount = counts + 10;
-    buf.ccdVtHitCap = ccd ? N * CCD_VT_HITS : 1;
-    buf.ccdEeHitCap = ccd ? E * CCD_EE_HITS : 1;
-    buf.ccdVtHits = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdVtHitCap, true);
-    buf.ccdEeHits = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdEeHitCap, true);
-    buf.ccdVtSorted = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdVtHitCap, true);
-    buf.ccdEeSorted = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdEeHitCap, true);
+    // every tested pair may be a hit, so that a contact list that is too short keeps the
+    // first of them all in order; the sorted hits lie where the tested pairs were
+    buf.ccdVtHits = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdVtCap, true);
+    buf.ccdEeHits = (int2*)dalloc(sizeof(int2) * (size_t)buf.ccdEeCap, true);
+    buf.ccdVtSorted = buf.ccdVtTest;
+    buf.ccdEeSorted = buf.ccdEeTest;
     buf.ccdVtHitTotal = counts + 6; buf.ccdEeHitTotal = counts + 7;
     buf.ccdVtHitCnt = (int*)dalloc(sizeof(int) * N, true);
     buf.ccdEeHitCnt = (int*)dalloc(sizeof(int) * E, true);

@@ -65,7 +65,7 @@ struct Buffers
     // test, and the hits among them with each query's number of hits
     int2* ccdVtPairs; int2* ccdEePairs; int* ccdVtPairCount; int* ccdEePairCount; int ccdVtCap, ccdEeCap;
     int2* ccdVtTest; int2* ccdEeTest; int* ccdVtTestCount; int* ccdEeTestCount;
-    int2* ccdVtHits; int2* ccdEeHits; int* ccdVtHitTotal; int* ccdEeHitTotal; int ccdVtHitCap, ccdEeHitCap;
+    int2* ccdVtHits; int2* ccdEeHits; int* ccdVtHitTotal; int* ccdEeHitTotal;
     int* ccdVtHitCnt; int* ccdEeHitCnt;
     int2* ccdVtSorted; int2* ccdEeSorted;
     // colouring scratch

@@ -1862,9 +1862,7 @@ __global__ void __launch_bounds__(128) k_ccd_test(DevCloth c, SolverParams P, Bu
         SCt rec;
         if (!(vt ? ccd_vt_test(c, P, p.x, p.y, rec) : ccd_ee_test(c, P, p.x, p.y, rec))) continue;
         atomicAdd(&(vt ? b.ccdVtHitCnt : b.ccdEeHitCnt)[p.x], 1);
-        const int h = atomicAdd(vt ? b.ccdVtHitTotal : b.ccdEeHitTotal, 1);
-        if (h < (vt ? b.ccdVtHitCap : b.ccdEeHitCap)) (vt ? b.ccdVtHits : b.ccdEeHits)[h] = p;
-        else atomicOr(c.status, ST_CCD_OVERFLOW);
+        (vt ? b.ccdVtHits : b.ccdEeHits)[atomicAdd(vt ? b.ccdVtHitTotal : b.ccdEeHitTotal, 1)] = p;
     }
 }
 
@@ -1878,7 +1876,7 @@ __device__ void append_hits(const DevCloth& c, const SolverParams& P, const Buff
     int* listCount = VT ? b.stCount : b.seCount;
     SCt* list = VT ? b.stList : b.seList;
     const int listCap = VT ? b.stCap : b.seCap;
-    const int base = *listCount, h = min(VT ? *b.ccdVtHitTotal : *b.ccdEeHitTotal, VT ? b.ccdVtHitCap : b.ccdEeHitCap);
+    const int base = *listCount, h = VT ? *b.ccdVtHitTotal : *b.ccdEeHitTotal;
     __syncthreads();
     if (threadIdx.x == 0) *listCount = min(listCap, base + h);
     if (h == 0) return;
@@ -1897,18 +1895,6 @@ __device__ void append_hits(const DevCloth& c, const SolverParams& P, const Buff
     }
     if (threadIdx.x == 0) off[n] = carry;
     __syncthreads();
-    if (carry > h)
-    {
-        // hits beyond the store (recorded in the status): the counts do not match it
-        for (int k = threadIdx.x; k < h; k += blockDim.x)
-        {
-            SCt rec;
-            const int2 p = hits[k];
-            if (VT) ccd_vt_test(c, P, p.x, p.y, rec); else ccd_ee_test(c, P, p.x, p.y, rec);
-            if (base + k < listCap) list[base + k] = rec;
-        }
-        return;
-    }
     for (int k = threadIdx.x; k < h; k += blockDim.x)
     {
         const int2 p = hits[k];
