@@ -2292,20 +2292,18 @@ static TileKernel tile_kernel(int threads, bool whole)
     return threads == 128 ? k_gs_tile<128, false> : threads == 256 ? k_gs_tile<256, false> : k_gs_tile<512, false>;
 }
 
-static void tile_attributes()
+// The shared memory limit is the device's own and this build's: raised with every plan
+// and launch that may need more than the 48 KB, static shared memory included, that
+// every kernel has (a once-flag for the process would leave a second device without it).
+static void tile_smem_limit(TileKernel k, size_t smem)
 {
-    static std::once_flag once;
-    std::call_once(once, [] {
-        for (int t : {128, 256, 512})
-            for (bool whole : {false, true}) cudaFuncSetAttribute(tile_kernel(t, whole), cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM_MAX);
-        cudaGetLastError();
-    });
+    if (smem > 32 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM_MAX);
 }
 
 int gs_tile_max_blocks_per_sm(int threads, bool whole, size_t smem)
 {
-    tile_attributes();
     int n = 0;
+    tile_smem_limit(tile_kernel(threads, whole), smem);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_kernel(threads, whole), threads, smem) != cudaSuccess) n = 0;
     cudaGetLastError();
     return n;
@@ -2315,7 +2313,8 @@ int gs_tile_max_blocks_per_sm(int threads, bool whole, size_t smem)
 bool launch_gs_tile(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, const TileView& tv,
                     int ctas, size_t smem, int iterations, int guard)
 {
-    tile_attributes();
+    const TileKernel kernel = tile_kernel(tv.threads, tv.identity != 0);
+    tile_smem_limit(kernel, smem);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
     cfg.blockDim = dim3(tv.threads);
@@ -2325,7 +2324,7 @@ bool launch_gs_tile(cudaStream_t s, const DevCloth& c, const SolverParams& P, co
     at.id = cudaLaunchAttributeCooperative;
     at.val.cooperative = tv.xch ? 1 : 0;
     cfg.attrs = &at; cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, tile_kernel(tv.threads, tv.identity != 0), c, P, b, colour_args(b), tv, iterations, guard) == cudaSuccess;
+    return cudaLaunchKernelEx(&cfg, kernel, c, P, b, colour_args(b), tv, iterations, guard) == cudaSuccess;
 }
 
 // ---------------------------------------------- per-colour path launchers
