@@ -794,7 +794,7 @@ int scGetIterationTotal(scModel m)
     host_sync(c);
     float v = 0.f;
     cudaMemcpy(&v, c->dc.scal + 10, sizeof(float), cudaMemcpyDeviceToHost);
-    cudaMemset(c->dc.scal + 10, 0, sizeof(float));
+    cudaMemsetAsync(c->dc.scal + 10, 0, sizeof(float), c->owner->stream);     // ahead of the next step
     return (int)v;
 }
 
@@ -1073,7 +1073,7 @@ int scGetStatus(scClothPatch p)
     P(p)->sync();
     int s = 0;
     cudaMemcpy(&s, P(p)->model.dc.status, sizeof(int), cudaMemcpyDeviceToHost);
-    cudaMemset(P(p)->model.dc.status, 0, sizeof(int));
+    cudaMemsetAsync(P(p)->model.dc.status, 0, sizeof(int), P(p)->stream);
     return s;
 }
 

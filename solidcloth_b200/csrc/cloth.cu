@@ -465,6 +465,13 @@ ClothModel::~ClothModel()
     if (mlpPrm) cudaFree(mlpPrm);
 }
 
+// Zeroes device memory and waits for it: cudaMemset returns before the legacy stream
+// has done it, and a model's streams do not wait for that stream.
+static bool zero_device(void* p, size_t bytes)
+{
+    return cudaMemset(p, 0, bytes) == cudaSuccess && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess;
+}
+
 void* ClothModel::dalloc(size_t bytes, bool contact)
 {
     void* p = nullptr;
@@ -474,7 +481,12 @@ void* ClothModel::dalloc(size_t bytes, bool contact)
         set_error(SC_ERR_CUDA, "cudaMalloc failed");
         return nullptr;
     }
-    cudaMemset(p, 0, bytes);
+    if (!zero_device(p, bytes))
+    {
+        cudaFree(p);
+        set_error(SC_ERR_CUDA, "cudaMemset failed");
+        return nullptr;
+    }
     (contact ? bufAllocs : allocs).push_back(p);
     return p;
 }
@@ -1330,7 +1342,7 @@ bool ClothModel::ensure_tile_plan()
         void* p = nullptr;
         if (!ok || cudaMalloc(&p, std::max<size_t>(bytes, 16)) != cudaSuccess) { cudaGetLastError(); ok = false; return nullptr; }
         tileAllocs.push_back(p);
-        if (h ? cudaMemcpy(p, h, bytes, cudaMemcpyHostToDevice) != cudaSuccess : cudaMemset(p, 0, bytes) != cudaSuccess) ok = false;
+        if (!(h ? cudaMemcpy(p, h, bytes, cudaMemcpyHostToDevice) == cudaSuccess : zero_device(p, bytes))) ok = false;
         return p;
     };
     TileView& v = tilePlan.view;
