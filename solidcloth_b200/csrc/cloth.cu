@@ -2444,6 +2444,52 @@ bool ClothPatch::record_substep(float h)
 }
 
 
+// What runs behind a tile launch when there are self contacts: the cluster solver up to
+// GUARD_CLUSTER particles, the grid solver above, with as many CTAs an SM as pay off.
+// Not tuned: most clothes with continuous collision never meet a contact there, and the
+// tuning of 14 kernels costs their first step 70 ms. Measured by it, ms a substep,
+// cluster / grid with one CTA an SM: 160 x 160 0.46 / 0.68, 200 x 200 0.59 / 0.69,
+// 256 x 256 0.78 / 0.69; grid with 1 / 2 / 3 an SM: 131,044 particles 0.73 / 0.88,
+// 229,076 1.08 / 0.92, 485,293 1.64 / 1.43, 1,886,304 6.7 / 4.3 / 3.6.
+constexpr int GUARD_CLUSTER = 52000, GUARD_GRID_1 = 180000, GUARD_GRID_2 = 1000000;
+
+// the cluster solver, its records staged in shared memory where they fit; false: no
+// cluster of that size, or its launch failed
+bool ClothPatch::record_cluster(cudaStream_t s, const SolverParams& P, GsPlan plan, int variant)
+{
+    ClothModel& m = model;
+    const SolverOps& ops = solver_ops(m.prm.fastMath);
+    int vpc = 0;
+    size_t smem = 0;
+    const int cluster = ops.cluster_size(m.N, vpc, smem);
+    if (cluster < 1) return false;
+    plan.vpc = vpc;
+    // records each CTA handles: per colour a contiguous chunk of ceil(count / cluster)
+    auto perCta = [&](const std::vector<int>& start) {
+        int most = 0;
+        for (int r = 0; r < cluster; r++)
+        {
+            int sum = 0;
+            for (size_t k = 0; k + 1 < start.size(); k++)
+            {
+                const int cnt = start[k + 1] - start[k], chunk = (cnt + cluster - 1) / cluster;
+                sum += std::max(0, std::min(chunk, cnt - r * chunk));
+            }
+            most = std::max(most, sum);
+        }
+        return most;
+    };
+    plan.femStage = perCta(m.triColourStart);
+    plan.bendStage = perCta(m.bendColourStart);
+    const size_t staged = smem + (size_t)plan.femStage * 3 * sizeof(float4) + (size_t)plan.bendStage * sizeof(uint4);
+    if (m.prm.stageRecords && staged <= (size_t)GS_SMEM_MAX)
+    {
+        plan.stage = 1;
+        smem = staged;
+    }
+    return m.launched(SOLVE_CLUSTER, [&] { return ops.cluster(s, m.dc, P, m.buf, plan, cluster, smem, variant); });
+}
+
 // One substep's Gauss-Seidel loop and velocity update, by the chosen solver:
 // the cluster-resident kernel, the grid-resident cooperative kernel (a tuned
 // variant), or one kernel per colour. The three are the same algorithm in the
@@ -2490,14 +2536,7 @@ bool ClothPatch::record_solve(cudaStream_t s, const SolverParams& P, const Solve
         plan.nLinkCol = (int)m.linkColourStart.size() - 1;
         for (size_t k = 0; k < m.linkColourStart.size(); k++) plan.linkStart[k] = m.linkColourStart[k];
     }
-    // a launch, unless the model refuses its kind (scSetLaunchFault); a failed one's error is taken
-    auto launched = [&](int kind, auto&& launch) {
-        if (!(m.launchFault >> kind & 1) && launch()) return true;
-        cudaGetLastError();
-        return false;
-    };
-    int vpc = 0;
-    size_t smem = 0;
+    auto launched = [&](int kind, auto&& launch) { return m.launched(kind, launch); };
     if (ch.kind == SOLVE_TILE && m.tilePlan.valid)
     {
         // self contacts across tiles go to the launch after it (GUARD_*)
@@ -2508,10 +2547,8 @@ bool ClothPatch::record_solve(cudaStream_t s, const SolverParams& P, const Solve
         {
             if (!other) return true;
             plan.guard = GUARD_IF_SELF;
-            const int cs = ops.cluster_size(m.N, vpc, smem);
-            plan.vpc = vpc;
-            if (cs > 0 && launched(SOLVE_CLUSTER, [&] { return ops.cluster(s, c, P, b, plan, cs, smem, 0); })) return true;
-            return launched(SOLVE_GRID, [&] { return ops.grid(s, c, P, b, plan, 0, 1); });
+            if (m.N <= GUARD_CLUSTER && record_cluster(s, P, plan, 0)) return true;
+            return launched(SOLVE_GRID, [&] { return ops.grid(s, c, P, b, plan, 0, m.N <= GUARD_GRID_1 ? 1 : m.N <= GUARD_GRID_2 ? 2 : 3); });
         }
         cudaMemsetAsync(c.scal, 0, sizeof(float), s);                // what k_gs_tile clears for the next prediction
     }
@@ -2519,36 +2556,8 @@ bool ClothPatch::record_solve(cudaStream_t s, const SolverParams& P, const Solve
             return ops.band(s, c, P, b, plan, m.bandPlan.view, m.bandPlan.clusterSize, m.band_smem(), ch.variant);
         }))
         return true;                                                 // includes the velocity update
-    const int cluster = (ch.kind == SOLVE_CLUSTER && planFits) ? ops.cluster_size(m.N, vpc, smem) : 0;
-    if (cluster > 0)
-    {
-        plan.vpc = vpc;
-        // records each CTA handles: per colour a contiguous chunk of ceil(count / cluster)
-        auto perCta = [&](const std::vector<int>& start) {
-            int most = 0;
-            for (int r = 0; r < cluster; r++)
-            {
-                int sum = 0;
-                for (size_t k = 0; k + 1 < start.size(); k++)
-                {
-                    const int cnt = start[k + 1] - start[k], chunk = (cnt + cluster - 1) / cluster;
-                    sum += std::max(0, std::min(chunk, cnt - r * chunk));
-                }
-                most = std::max(most, sum);
-            }
-            return most;
-        };
-        plan.femStage = perCta(m.triColourStart);
-        plan.bendStage = perCta(m.bendColourStart);
-        const size_t staged = smem + (size_t)plan.femStage * 3 * sizeof(float4) + (size_t)plan.bendStage * sizeof(uint4);
-        if (m.prm.stageRecords && staged <= (size_t)GS_SMEM_MAX)
-        {
-            plan.stage = 1;
-            smem = staged;
-        }
-        if (launched(SOLVE_CLUSTER, [&] { return ops.cluster(s, c, P, b, plan, cluster, smem, ch.variant); }))
-            return true;                                             // includes the velocity update
-    }
+    if (ch.kind == SOLVE_CLUSTER && planFits && record_cluster(s, P, plan, ch.variant))
+        return true;                                                 // includes the velocity update
     if (ch.kind == SOLVE_GRID && planFits && launched(SOLVE_GRID, [&] { return ops.grid(s, c, P, b, plan, ch.variant, ch.blocksPerSm); }))
         return true;
     if (P.resTol > 0.f) launch_residual_exit(s, c, P, -1);

@@ -198,6 +198,14 @@ public:
     bool tuned = false;
     uint64_t tunedVersion = 0;
     int launchFault = 0;                        // solver kinds whose launches are refused (scSetLaunchFault)
+    // a solver launch, unless its kind is refused; a failed one's error is taken
+    template <class F>
+    bool launched(int kind, F&& launch)
+    {
+        if (!(launchFault >> kind & 1) && launch()) return true;
+        cudaGetLastError();
+        return false;
+    }
     std::vector<SolverChoice> tuneLog;          // candidates and their times of the last tuning
     int broadMode = -1;                         // what scSetBroadPhaseMode asked for
     void colour_constraints();
@@ -284,6 +292,7 @@ public:
     void update_mesh();
     bool record_substep(float h);
     bool record_solve(cudaStream_t s, const SolverParams& P, const SolverChoice& ch);
+    bool record_cluster(cudaStream_t s, const SolverParams& P, GsPlan plan, int variant);
     bool autotune(float h);
     void sync();
 };

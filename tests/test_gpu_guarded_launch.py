@@ -1,0 +1,81 @@
+"""Clothes split into tiles that do meet self contacts: the launches behind the tile
+launch (the cluster solver and the grid solver, by size) against the per-colour path,
+bit for bit."""
+import numpy as np
+import pytest
+
+from solidcloth_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+TILE, CLUSTER, GRID, KERNELS = 5, 1, 2, 3
+
+
+def _colours(p):
+    return sum(int(np.count_nonzero(p.model.contact_colours(k))) for k in (2, 3))
+
+
+def _run(build, frames, dt, mode, faults=()):
+    """states after each frame, the contact colours of each frame's last substep, the solver kind"""
+    p = build()
+    p.model.set_solver_mode(mode)
+    p.model.set_launch_fault(*faults)
+    out, colours = [], []
+    for _ in range(frames):
+        p.step(dt)
+        out.append([np.ascontiguousarray(a, np.float32).view(np.uint32) for a in (p.model.positions(), p.model.velocities())])
+        colours.append(_colours(p))
+    kind, status = p.model.solver_choice()[0][0], p.status()
+    p.free()
+    return out, colours, kind, status
+
+
+def _compare(build, frames, dt, faults=()):
+    got, c0, kind, s0 = _run(build, frames, dt, 0, faults)
+    want, c1, _, s1 = _run(build, frames, dt, KERNELS)
+    assert kind == TILE and c0 == c1 and s0 == s1 and s0 & 256 == 0
+    for f, (a, b) in enumerate(zip(got, want)):
+        for x, y in zip(a, b):
+            assert np.array_equal(x, y), f
+    return c0
+
+
+@pytest.mark.parametrize("n,faults", [(44, ()), (44, (CLUSTER,))])
+def test_continuous_contacts(n, faults):
+    """behind a split cloth: the cluster solver, and the grid solver where that one is not launched"""
+    from solidcloth_b200 import api
+    sc, state = scenes.ccd_scene(n)
+    sc.params.flags &= ~scenes.CF_SELF
+
+    def build():
+        p = api.load_scene(sc)[1]
+        p.model.set_state(*state)
+        return p
+    assert max(_compare(build, 2, sc.dt, faults)) > 0
+
+
+@pytest.mark.parametrize("count,n", [(3, 40), (60, 30)])
+def test_batch_with_one_instance_in_contact(count, n):
+    """the cluster solver behind a small batch, the grid solver behind one of 54,000 particles;
+    an instance out of contact moves as in a batch of its own"""
+    from solidcloth_b200 import api
+    sc, state = scenes.ccd_scene(n)
+    sc.params.flags &= ~scenes.CF_SELF
+    calm = (sc.positions, sc.positions, np.zeros_like(sc.positions))
+    every = [state] + [calm] * (count - 1)
+    whole = tuple(np.concatenate([s[k] for s in every]).astype(np.float32) for k in range(3))
+
+    def build():
+        b = api.load_batch([sc] * count)
+        b.model.set_state(*whole)
+        return b
+    assert max(_compare(build, 2, sc.dt)) > 0
+    got = _run(build, 2, sc.dt, 0)[0]
+
+    def alone():
+        p = api.load_scene(sc)[1]
+        p.model.set_state(*calm)
+        return p
+    one = _run(alone, 2, sc.dt, 0)[0]
+    for a, b in zip(got, one):
+        assert np.array_equal(a[0][n * n:2 * n * n], b[0])
