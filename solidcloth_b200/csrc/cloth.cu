@@ -1013,7 +1013,7 @@ void ClothModel::release_tile_plan()
 {
     for (void* p : tileAllocs) cudaFree(p);
     tileAllocs.clear();
-    tilePlan = TilePlan{};
+    tilePlan = wholePlan = TilePlan{};
 }
 
 // colliders that make triangle / edge contacts
@@ -1040,20 +1040,45 @@ bool ClothModel::tile_eligible() const
     return dc.nTriColours <= 64 && dc.nEdgeColours <= 64;
 }
 
+// Live self-proximity of a cloth that fits one tile. Solved in one closed tile, a contact
+// colour is a CTA barrier, and a cluster barrier otherwise; but the FEM and bend sweeps
+// then have one SM (us an iteration, one tile / cluster, by contact colours):
+//   24 x 24   14 / 19 (0)     41 / 103 (36)
+//   32 x 32   16 / 19 (0)     50 / 107 (33)
+//   48 x 48   33 / 20 (0)     85 / 135 (54)    152 / 255 (126)
+//   64 x 64   46 / 20 (0)    133 / 188 (90)    244 / 349 (156)
+//   80 x 80   68 / 20 (0)    119 / 116 (40)    304 / 368 (153)
+//   96 x 96   91 / 22 (0)    161 / 139 (51)    215 / 233 (110)   409 / 398 (158)
+//   112 x 112 119 / 24 (0)   213 / 149 (59)    263 / 239 (117)
+// So up to 1,600 particles one tile always. Up to 9,216 the cloth is split, and behind
+// the tile launch the closed tile takes a substep of N / 120 contact colours or more
+// and the cluster solver one of fewer. Larger clothes have the cluster solver alone.
+constexpr int SELF_CLOSED = 1600, SELF_BOTH = 9216, SELF_PARTICLES_A_COLOUR = 120;
+
 bool ClothModel::ensure_tile_plan()
 {
     if (!tile_eligible()) { release_tile_plan(); return false; }
     const bool selfProx = (prm.flags & CF_SELF) != 0;
-    const int edgeSlots = (prm.flags & CF_EDGES) && instV.empty() ? feature_colliders() : 0;
-    const int triSlots = (prm.flags & CF_TRIANGLES) && instV.empty() ? feature_colliders() : 0;
-    const std::vector<int> key = {N, prm.fem, prm.dihedral, selfProx, prm.ccd, edgeSlots, triSlots, (int)tris.size(), (int)bends.size(), (int)links.size(),
+    const std::vector<int> key = {N, prm.fem, prm.dihedral, selfProx, prm.ccd, prm.flags & (CF_EDGES | CF_TRIANGLES), feature_colliders(), (int)tris.size(), (int)bends.size(), (int)links.size(),
                                   buf.stCap, buf.seCap};
     if (tilePlan.key == key) return tilePlan.valid;
     release_tile_plan();
+    build_tile_plan(tilePlan, selfProx && N <= SELF_CLOSED);
+    if (tilePlan.valid && tilePlan.open && instV.size() <= 2 && selfProx && N <= SELF_BOTH) build_tile_plan(wholePlan, true);
     tilePlan.key = key;
+    return tilePlan.valid;
+}
+
+// closed: one tile, even if the cloth is large enough to be split
+void ClothModel::build_tile_plan(TilePlan& plan, bool closed)
+{
+    plan = TilePlan{};
+    const bool selfProx = (prm.flags & CF_SELF) != 0;
+    const int edgeSlots = (prm.flags & CF_EDGES) && instV.empty() ? feature_colliders() : 0;
+    const int triSlots = (prm.flags & CF_TRIANGLES) && instV.empty() ? feature_colliders() : 0;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (sms < 1) return false;
+    if (sms < 1) return;
     constexpr int K = 5;                        // FEM, bends, links, edge contacts, triangle contacts
     TileSource src[K];
     auto fill = [&](TileSource& q, int arity, const std::vector<int>& order, const std::vector<int>& start, double step, double each) {
@@ -1094,10 +1119,8 @@ bool ClothModel::ensure_tile_plan()
         // tile / 64 a tile): 24 x 24 drop 519 / 548, 28 x 28 582 / 560, 32 x 32 603 / 569,
         // 36 x 36 706 / 591; 32 x 32 SDF drape 2356 / 1970. Every SM where there are fewer
         // than 64 particles for each: 45 x 45 links 145 / 134 with 64 a tile, 64 x 64 SDF
-        // drape 2123 / 2064. With live self-proximity a cloth that fits stays in one tile:
-        // its contacts take a hundred colours an iteration, each a CTA barrier there and a
-        // cluster or grid barrier otherwise.
-        if (N >= 700 && !(selfProx && N <= fit)) parts[0] = std::min(sms, N / 64);
+        // drape 2123 / 2064.
+        if (N >= 700 && !closed) parts[0] = std::min(sms, N / 64);
     }
     else
     {
@@ -1113,7 +1136,7 @@ bool ClothModel::ensure_tile_plan()
             parts[g] = k;
             if (k > 1) open += k;
         }
-        if (open > sms) return false;
+        if (open > sms) return;
     }
     std::vector<std::vector<int>> own;             // particles of each tile
     std::vector<int> tileInst, instTile(G + 1, 0);
@@ -1173,7 +1196,7 @@ bool ClothModel::ensure_tile_plan()
                 for (int a = 0; a < q.arity; a++)
                 {
                     int& slot = q.conOf[(size_t)c * N + v[a]];
-                    if (slot >= 0) return false;                   // the overflow colour of a greedy colouring
+                    if (slot >= 0) return;                         // the overflow colour of a greedy colouring
                     slot = j;
                 }
             }
@@ -1292,7 +1315,7 @@ bool ClothModel::ensure_tile_plan()
                     const int i = (*src[k].order)[j];
                     uint32_t pv[4];
                     src[k].get(i, pv);
-                    for (int a = 0; a < src[k].arity; a++) if (loc[pv[a]] < 0) return false;    // not a particle of the tile
+                    for (int a = 0; a < src[k].arity; a++) if (loc[pv[a]] < 0) return;    // not a particle of the tile
                     if (k == 0)
                     {
                         const FemHost& f = tris[i];
@@ -1310,7 +1333,7 @@ bool ClothModel::ensure_tile_plan()
         }
         for (int i = d.idBase; i < (int)ids.size(); i++) loc[ids[i]] = -1;
     }
-    if (mostLoc > (size_t)fit) return false;
+    if (mostLoc > (size_t)fit) return;
     // ---- CTAs: open tiles one each (all resident), closed ones to the least loaded, largest first
     std::vector<int> idx(nt);
     std::iota(idx.begin(), idx.end(), 0);
@@ -1330,12 +1353,13 @@ bool ClothModel::ensure_tile_plan()
     }
     std::vector<int> ctaStart{0}, ctaTile;
     for (auto& o : of) { ctaTile.insert(ctaTile.end(), o.begin(), o.end()); ctaStart.push_back((int)ctaTile.size()); }
-    tilePlan.smem = mostLoc * sizeof(float4);
+    plan.smem = mostLoc * sizeof(float4);
     // as many threads as the largest colour of a tile has records: idle warps cost
     // issue slots (a 17 x 17 cloth, 64 records a colour: 107 us a substep with 512
     // threads, 95 with 128)
-    const int threads = mostRec <= 128 && !selfProx ? 128 : mostRec <= 256 && !selfProx ? 256 : 512;
-    if (gs_tile_max_blocks_per_sm(threads, identity, tilePlan.smem) < 1) return false;
+    const bool contacts = identity && selfProx;
+    const int threads = mostRec <= 128 && !contacts ? 128 : mostRec <= 256 && !contacts ? 256 : 512;
+    if (gs_tile_max_blocks_per_sm(threads, identity, plan.smem) < 1) return;
     // ---- device copies
     bool ok = true;
     auto put = [&](const void* h, size_t bytes) -> void* {
@@ -1345,7 +1369,7 @@ bool ClothModel::ensure_tile_plan()
         if (!(h ? cudaMemcpy(p, h, bytes, cudaMemcpyHostToDevice) == cudaSuccess : zero_device(p, bytes))) ok = false;
         return p;
     };
-    TileView& v = tilePlan.view;
+    TileView& v = plan.view;
     v.nTiles = nt;
     v.N = N;
     v.threads = threads;
@@ -1378,11 +1402,10 @@ bool ClothModel::ensure_tile_plan()
         v.xch = (float4*)put(nullptr, sizeof(float4) * 2 * (size_t)N);
         v.xred = (unsigned long long*)put(nullptr, sizeof(unsigned long long) * 2 * (size_t)nt);
     }
-    if (!ok) { release_tile_plan(); tilePlan.key = key; return false; }
-    tilePlan.ctas = ctas;
-    tilePlan.open = open;
-    tilePlan.valid = true;
-    return true;
+    if (!ok) return;                            // what was allocated goes with the plans
+    plan.ctas = ctas;
+    plan.open = open;
+    plan.valid = true;
 }
 
 bool ClothModel::upload_topology(const HMesh& mesh)
@@ -1916,7 +1939,7 @@ bool ClothModel::ensure_buffers(const CollisionWorld& world, cudaStream_t s)
     buf.ecFlag = (int*)dalloc(sizeof(int) * (size_t)buf.ecCap, true);
     buf.ecList = (EC*)dalloc(sizeof(EC) * (size_t)buf.ecCap, true);
     int* counts = (int*)dalloc(sizeof(int) * 16, true);
-    buf.meshQueryCount = counts + 11;
+    buf.meshQueryCount = counts + 11; buf.selfColours = counts + 14;
     buf.tcCount = counts; buf.ecCount = counts + 1; buf.stCount = counts + 2; buf.seCount = counts + 3;
     buf.ccdVtPairCount = counts + 4; buf.ccdEePairCount = counts + 5; buf.scanTot = counts + 8;
     // self contacts
@@ -2542,11 +2565,15 @@ bool ClothPatch::record_solve(cudaStream_t s, const SolverParams& P, const Solve
         // self contacts across tiles go to the launch after it (GUARD_*)
         const bool other = !m.tilePlan.view.identity && ((m.prm.flags & CF_SELF) || m.prm.ccd);
         if (launched(SOLVE_TILE, [&] {
-                return ops.tile(s, c, P, b, m.tilePlan.view, m.tilePlan.ctas, m.tilePlan.smem, iterations, other ? GUARD_IF_NO_SELF : GUARD_NONE);
+                return ops.tile(s, c, P, b, m.tilePlan.view, m.tilePlan.ctas, m.tilePlan.smem, iterations, SolveGuard{other ? GUARD_IF_NO_SELF : GUARD_NONE, 0});
             }))
         {
             if (!other) return true;
-            plan.guard = GUARD_IF_SELF;
+            plan.guard = {GUARD_IF_SELF, 0};
+            const ClothModel::TilePlan& whole = m.wholePlan;
+            const SolveGuard many = {GUARD_IF_MANY, m.N / SELF_PARTICLES_A_COLOUR};
+            if (whole.valid && launched(SOLVE_TILE, [&] { return ops.tile(s, c, P, b, whole.view, whole.ctas, whole.smem, iterations, many); }))
+                plan.guard = {GUARD_IF_FEW, many.colours};
             if (m.N <= GUARD_CLUSTER && record_cluster(s, P, plan, 0)) return true;
             return launched(SOLVE_GRID, [&] { return ops.grid(s, c, P, b, plan, 0, m.N <= GUARD_GRID_1 ? 1 : m.N <= GUARD_GRID_2 ? 2 : 3); });
         }

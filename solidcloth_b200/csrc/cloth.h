@@ -223,7 +223,8 @@ public:
         BandView view{};                                   // device arrays (in allocs)
     } bandPlan;
     void build_band_plan();
-    // tile solver (k_gs_tile): the plan in use, rebuilt when what it depends on changes
+    // tile solver (k_gs_tile): the plan in use, rebuilt when what it depends on changes;
+    // behind a split cloth with live proximity also the cloth in one closed tile
     struct TilePlan
     {
         bool valid = false;
@@ -232,9 +233,10 @@ public:
         bool open = false;                                 // some cloth spans several tiles
         size_t smem = 0;
         TileView view{};
-    } tilePlan;
+    } tilePlan, wholePlan;
     std::vector<void*> tileAllocs;
     bool ensure_tile_plan();
+    void build_tile_plan(TilePlan& plan, bool closed);
     bool tile_eligible() const;
     int feature_colliders() const;
     void release_tile_plan();

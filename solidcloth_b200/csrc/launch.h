@@ -70,6 +70,7 @@ struct Buffers
     int2* ccdVtSorted; int2* ccdEeSorted;
     // colouring scratch
     ColourScratch colouring[2];  // self vertex-triangle, self edge-edge
+    int* selfColours;            // colours of the two classes in this substep
     int* colour; int* order; int* colourStart; int colourCap;
     // scan scratch: block sums, per-item offsets, totals
     int* scanBlock; int* scanOff; int* scanTot;
@@ -146,6 +147,12 @@ void launch_gs_exit_test(cudaStream_t s, const DevCloth& c, const SolverParams& 
 // cluster-resident Gauss-Seidel solver (one cluster per cloth, one launch per substep)
 constexpr int GS_THREADS = 512;
 constexpr int GS_SMEM_MAX = 200 * 1024; // dynamic shared memory per CTA: particles + staged records
+// A tile launch cannot solve self contacts that reach across its tiles: it works
+// only while there are none, and a launch after it only when there are some (the
+// counts are known on the device alone); of two launches after it, one with fewer
+// contact colours than `colours` and the other with as many or more.
+enum { GUARD_NONE = 0, GUARD_IF_SELF = 1, GUARD_IF_NO_SELF = 2, GUARD_IF_FEW = 3, GUARD_IF_MANY = 4 };
+struct SolveGuard { int kind, colours; };
 struct GsPlan
 {
     int iterations, vpc, nFemCol, nBendCol;   // vpc: particles per CTA (cluster solver)
@@ -155,12 +162,8 @@ struct GsPlan
     int bendStart[65];
     int nLinkCol;            // mass-spring path (FEM off): link colours
     int linkStart[65];
-    int guard;               // GUARD_*: whether the launch does its work
+    SolveGuard guard;        // whether the launch does its work
 };
-// A tile launch cannot solve self contacts that reach across its tiles: it works
-// only while there are none, and the launch after it only when there are some
-// (the counts are known on the device alone).
-enum { GUARD_NONE = 0, GUARD_IF_SELF = 1, GUARD_IF_NO_SELF = 2 };
 // cluster size usable for N particles (0: too large or unsupported); sets the
 // particles per CTA and the dynamic shared memory per CTA
 int gs_cluster_size(int N, int& vpc, size_t& smem);
@@ -273,7 +276,7 @@ struct SolverOps
     bool (*grid)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&, GsPlan, int, int);
     bool (*band)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&, GsPlan, const BandView&, int, size_t,
                  int);
-    bool (*tile)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&, const TileView&, int, size_t, int, int);
+    bool (*tile)(cudaStream_t, const DevCloth&, const SolverParams&, const Buffers&, const TileView&, int, size_t, int, SolveGuard);
 };
 const SolverOps& solver_ops(bool fast);
 

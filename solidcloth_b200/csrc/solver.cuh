@@ -692,12 +692,13 @@ __global__ void k_reset_bend_error(DevCloth c)
 }
 
 
-// GUARD_*: does this launch do its work? (the same answer in every thread)
-__device__ __forceinline__ bool guard_open(int guard, const ColourArgs& ca)
+// does this launch do its work? (the same answer in every thread)
+__device__ __forceinline__ bool guard_open(SolveGuard g, const ColourArgs& ca, const Buffers& b)
 {
-    if (guard == GUARD_NONE) return true;
+    if (g.kind == GUARD_NONE) return true;
     const bool self = *ca.cls[2].count + *ca.cls[3].count > 0;
-    return self == (guard == GUARD_IF_SELF);
+    if (g.kind == GUARD_IF_SELF || g.kind == GUARD_IF_NO_SELF) return self == (g.kind == GUARD_IF_SELF);
+    return self && (b.selfColours[0] + b.selfColours[1] >= g.colours) == (g.kind == GUARD_IF_MANY);
 }
 
 // The cloth's particles in equal blocks over the cluster's CTAs. The block size is
@@ -952,7 +953,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_cluster(DevCloth c, SolverPar
 {
     extern __shared__ float4 sPos[];
     __shared__ float sErr[8];
-    if (!guard_open(plan.guard, ca)) return;
+    if (!guard_open(plan.guard, ca, b)) return;
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
     const int nRank = (int)cl.num_blocks();
@@ -1750,7 +1751,7 @@ __device__ __forceinline__ void tile_contact_classes(const TilePos& pa, const De
 // kernel of its own, because its contact solves cost the other one registers
 template <int NT, bool WHOLE>
 __global__ void __launch_bounds__(NT, 1) k_gs_tile(DevCloth c, SolverParams P, Buffers b, ColourArgs ca,
-                                                              __grid_constant__ const TileView tv, int iterations, int guard)
+                                                              __grid_constant__ const TileView tv, int iterations, SolveGuard guard)
 {
     extern __shared__ float4 sPos[];
     __shared__ float sErr[8];
@@ -1759,7 +1760,7 @@ __global__ void __launch_bounds__(NT, 1) k_gs_tile(DevCloth c, SolverParams P, B
     __shared__ int sCnt[2][MAX_COLOURS];
     __shared__ int sStart[WHOLE ? 2 : 1][MAX_COLOURS + 1];
     if (blockIdx.x == 0 && threadIdx.x == 0) c.scal[0] = 0.f;      // for the next prediction; the detection is done
-    if (!guard_open(guard, ca)) return;
+    if (!guard_open(guard, ca, b)) return;
     const int tid = (int)threadIdx.x;
     const bool track = !P.fixedIterations;
     // collider contacts of this substep (the same answer in every tile)
@@ -1984,7 +1985,7 @@ __device__ __forceinline__ float bend_tiles(const DevCloth& c, const SolverParam
 template <int NT, int FT, int BT>
 __global__ void __launch_bounds__(NT) k_gs_grid(DevCloth c, SolverParams P, Buffers b, ColourArgs ca, GsPlan plan)
 {
-    if (!guard_open(plan.guard, ca)) return;
+    if (!guard_open(plan.guard, ca, b)) return;
     cg::grid_group grid = cg::this_grid();
     __shared__ float sErr[8];
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
@@ -2285,7 +2286,7 @@ bool launch_gs_band(cudaStream_t s, const DevCloth& c, const SolverParams& P, co
 }
 
 // ---------------------------------------------- tile solver launcher
-using TileKernel = void (*)(DevCloth, SolverParams, Buffers, ColourArgs, const TileView, int, int);
+using TileKernel = void (*)(DevCloth, SolverParams, Buffers, ColourArgs, const TileView, int, SolveGuard);
 static TileKernel tile_kernel(int threads, bool whole)
 {
     if (whole) return threads == 128 ? k_gs_tile<128, true> : threads == 256 ? k_gs_tile<256, true> : k_gs_tile<512, true>;
@@ -2311,7 +2312,7 @@ int gs_tile_max_blocks_per_sm(int threads, bool whole, size_t smem)
 
 // a cooperative launch where tiles wait for one another (all of them resident)
 bool launch_gs_tile(cudaStream_t s, const DevCloth& c, const SolverParams& P, const Buffers& b, const TileView& tv,
-                    int ctas, size_t smem, int iterations, int guard)
+                    int ctas, size_t smem, int iterations, SolveGuard guard)
 {
     const TileKernel kernel = tile_kernel(tv.threads, tv.identity != 0);
     tile_smem_limit(kernel, smem);

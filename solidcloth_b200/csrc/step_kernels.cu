@@ -960,6 +960,7 @@ __device__ void colour_class(const DevCloth& c, const Buffers& b, const ClassVie
         round++;
     }
     for (int k = round + tid; k <= MAX_COLOURS; k += nt) cv.start[k] = k < MAX_COLOURS ? head : n;
+    if (tid == 0) b.selfColours[cv.kind - 2] = round + (head < n);
     if (head < n)
     {
         // not expected for contact graphs of bounded degree: the rest go to the
@@ -1035,6 +1036,7 @@ __global__ void __launch_bounds__(1024) k_colour(DevCloth c, Buffers b, ColourAr
     if (*cv.count == 0)
     {
         if (threadIdx.x <= MAX_COLOURS) cv.start[threadIdx.x] = 0;
+        if (threadIdx.x == 0 && cv.kind >= 2) b.selfColours[cv.kind - 2] = 0;
         return;
     }
     if (cv.kind <= 1) static_colour_class(c, b, cv);

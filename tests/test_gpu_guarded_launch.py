@@ -1,6 +1,6 @@
 """Clothes split into tiles that do meet self contacts: the launches behind the tile
-launch (the cluster solver and the grid solver, by size) against the per-colour path,
-bit for bit."""
+launch (one closed tile, the cluster and the grid solver, by size and by the number
+of contact colours) against the per-colour path, bit for bit."""
 import numpy as np
 import pytest
 
@@ -9,6 +9,23 @@ from solidcloth_b200 import scenes
 pytestmark = pytest.mark.gpu
 
 TILE, CLUSTER, GRID, KERNELS = 5, 1, 2, 3
+
+
+def _flap(n, rows, iterations=3, substeps=2):
+    """a cloth on the floor, its last rows folded over: rows == n // 2 folds it in half"""
+    inc = 1.0 / (n - 1)
+    t = min(0.005, 0.35 * inc)
+    p = scenes.Params(thickness=t, tolerance=t, friction=0.3, iterations=iterations, substeps=substeps, flags=scenes.CF_SELF | scenes.CF_WALLS)
+    sc = scenes.make_grid_scene("flap", n, 1.0, p.thickness, p, seed=1)
+    noise = np.random.default_rng(1).uniform(-0.1 * inc, 0.1 * inc, (n * n, 3))
+    sc.positions = (scenes.grid_positions(n, sc.inc, sc.offset) + noise).astype(np.float32)
+    sc.walls = np.array([-20.0, 0.0, -20.0, 20.0, 20.0, 20.0], dtype=np.float32)
+    pos = sc.positions.copy().reshape(n, n, 3)
+    for k in range(rows):
+        pos[:, n - 1 - k, 2] = pos[:, n - 1 - 2 * rows + k, 2]
+        pos[:, n - 1 - k, 1] += np.float32(sc.inc)
+    pos = pos.reshape(-1, 3).astype(np.float32)
+    return sc, (pos, pos.copy(), np.zeros_like(pos))
 
 
 def _colours(p):
@@ -38,6 +55,35 @@ def _compare(build, frames, dt, faults=()):
         for x, y in zip(a, b):
             assert np.array_equal(x, y), f
     return c0
+
+
+# 40: the last size in one tile; 41: split, with one closed tile behind; 96 and 97: the
+# last size with one and the first without. Few and many colours: both launches of a guard.
+@pytest.mark.parametrize("n,rows", [(40, 4), (41, 2), (41, 4), (48, 24), (64, 4), (96, 3), (96, 6), (97, 4)])
+def test_live_proximity(n, rows):
+    from solidcloth_b200 import api
+    sc, state = _flap(n, rows)
+
+    def build():
+        p = api.load_scene(sc)[1]
+        p.model.set_state(*state)
+        return p
+    assert max(_compare(build, 4, sc.dt)) > 0
+
+
+def test_both_sides_of_the_colour_rule():
+    """fewer contact colours than one in 120 particles, and more"""
+    from solidcloth_b200 import api
+    seen = []
+    for n, rows in ((80, 2), (96, 2), (64, 4)):
+        sc, state = _flap(n, rows, 15, 8)
+
+        def build():
+            p = api.load_scene(sc)[1]
+            p.model.set_state(*state)
+            return p
+        seen += [c / (n * n // 120) for c in _compare(build, 4, sc.dt)]
+    assert any(0 < c < 1 for c in seen) and any(c >= 1 for c in seen), seen
 
 
 @pytest.mark.parametrize("n,faults", [(44, ()), (44, (CLUSTER,))])
