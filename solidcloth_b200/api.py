@@ -375,6 +375,8 @@ class ClothModel:
         n = lib().scGetSolverChoice(self.h, out.ctypes.data_as(_i), log.ctypes.data_as(_f), 64)
         return tuple(int(x) for x in out), log[:min(n, 64)].copy()
 
+    # names of the broad-phase modes 0 and 1, kept for callers: the tree walks they
+    # named are gone, both run the blocked join
     BROAD_WALKS = ("per-query stack walk", "warp packet")
 
     def set_broad_phase_mode(self, mode: int):

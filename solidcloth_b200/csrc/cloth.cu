@@ -2643,8 +2643,10 @@ bool ClothPatch::autotune(float h)
     }
     std::vector<SolverChoice> cand;
     int shift = 0; size_t smem = 0;
-    // the tile solver where it applies: it measured faster than every other one over
-    // the whole range (16 x 16 to 256 x 256, batches), so nothing else is timed
+    // the tile solver where it applies; nothing else is timed. Its solve against the
+    // fastest other one, ms a substep: 24 x 24 drop 0.12 / 0.18, 128 x 128 drape in the
+    // fast build 0.21 / 0.34, 200 x 200 0.23 / 0.75, 512 instances of 1.9 M particles
+    // 3.0 / 3.6. (Self contacts of split clothes: SELF_CLOSED, GUARD_CLUSTER.)
     const bool tile = m.tilePlan.valid;
     if (tile) cand.push_back({SOLVE_TILE, 0, 0, 0.f});
     const bool fits = m.triColourStart.size() <= 65 && m.bendColourStart.size() <= 65 && m.linkColourStart.size() <= 65;
