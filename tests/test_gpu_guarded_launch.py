@@ -86,6 +86,28 @@ def test_both_sides_of_the_colour_rule():
     assert any(0 < c < 1 for c in seen) and any(c >= 1 for c in seen), seen
 
 
+def test_with_collider_contacts():
+    """triangle and edge contacts of a collider beside the self contacts, in the closed tile behind"""
+    from solidcloth_b200 import api
+    sc, state = _flap(48, 4)
+    sc.params.flags |= scenes.CF_VERTICES | scenes.CF_TRIANGLES | scenes.CF_EDGES
+    sc.masses = np.ones(sc.num_vertices, np.float32)
+    sc.meshes.append(scenes.icosphere(3, 0.2, (0.0, -0.195, 0.0)))
+    found = []
+
+    def build():
+        p = api.load_scene(sc)[1]
+        p.model.set_state(*state)
+        step = p.step
+        def stepped(dt):
+            step(dt)
+            found.append([len(p.model.contacts(k)[0]) for k in (1, 2)])
+        p.step = stepped
+        return p
+    assert max(_compare(build, 3, sc.dt)) > 0
+    assert min(max(f[k] for f in found) for k in (0, 1)) > 0
+
+
 @pytest.mark.parametrize("n,faults", [(44, ()), (44, (CLUSTER,))])
 def test_continuous_contacts(n, faults):
     """behind a split cloth: the cluster solver, and the grid solver where that one is not launched"""
