@@ -276,7 +276,8 @@ SCEXP void scSetClusterSolver(scModel model, bool val);
 /* Solver for the Gauss-Seidel loop (additions, no reference counterpart).
    0 = automatic (default: the tile kernel where the cloth has a tile plan, else
    the fastest of the cluster kernel, the grid-resident cooperative kernel's
-   variants and the per-colour kernels, timed on this cloth at the first step), 1 = cluster kernel (clothes up to 131,072 particles),
+   variants and the per-colour kernels, timed on this cloth at the first step),
+   1 = cluster kernel (clothes up to 131,072 particles),
    2 = grid kernel (tuned variant), 3 = per-colour kernels, 4 = band-parallel
    kernel (clothes with a band plan, scGetBandPlan; its thread count timed at
    the first step). Modes 0-3 give identical results (the colour order); the
@@ -288,7 +289,8 @@ SCEXP void scSetSolverMode(scModel model, int mode);
 SCEXP void scSetGridSolver(scModel model, int variant, int blocksPerSm);
 /* force the cluster kernel with 1 (variant 0) or 2 (variant 1) constraints per thread */
 SCEXP void scSetClusterVariant(scModel model, int variant);
-/* out4 = {kind, grid variant, CTAs per SM, threads per CTA} of the solver in use;
+/* out4 = {kind (1 .. 4 as scSetSolverMode, 5: the tile kernel), grid variant, CTAs per
+   SM, threads per CTA} of the solver in use;
    tuneMs (4 floats per candidate: kind, variant, CTAs per SM, ms per substep)
    gets up to cap candidates of the last tuning; returns the candidate count */
 SCEXP int scGetSolverChoice(scModel model, int* out4, float* tuneMs, int cap);
