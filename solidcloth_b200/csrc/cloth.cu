@@ -1065,6 +1065,7 @@ bool ClothModel::ensure_tile_plan()
     release_tile_plan();
     build_tile_plan(tilePlan, selfProx && N <= SELF_CLOSED);
     if (tilePlan.valid && tilePlan.open && instV.size() <= 2 && selfProx && N <= SELF_BOTH) build_tile_plan(wholePlan, true);
+    if (!tilePlan.valid) release_tile_plan();
     tilePlan.key = key;
     return tilePlan.valid;
 }
@@ -1402,7 +1403,7 @@ void ClothModel::build_tile_plan(TilePlan& plan, bool closed)
         v.xch = (float4*)put(nullptr, sizeof(float4) * 2 * (size_t)N);
         v.xred = (unsigned long long*)put(nullptr, sizeof(unsigned long long) * 2 * (size_t)nt);
     }
-    if (!ok) return;                            // what was allocated goes with the plans
+    if (!ok) return;                            // what was allocated goes with the plans (tileAllocs)
     plan.ctas = ctas;
     plan.open = open;
     plan.valid = true;
@@ -2456,8 +2457,7 @@ bool ClothPatch::record_substep(float h)
     timing_mark(SEC_GS, false, s);
     if (!record_solve(s, P, m.choice))
     {
-        const cudaError_t e = cudaGetLastError();
-        set_error(SC_ERR_CUDA, std::string("solver launch failed: ") + cudaGetErrorString(e));
+        set_error(SC_ERR_CUDA, "solver launch failed");
         return false;
     }
     timing_mark(SEC_GS, true, s);
